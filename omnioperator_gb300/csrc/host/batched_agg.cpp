@@ -98,6 +98,9 @@ struct BatchedAggregation::Impl {
     DevArray<uint32_t> counts;  // padded to 64 rows per task (output regions)
     DevArray<uint32_t> groups;  // exact groups per task
     DevArray<int64_t> offsets;
+    DevArray<omg::TaskChunk> chunks;
+    int32_t nChunks = 0;
+    DevArray<unsigned long long> cursor;
     DevArray<int64_t> blockSums;
     DevArray<long long> total;
     DevArray<unsigned long long> scratch;  // extraction's error / ambiguity words
@@ -158,7 +161,7 @@ struct BatchedAggregation::Impl {
         CudaCheck(cudaMemsetAsync(failed.Get(), 0, sizeof(uint32_t) * n, s), "reset task flags");
         CudaCheck(omg::LaunchAggInitTable(p, s), "init task tables");
         CudaCheck(omg::LaunchAggTasks(p, variant, s), "batched aggregation");
-        CudaCheck(omg::LaunchAggTaskCount(tables.Get(), n, plan.key.kind, groups.Get(), s), "count task groups");
+        CudaCheck(omg::LaunchAggTaskCount(tables.Get(), n, chunks.Get(), nChunks, plan.key.kind, groups.Get(), s), "count task groups");
         CudaCheck(omg::LaunchAggTaskPad(groups.Get(), n, counts.Get(), s), "pad task regions");
         CudaCheck(omg::LaunchScanCounts(counts.Get(), n, offsets.Get(), blockSums.Get(), total.Get(), s),
             "place task outputs");
@@ -187,7 +190,8 @@ struct BatchedAggregation::Impl {
         e.nAmbiguous = scratch.Get() + 3;
         e.ambiguousSlots = scratch.Get() + 4;
         e.ambiguousCap = 0;
-        CudaCheck(omg::LaunchAggTaskExtract(e, tables.Get(), n, offsets.Get(), s), "extract task groups");
+        CudaCheck(omg::LaunchAggTaskExtract(e, tables.Get(), n, chunks.Get(), nChunks, offsets.Get(), cursor.Get(), s),
+            "extract task groups");
     }
 
     void Prepare(cudaStream_t s)
@@ -276,6 +280,19 @@ struct BatchedAggregation::Impl {
         counts.Reset(n, s);
         groups.Reset(n, s);
         offsets.Reset(n, s);
+        std::vector<omg::TaskChunk> hostChunks;
+        hostChunks.reserve(totalSlots / omg::kTaskChunkSlots + n);
+        for (int32_t t = 0; t < n; ++t) {
+            for (uint64_t c = 0; c * omg::kTaskChunkSlots < capacity[t] + 2; ++c) {
+                hostChunks.push_back(omg::TaskChunk{t, static_cast<uint32_t>(c)});
+            }
+        }
+        nChunks = static_cast<int32_t>(hostChunks.size());
+        chunks.Reset(hostChunks.size(), s);
+        CudaCheck(cudaMemcpyAsync(chunks.Get(), hostChunks.data(), sizeof(omg::TaskChunk) * hostChunks.size(),
+                      cudaMemcpyHostToDevice, s),
+            "upload task chunks");
+        cursor.Reset(n, s);
         blockSums.Reset(static_cast<size_t>(n) / 1024 + 2, s);
         total.Reset(1, s, true);
         hGroups.Reset(n);
@@ -289,7 +306,7 @@ struct BatchedAggregation::Impl {
             outCols[o].nulls = omg::Buffer::NewDevice(omg::NullBitmapBytes(static_cast<int64_t>(outBound)), s, true);
             outCols[o].hasNull = plan.outs[o].kind != omg::OUT_COUNT && plan.outs[o].kind != omg::OUT_IS_EMPTY;
         }
-        CudaCheck(cudaStreamSynchronize(s), "cudaStreamSynchronize");  // hostTables is on the stack
+        CudaCheck(cudaStreamSynchronize(s), "cudaStreamSynchronize");  // hostTables and hostChunks are on the stack
         prepareUs = NowUs() - t0;
         Tune(s);
         // Capture the per-run sequence once (a private stream is needed for capture).

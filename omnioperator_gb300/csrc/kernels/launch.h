@@ -40,11 +40,12 @@ cudaError_t LaunchAggTaskSketch(const AggLaunch &p, int32_t nTasks, unsigned lon
 int32_t AggTasksVariants();
 void AggTasksVariantShape(int32_t variant, int32_t *threads, int32_t *blocksPerSM);
 cudaError_t LaunchAggTasks(const AggLaunch &p, int32_t variant, cudaStream_t stream);
-cudaError_t LaunchAggTaskCount(const AggTable *tables, int32_t nTasks, int32_t keyKind, uint32_t *counts,
-    cudaStream_t stream);
+cudaError_t LaunchAggTaskCount(const AggTable *tables, int32_t nTasks, const TaskChunk *chunks, int32_t nChunks,
+    int32_t keyKind, uint32_t *counts, cudaStream_t stream);
 cudaError_t LaunchAggTaskPad(const uint32_t *groups, int32_t nTasks, uint32_t *padded, cudaStream_t stream);
-cudaError_t LaunchAggTaskExtract(const AggExtract &e, const AggTable *tables, int32_t nTasks, const int64_t *offsets,
-    cudaStream_t stream);
+// cursor: nTasks words of scratch.
+cudaError_t LaunchAggTaskExtract(const AggExtract &e, const AggTable *tables, int32_t nTasks, const TaskChunk *chunks,
+    int32_t nChunks, const int64_t *offsets, unsigned long long *cursor, cudaStream_t stream);
 cudaError_t LaunchAggCount(const AggTable &t, int keyKind, unsigned long long *out, cudaStream_t stream);
 cudaError_t LaunchAggExtract(const AggExtract &e, cudaStream_t stream);
 // Ordered replay of order-dependent sticky-overflow groups; sets forced[slot] bit k when

@@ -194,6 +194,14 @@ struct AggLaunch {
 constexpr int kTaskSketchRows = 1024;   // rows sampled per task by the batched sketch
 constexpr int kTaskSketchSlots = 2048;
 
+// Slots [chunk * kTaskChunkSlots, ...) of task `task`'s table: the unit in which the tasks' groups
+// are counted and extracted.
+constexpr uint64_t kTaskChunkSlots = 2048;
+struct TaskChunk {
+    int32_t task;
+    uint32_t chunk;
+};
+
 // ---- hash partitioning of aggregation input -------------------------------------------------
 // Rows go to partition (hash >> kPartShift) & (nParts - 1); the shared tables index slots with
 // the hash's top 32 bits and the global table with its low bits, so the three are independent.

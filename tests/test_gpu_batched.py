@@ -118,3 +118,19 @@ def test_batched_with_learned_sizer(gpu):
     _check(tasks, per)
     assert info["learned"] == 1
     model.close()
+
+
+@pytest.mark.parametrize("groups", [1, 511, 512, 1023, 1024, 1025, 9000])
+def test_batched_tables_around_a_chunk_of_slots(gpu, groups):
+    """Tables are counted and extracted 2048 slots at a time: group counts whose tables end just
+    below, at and just past a chunk (two special slots follow the power-of-two capacity), next to a
+    one-row task and NULL and EMPTY keys (the special slots of the last chunk)."""
+    rng = np.random.default_rng(groups)
+    tasks = []
+    for n in (1, 3 * groups + 7):
+        key = (np.arange(n) % groups).astype(np.int64) * 7919
+        key[-1] = np.iinfo(np.int64).min
+        km = np.arange(n) % 97 == 5
+        tasks.append((key, rng.integers(-10**6, 10**6, n, dtype=np.int64), rng.random(n), km, None, None))
+    (per,), _ = _run(tasks)
+    _check(tasks, per)
