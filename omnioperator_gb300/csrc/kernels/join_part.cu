@@ -123,73 +123,89 @@ __global__ void __launch_bounds__(kPartThreads) KeyHistKernel(const int64_t *key
     }
 }
 
-// Partition totals and starts: total[p] = sum over chunks; start[p] = exclusive prefix of the
-// totals (start[P] = all rows).  One block.
-__global__ void PartTotalsKernel(const uint32_t *hist, int32_t nChunks, int32_t P, int64_t *start)
-{
-    __shared__ long long warpSum[32];
-    __shared__ long long carry;
-    if (threadIdx.x == 0) {
-        carry = 0;
-    }
-    __syncthreads();
-    for (int base = 0; base < P; base += blockDim.x) {
-        const int p = base + threadIdx.x;
-        long long t = 0;
-        if (p < P) {
-            for (int c = 0; c < nChunks; ++c) {
-                t += hist[static_cast<int64_t>(c) * P + p];
-            }
-        }
-        // block-wide exclusive scan of t
-        const int lane = threadIdx.x & 31;
-        const int warp = threadIdx.x >> 5;
-        long long inc = t;
-        for (int o = 1; o < 32; o <<= 1) {
-            const long long y = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) {
-                inc += y;
-            }
-        }
-        if (lane == 31) {
-            warpSum[warp] = inc;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            long long run = 0;
-            for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) {
-                const long long v = warpSum[w];
-                warpSum[w] = run;
-                run += v;
-            }
-        }
-        __syncthreads();
-        if (p < P) {
-            start[p] = carry + warpSum[warp] + inc - t;
-        }
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) {
-            carry += warpSum[warp] + inc;
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        start[P] = carry;
-    }
-}
+// Placement within a partition: place[c * P + p] = rows of partition p in chunks before c, and
+// total[p] = all its rows.  A CTA takes 32 partitions; its 32 rows of threads take 1/32 of the chunks
+// each, so a row of the histogram matrix is read 128 bytes at a time by P / 32 CTAs (one block for the
+// totals and one thread per partition for the placement ran 1056 + 448 us on 1024 x 4096 counts; the
+// probe of 2^26 keys through 4096 partitions went from 4.50 to 3.18 ms).
+constexpr int kPlaceParts = 32;
 
-// Placement of each (chunk, partition): place[c * P + p] = start[p] + rows of partition p in
-// chunks before c.  One thread per partition.
-__global__ void PlaceKernel(const uint32_t *hist, int32_t nChunks, int32_t P, const int64_t *start, int64_t *place)
+__global__ void __launch_bounds__(kPlaceParts * 32) PlaceKernel(const uint32_t *hist, int32_t nChunks, int32_t P,
+    int64_t *place, int64_t *total)
 {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ long long part[32][kPlaceParts];
+    const int x = threadIdx.x % kPlaceParts;
+    const int y = threadIdx.x / kPlaceParts;
+    const int p = blockIdx.x * kPlaceParts + x;
+    const int per = (nChunks + 31) / 32;
+    const int c0 = min(y * per, nChunks);
+    const int c1 = min(c0 + per, nChunks);
+    long long mine = 0;
+    if (p < P) {
+#pragma unroll 8
+        for (int c = c0; c < c1; ++c) {
+            mine += __ldg(hist + static_cast<int64_t>(c) * P + p);
+        }
+    }
+    part[y][x] = mine;
+    __syncthreads();
+    long long run = 0;
+    for (int j = 0; j < y; ++j) {
+        run += part[j][x];
+    }
     if (p >= P) {
         return;
     }
-    int64_t run = start[p];
-    for (int c = 0; c < nChunks; ++c) {
+    if (y == 31) {
+        total[p] = run + mine;
+    }
+#pragma unroll 8
+    for (int c = c0; c < c1; ++c) {
         place[static_cast<int64_t>(c) * P + p] = run;
-        run += hist[static_cast<int64_t>(c) * P + p];
+        run += __ldg(hist + static_cast<int64_t>(c) * P + p);
+    }
+}
+
+// start[p] = exclusive prefix of the totals (in place), start[P] = all rows.  One block.
+__global__ void __launch_bounds__(1024) PartStartsKernel(int32_t P, int64_t *start)
+{
+    __shared__ long long warpSum[32];
+    constexpr int kPer = kMaxJoinParts / 1024;
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    long long v[kPer];
+    long long mine = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        const int p = threadIdx.x * kPer + j;
+        v[j] = p < P ? start[p] : 0;
+        mine += v[j];
+    }
+    long long inc = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) {
+            inc += y;
+        }
+    }
+    if (lane == 31) {
+        warpSum[warp] = inc;
+    }
+    __syncthreads();
+    long long run = inc - mine;
+    for (int w = 0; w < warp; ++w) {
+        run += warpSum[w];
+    }
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        const int p = threadIdx.x * kPer + j;
+        if (p < P) {
+            start[p] = run;
+            run += v[j];
+            if (p == P - 1) {
+                start[P] = run;
+            }
+        }
     }
 }
 
@@ -209,8 +225,8 @@ __device__ __forceinline__ void CopyBytes(uint8_t *dst, const uint8_t *src, int 
 // Scatter of a chunk's non-NULL rows to their partitions: key, and (build side) the packed
 // payload bytes of the row's output columns.
 __global__ void __launch_bounds__(kPartThreads) KeyScatterKernel(const int64_t *keys, const uint8_t *nulls, int64_t n,
-    const __grid_constant__ JoinPartFn f, int32_t nChunks, const int64_t *place, int64_t *outKeys,
-    const __grid_constant__ PayloadCols pay, uint8_t *outPay)
+    const __grid_constant__ JoinPartFn f, int32_t nChunks, const int64_t *start,
+    const int64_t *place, int64_t *outKeys, const __grid_constant__ PayloadCols pay, uint8_t *outPay)
 {
     extern __shared__ unsigned char smem[];
     unsigned long long *cur = reinterpret_cast<unsigned long long *>(smem + kRangeSmem);
@@ -218,7 +234,7 @@ __global__ void __launch_bounds__(kPartThreads) KeyScatterKernel(const int64_t *
     const RangeLut rl = StageSplits(f, smem);
     for (int c = blockIdx.x; c < nChunks; c += gridDim.x) {
         for (int i = threadIdx.x; i < P; i += blockDim.x) {
-            cur[i] = static_cast<unsigned long long>(place[static_cast<int64_t>(c) * P + i]);
+            cur[i] = static_cast<unsigned long long>(start[i] + place[static_cast<int64_t>(c) * P + i]);
         }
         __syncthreads();
         int64_t b, e;
@@ -416,10 +432,10 @@ cudaError_t LaunchKeyPartition(const int64_t *keys, const uint8_t *nulls, int64_
     }
     const int grid = nChunks < SMs() * 4 ? nChunks : SMs() * 4;
     KeyHistKernel<<<grid, kPartThreads, smemHist, stream>>>(keys, nulls, n, f, nChunks, hist);
-    PartTotalsKernel<<<1, 1024, 0, stream>>>(hist, nChunks, P, start);
-    PlaceKernel<<<(P + 255) / 256, 256, 0, stream>>>(hist, nChunks, P, start, place);
-    KeyScatterKernel<<<grid, kPartThreads, smemScatter, stream>>>(keys, nulls, n, f, nChunks, place, outKeys, pay,
-        outPay);
+    PlaceKernel<<<(P + kPlaceParts - 1) / kPlaceParts, kPlaceParts * 32, 0, stream>>>(hist, nChunks, P, place, start);
+    PartStartsKernel<<<1, 1024, 0, stream>>>(P, start);
+    KeyScatterKernel<<<grid, kPartThreads, smemScatter, stream>>>(keys, nulls, n, f, nChunks, start, place, outKeys,
+        pay, outPay);
     return cudaGetLastError();
 }
 

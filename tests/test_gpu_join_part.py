@@ -168,3 +168,12 @@ def test_quantile_choice_matches_learned_choice(gpu, s):
     pf.close()
     bf.close()
     assert chose_l == chose_q
+
+
+@pytest.mark.parametrize("bits,npb", [(1, 1), (5, 33), (6, 5_000), (11, 40_000), (12, 700_001)])
+def test_partition_placement_sizes(gpu, bits, npb):
+    """Placement over fewer partitions than one CTA's 32, over partition counts that are not a
+    multiple of 1024, and over chunk counts that do not divide by 32."""
+    data = _skewed(6, 3_000, npb)
+    got, _ = _join(*data, strategy=omg.JOIN_HASH_PARTITIONED, bits=bits)
+    assert got == _expected(*data)
