@@ -18,6 +18,7 @@
 
 #include "host/gpu_runtime.h"
 #include "host/sizer.h"
+#include "kernels/agg_radix.h"
 #include "kernels/launch.h"
 
 namespace omniruntime {
@@ -794,10 +795,15 @@ struct HashAggregationOperator::Impl {
     omg::KernelTimer timer;
     DevArray<uint64_t> slots;
     DevArray<uint32_t> special;
-    // stats[0] = groupCount, [1] = nRetry, [2] = nSpill, [3] = error
+    // stats[0] = groupCount, [1] = nRetry, [2] = nSpill, [3] = error; radix aggregation: [4] = groups
+    // appended to `dense`, [5] = unit counter
     DevArray<unsigned long long> stats;
     uint64_t capacity = 0;
-    uint64_t groups = 0;
+    uint64_t groups = 0;  // in the table
+    // Finished groups of a radix aggregation (slots without free ones between them, in no hash
+    // order), beside the table.
+    DevArray<uint64_t> dense;
+    uint64_t denseGroups = 0;
     // Batches kept for the ordered sticky-overflow path (order-dependent plans only).
     std::vector<VectorBatch *> retained;
     // Sizing, decided at the first flush: the sketch of a row sample, the group estimate used,
@@ -1029,7 +1035,7 @@ int32_t HashAggregationOperator::GetSizingLog(int64_t *out, int32_t n) const
     }
     v.push_back(static_cast<int64_t>(im.estimate));
     v.push_back(im.partBits);
-    v.push_back(static_cast<int64_t>(std::max<uint64_t>(im.groups, uniqueKeys_)));
+    v.push_back(static_cast<int64_t>(std::max<uint64_t>(im.groups + im.denseGroups, uniqueKeys_)));
     v.push_back(static_cast<int64_t>(im.plainEstimate));
     v.push_back(im.learned ? 1 : 0);
     v.push_back(strategy_ == 1 ? 1 : 0);
@@ -1157,6 +1163,185 @@ void HashAggregationOperator::Partition(omg::BatchTable &bt, omg::AggLaunch &p, 
     p.nTiles = a.maxTiles;
     p.nParts = nParts;
     p.partTileStart = pb.tileStart.Get();
+}
+
+// One radix aggregation (kernels/agg_radix.cu): its record layout, partitions and buffers.
+struct HashAggregationOperator::RadixRun {
+    omg::RecLayout layout;
+    int32_t bits = 0;
+    int32_t passBits = 0;
+    int32_t indexSize = 0;
+    std::vector<omg::RadixUnit> units;
+    uint64_t denseCap = 0;
+    uint64_t tableGroups = 0;  // groups expected in the table: those of multi units
+    uint64_t spillCap = 0;     // slots that the multi units could merge
+    DevArray<unsigned int> cursor;
+    DevArray<omg::RadixUnit> dUnits;
+    DevArray<uint64_t> records;
+    DevArray<uint64_t> dense;
+};
+
+namespace {
+// Rows of a unit, and of the largest partition that is one unit: a hot key's partition is spread over
+// several CTAs, and the merge of a unit's table (some thousand slots) stays small beside its rows.
+constexpr uint64_t kRadixUnitRows = 1 << 14;
+constexpr uint64_t kRadixWholeRows = 1 << 15;
+// Target fill of a unit's slots: the partitions' group counts vary by a few percent, and the estimate by
+// 1.6 (one standard error of 2^12 registers); groups beyond the slots go to the global table.
+constexpr double kRadixLoad = 0.85;
+
+// The record of the inputs: widest first, then a byte per nullable input.  False: too wide.
+bool LayoutRecord(const AggPlan &plan, const omg::BatchTable &bt, omg::RecLayout &l)
+{
+    std::memset(&l, 0, sizeof(l));
+    l.nInputs = static_cast<int32_t>(plan.inputCols.size());
+    int at = 0;
+    auto add = [&](int input, int width, int half) {
+        if (at + std::max(width, 1) > omg::kMaxRecWords * 8 || l.nSrc >= omg::kMaxRecSrc) {
+            return false;
+        }
+        l.src[l.nSrc++] = omg::RecSrc{static_cast<int8_t>(input), static_cast<int8_t>(width), static_cast<int8_t>(half),
+            static_cast<int8_t>(at / 8), static_cast<int8_t>(at % 8 * 8)};
+        at += std::max(width, 1);
+        return true;
+    };
+    for (int width : {16, 8, 4, 2, 1}) {
+        for (int i = 0; i < l.nInputs; ++i) {
+            if (plan.inputWidths[i] != width) {
+                continue;
+            }
+            l.off[i] = static_cast<int16_t>(at);
+            l.width[i] = static_cast<int16_t>(width <= 8 ? width : 0);
+            if (width == 16 ? !(add(i, 8, 0) && add(i, 8, 1)) : !add(i, width, -1)) {
+                return false;
+            }
+        }
+    }
+    for (int i = 0; i < l.nInputs; ++i) {
+        l.nullOff[i] = bt.AnyNulls(i) ? static_cast<int16_t>(at) : int16_t(-1);
+        if (bt.AnyNulls(i) && !add(i, 0, -1)) {
+            return false;
+        }
+    }
+    l.words = std::max(1, (at + 7) / 8);
+    if (l.words > 2) {
+        l.words = (l.words + 3) / 4 * 4;  // stored 32 bytes at a time
+    }
+    return true;
+}
+}  // namespace
+
+// The key pass and what follows from it: how many partitions, their records and units, and every
+// buffer of the run.  False (nothing changed): the plan's rows do not fit a record, there are more
+// groups than the passes hold, or the device has no memory for the records.
+bool HashAggregationOperator::PlanRadix(omg::BatchTable &bt, RadixRun &run, cudaStream_t s)
+{
+    Impl &im = *impl_;
+    const uint64_t rows = static_cast<uint64_t>(bt.TotalRows());
+    const int32_t nSlots = omg::AggRadixSlots(plan_.slotWords, &run.indexSize);
+    if (nSlots < 64 || rows >= (uint64_t(1) << 32) || !LayoutRecord(plan_, bt, run.layout)) {
+        return false;
+    }
+    constexpr size_t kWords = omg::kRadixFineParts + omg::kRadixHllRegs;
+    omg::PinnedArray<unsigned int> h(kWords);
+    try {
+        DevArray<unsigned int> counts(kWords, s, true);
+        omg::AggLaunch p = MakeLaunch(plan_, nullptr, 0, nullptr, nullptr);
+        p.batches = bt.DeviceBatches();
+        p.tiles = bt.DeviceTiles();
+        p.nTiles = bt.NumTiles();
+        CudaCheck(omg::LaunchRadixKeys(p, counts.Get(), counts.Get() + omg::kRadixFineParts, s), "radix key pass");
+        ++counters_[0];
+        CudaCheck(cudaMemcpyAsync(h.Get(), counts.Get(), sizeof(unsigned int) * kWords, cudaMemcpyDeviceToHost, s),
+            "read partition counts");
+        im.stream.Sync();
+        const double groups = omg::HllDistinct(h.Get() + omg::kRadixFineParts, omg::kRadixHllRegs);
+        const uint64_t tables = NextPow2(static_cast<uint64_t>(std::ceil(groups / (kRadixLoad * nSlots))));
+        while (run.bits < omg::kRadixFineBits && (uint64_t(1) << run.bits) < tables) {
+            ++run.bits;
+        }
+        while ((uint64_t(1) << (run.bits + run.passBits)) < tables) {
+            if (++run.passBits > omg::kRadixMaxPassBits) {
+                return false;
+            }
+        }
+        const uint32_t nParts = 1u << run.bits;
+        const uint32_t fine = omg::kRadixFineParts >> run.bits;
+        const uint64_t unitSlots = static_cast<uint64_t>(nSlots) << run.passBits;
+        std::vector<unsigned int> start(nParts);
+        std::vector<omg::RadixUnit> whole;
+        uint64_t first = 0;
+        uint64_t multi = 0;
+        for (uint32_t q = 0; q < nParts; ++q) {
+            uint64_t n = 0;
+            for (uint32_t f = q * fine; f < (q + 1) * fine; ++f) {
+                n += h[f];
+            }
+            start[q] = static_cast<unsigned int>(first);
+            if (n > kRadixWholeRows) {
+                ++multi;
+                for (uint64_t r = 0; r < n; r += kRadixUnitRows) {
+                    const uint64_t m = std::min(kRadixUnitRows, n - r);
+                    run.units.push_back(omg::RadixUnit{static_cast<uint32_t>(first + r), static_cast<uint32_t>(m), 1, 0});
+                    run.spillCap += std::min(m, unitSlots);
+                }
+            } else if (n > 0) {
+                whole.push_back(omg::RadixUnit{static_cast<uint32_t>(first), static_cast<uint32_t>(n), 0, 0});
+                run.denseCap += std::min(n, unitSlots);
+            }
+            first += n;
+        }
+        run.units.insert(run.units.end(), whole.begin(), whole.end());
+        run.tableGroups = static_cast<uint64_t>(1.1 * groups / nParts * static_cast<double>(multi)) + 64;
+        run.cursor.Reset(nParts, s);
+        CudaCheck(cudaMemcpyAsync(run.cursor.Get(), start.data(), sizeof(unsigned int) * nParts, cudaMemcpyHostToDevice,
+                      s),
+            "upload partition starts");
+        run.dUnits.Reset(run.units.size(), s);
+        CudaCheck(cudaMemcpyAsync(run.dUnits.Get(), run.units.data(), sizeof(omg::RadixUnit) * run.units.size(),
+                      cudaMemcpyHostToDevice, s),
+            "upload radix units");
+        run.records.Reset(rows * run.layout.words + 2, s);
+        run.dense.Reset(std::max<uint64_t>(run.denseCap, 1) * plan_.slotWords, s);
+        if (2 * static_cast<uint64_t>(groups) > NextPow2(2 * im.estimate)) {
+            ++counters_[1];  // the estimate would have undersized the table: resized by the key pass
+        }
+    } catch (const OmniException &e) {
+        if (e.GetCode() != "MEM_CAP_EXCEEDED") {
+            throw;
+        }
+        return false;
+    }
+    return true;
+}
+
+// Move the dense groups into the table, grown to hold them, for more input or an ordered replay.
+void HashAggregationOperator::FoldDense(cudaStream_t s)
+{
+    Impl &im = *impl_;
+    if (im.denseGroups == 0) {
+        return;
+    }
+    const uint64_t all = im.groups + im.denseGroups;
+    const uint64_t need = NextPow2(std::max<uint64_t>(im.capacity, 4 * all));
+    DevArray<uint64_t> newSlots((need + 2) * plan_.slotWords, s);
+    DevArray<uint32_t> newSpecial(2, s, true);
+    DevArray<uint32_t> noSpecial(2, s, true);
+    omg::AggLaunch to = MakeLaunch(plan_, newSlots.Get(), need, newSpecial.Get(), im.stats.Get());
+    CudaCheck(omg::LaunchAggInitTable(to, s), "init grown table");
+    omg::AggLaunch from = MakeLaunch(plan_, im.slots.Get(), im.capacity, im.special.Get(), im.stats.Get());
+    CudaCheck(omg::LaunchAggRehash(to, from.table, to.table, s), "rehash");
+    omg::AggLaunch dense = MakeLaunch(plan_, im.dense.Get(), im.denseGroups, noSpecial.Get(), im.stats.Get());
+    CudaCheck(omg::LaunchAggRehash(to, dense.table, to.table, s), "rehash dense groups");
+    const unsigned long long count = all;
+    CudaCheck(cudaMemcpyAsync(im.stats.Get(), &count, sizeof(count), cudaMemcpyHostToDevice, s), "group count");
+    im.stream.Sync();
+    im.slots = newSlots;
+    im.special = newSpecial;
+    im.capacity = need;
+    im.groups = all;
+    im.denseGroups = 0;
+    im.dense.Release();
 }
 
 namespace {
@@ -1314,9 +1499,17 @@ void HashAggregationOperator::Flush()
     if (!im.decided) {
         Decide(bt, s);
     }
+    FoldDense(s);
+    // More groups than the partitions of the partitioned strategy hold: the radix aggregation, on the
+    // operator's first rows (later ones go to the table).  The line is where the estimate leaves the
+    // partitioned strategy; the global table it replaces there was behind at every size measured.
+    RadixRun radixRun;
+    const bool radix = strategy_ == 0 && im.capacity == 0 && im.partBits < 0 && im.estimate > 0 &&
+        rows >= kSketchMinRows && PlanRadix(bt, radixRun, s);
     // Create the table on first use, sized for the group estimate (load factor <= 1/2).
     if (im.capacity == 0) {
-        uint64_t cap = im.estimate > 0 ? NextPow2(im.estimate * 2) : kDefaultCapacity;
+        uint64_t cap = radix ? NextPow2(radixRun.tableGroups * 2)
+                             : (im.estimate > 0 ? NextPow2(im.estimate * 2) : kDefaultCapacity);
         cap = std::max<uint64_t>(cap, 1024);
         im.slots.Reset((cap + 2) * plan_.slotWords, s);
         im.special.Reset(2, s, true);
@@ -1350,20 +1543,39 @@ void HashAggregationOperator::Flush()
         Partition(bt, p, part, s);
         rowBatches = p.batches;
     }
-    const size_t spillCap = static_cast<size_t>(smemSlots) * maxGrid;
+    const size_t spillCap = radix ? radixRun.spillCap : static_cast<size_t>(smemSlots) * maxGrid;
     DevArray<uint64_t> spillA(std::max<size_t>(spillCap, 1) * plan_.slotWords, s);
     DevArray<uint64_t> spillB;
-    CudaCheck(cudaMemsetAsync(im.stats.Get() + 1, 0, 3 * sizeof(unsigned long long), s), "reset stats");
+    CudaCheck(cudaMemsetAsync(im.stats.Get() + 1, 0, 5 * sizeof(unsigned long long), s), "reset stats");
     p.retry = retryA.Get();
     p.retryCap = static_cast<uint32_t>(rows);
     p.smemSlots = smemSlots;
     unsigned int *nSpill = reinterpret_cast<unsigned int *>(im.stats.Get() + 2);
     im.timer.Start(s);
-    CudaCheck(omg::LaunchAgg(p, spillA.Get(), nSpill, static_cast<uint32_t>(spillCap), nullptr, 0, grid, s),
-        "aggregation kernel");
+    if (radix) {
+        CudaCheck(omg::LaunchRadixScatter(p, radixRun.layout, radixRun.bits, radixRun.cursor.Get(),
+                      radixRun.records.Get(), s),
+            "radix scatter");
+        omg::RadixAgg ra;
+        ra.records = radixRun.records.Get();
+        ra.units = radixRun.dUnits.Get();
+        ra.nUnits = static_cast<int32_t>(radixRun.units.size());
+        ra.passBits = radixRun.passBits;
+        ra.next = reinterpret_cast<unsigned int *>(im.stats.Get() + 5);
+        ra.dense = radixRun.dense.Get();
+        ra.denseCount = im.stats.Get() + 4;
+        ra.denseCap = radixRun.denseCap;
+        p.smemSlots = omg::AggRadixSlots(plan_.slotWords, &ra.indexSize);
+        CudaCheck(omg::LaunchRadixAgg(p, radixRun.layout, ra, spillA.Get(), nSpill, static_cast<uint32_t>(spillCap), s),
+            "radix aggregation");
+        ++counters_[0];
+    } else {
+        CudaCheck(omg::LaunchAgg(p, spillA.Get(), nSpill, static_cast<uint32_t>(spillCap), nullptr, 0, grid, s),
+            "aggregation kernel");
+    }
     im.timer.Stop(s);
     ++counters_[0];
-    unsigned long long h[4];
+    unsigned long long h[5];
     CudaCheck(cudaMemcpyAsync(h, im.stats.Get(), sizeof(h), cudaMemcpyDeviceToHost, s), "read stats");
     im.stream.Sync();
     counters_[6] += im.timer.ElapsedNs();
@@ -1376,6 +1588,10 @@ void HashAggregationOperator::Flush()
             err == 7 ? -7 : -9);
     }
     im.groups = h[0];
+    if (radix) {
+        im.dense = radixRun.dense;
+        im.denseGroups = h[4];
+    }
     // Exact resize path: grow the table and re-run the rows (and partial states) that could
     // not be placed.  Each round at least doubles the capacity.
     while (nRetry > 0 || nSpillH > 0) {
@@ -1402,8 +1618,11 @@ void HashAggregationOperator::Flush()
         r.retryIn = retryA.Get();
         r.nRetryIn = static_cast<uint32_t>(nRetry);
         const int rgrid = static_cast<int>(std::min<uint64_t>((nRetry + nSpillH + 511) / 512 + 1, sms * 8ull));
-        CudaCheck(omg::LaunchAgg(r, spillB.Get(), nSpill, static_cast<uint32_t>(std::max<uint64_t>(nSpillH, 1)),
-                      spillA.Get(), static_cast<uint32_t>(nSpillH), rgrid, s),
+        CudaCheck(radix ? omg::LaunchRadixRetry(r, radixRun.layout, radixRun.records.Get(), spillB.Get(), nSpill,
+                              static_cast<uint32_t>(std::max<uint64_t>(nSpillH, 1)), spillA.Get(),
+                              static_cast<uint32_t>(nSpillH), rgrid, s)
+                        : omg::LaunchAgg(r, spillB.Get(), nSpill, static_cast<uint32_t>(std::max<uint64_t>(nSpillH, 1)),
+                              spillA.Get(), static_cast<uint32_t>(nSpillH), rgrid, s),
             "aggregation retry kernel");
         ++counters_[0];
         CudaCheck(cudaMemcpyAsync(h, im.stats.Get(), sizeof(h), cudaMemcpyDeviceToHost, s), "read stats");
@@ -1433,7 +1652,7 @@ void HashAggregationOperator::Flush()
         ++counters_[1];
         im.stream.Sync();
     }
-    counters_[3] = static_cast<int64_t>(im.groups);
+    counters_[3] = static_cast<int64_t>(im.groups + im.denseGroups);
     if (!plan_.orderDependent) {
         im.keptIds.clear();  // freed stream-ordered, after the kernels that read them
     }
@@ -1792,6 +2011,7 @@ void HashAggregationOperator::Extract()
     unsigned long long nGroups = 0;
     CudaCheck(cudaMemcpyAsync(&nGroups, cnt.Get(), sizeof(nGroups), cudaMemcpyDeviceToHost, s), "read group count");
     im.stream.Sync();
+    nGroups += im.denseGroups;
     uniqueKeys_ = nGroups;
     counters_[3] = static_cast<int64_t>(nGroups);
     if (nGroups == 0) {
@@ -1840,9 +2060,31 @@ void HashAggregationOperator::Extract()
     e.ambiguousCap = ambCap;
     CudaCheck(omg::LaunchAggExtract(e, s), "extract groups");
     ++counters_[0];
+    DevArray<uint32_t> noSpecial;
+    if (im.denseGroups > 0) {
+        noSpecial.Reset(2, s, true);
+        omg::AggExtract d = e;
+        d.table = MakeLaunch(plan_, im.dense.Get(), im.denseGroups, noSpecial.Get(), im.stats.Get()).table;
+        CudaCheck(omg::LaunchAggExtract(d, s), "extract dense groups");
+        ++counters_[0];
+    }
     unsigned long long hc[4];
     CudaCheck(cudaMemcpyAsync(hc, cnt.Get(), sizeof(hc), cudaMemcpyDeviceToHost, s), "read extract counters");
     im.stream.Sync();
+    if (hc[2] > 0 && im.denseGroups > 0) {
+        // The ordered replay finds its groups in the table: everything into the table, and again.
+        FoldDense(s);
+        base = MakeLaunch(plan_, im.slots.Get(), im.capacity, im.special.Get(), im.stats.Get());
+        e.table = base.table;
+        for (size_t o = 0; o < nOut; ++o) {
+            CudaCheck(cudaMemsetAsync(cols[o].nulls->Data(), 0, cols[o].nulls->Bytes(), s), "reset nulls");
+        }
+        CudaCheck(cudaMemsetAsync(cnt.Get(), 0, 4 * sizeof(unsigned long long), s), "reset counters");
+        CudaCheck(omg::LaunchAggExtract(e, s), "extract groups");
+        ++counters_[0];
+        CudaCheck(cudaMemcpyAsync(hc, cnt.Get(), sizeof(hc), cudaMemcpyDeviceToHost, s), "read extract counters");
+        im.stream.Sync();
+    }
     if (hc[2] > 0) {
         // Some groups' sticky-overflow outcome depends on row order: replay those groups in
         // arrival order over the retained batches, then extract again with the answers.

@@ -40,12 +40,12 @@ struct SplitMix {
 };
 }  // namespace
 
-uint64_t HllGroupEstimate(const unsigned int *regs, int64_t rows)
+double HllDistinct(const unsigned int *regs, int n)
 {
-    const double m = static_cast<double>(kHllRegs);
+    const double m = static_cast<double>(n);
     double z = 0.0;
     int64_t zeros = 0;
-    for (int i = 0; i < kHllRegs; ++i) {
+    for (int i = 0; i < n; ++i) {
         z += std::ldexp(1.0, -static_cast<int>(regs[i]));
         zeros += regs[i] == 0 ? 1 : 0;
     }
@@ -54,6 +54,12 @@ uint64_t HllGroupEstimate(const unsigned int *regs, int64_t rows)
     if (e <= 2.5 * m && zeros > 0) {
         e = m * std::log(m / static_cast<double>(zeros));
     }
+    return e;
+}
+
+uint64_t HllGroupEstimate(const unsigned int *regs, int64_t rows)
+{
+    double e = HllDistinct(regs, kHllRegs);
     e += static_cast<double>(regs[kHllRegs] + regs[kHllRegs + 1]);
     const double capped = std::min(std::max(e, 1.0), static_cast<double>(std::max<int64_t>(rows, 1)));
     return static_cast<uint64_t>(std::llround(capped));

@@ -21,6 +21,8 @@ uint64_t PlainGroupEstimate(const unsigned long long *sketch, int64_t rows);
 // al. 2007: alpha_m m^2 / sum 2^-M[j], with linear counting m ln(m / V) below 2.5 m when V
 // registers are zero); at most `rows`.
 uint64_t HllGroupEstimate(const unsigned int *regs, int64_t rows);
+// The same estimate from n registers, uncapped and without special keys.
+double HllDistinct(const unsigned int *regs, int n);
 
 // Features of a sizing record (the layout written by HashAggregationOperator::GetSizingLog):
 // scale-free functions of the rows N, the sampled rows n, the distinct hashes d of the sample,

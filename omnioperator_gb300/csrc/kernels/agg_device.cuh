@@ -21,19 +21,49 @@ struct RowKey {
     int special;    // -1 normal, kNullSlotOffset / kSentinelSlotOffset for the special groups
 };
 
-__device__ __forceinline__ RowKey ReadKey(const KeySpec &ks, const BatchDesc &b, int64_t row, int kind)
+__device__ __forceinline__ void OrKeyWord(RowKey &k, int i, uint64_t v)
+{
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        k.w[j] |= j == i ? v : 0ull;
+    }
+}
+
+__device__ __forceinline__ uint64_t KeyWordsHash(const RowKey &k, int words)
+{
+    uint64_t h = 0x9e3779b97f4a7c15ull;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        h = j < words ? Mix64(h ^ k.w[j]) : h;
+    }
+    return h;
+}
+
+// Where a row's inputs are read from: row `row` of a batch's columns.
+struct BatchRow {
+    const BatchDesc &b;
+    int64_t row;
+    __device__ __forceinline__ bool Null(int input) const { return NullRO(b.nulls[input], row); }
+    __device__ __forceinline__ uint64_t Bits(int input, int width) const { return LoadBitsRO(b.cols[input], row, width); }
+    __device__ __forceinline__ const uint64_t *Wide(int input) const
+    {
+        return static_cast<const uint64_t *>(b.cols[input]) + 2 * row;
+    }
+};
+
+template <class Row> __device__ __forceinline__ RowKey ReadKeyOf(const KeySpec &ks, const Row &src, int kind)
 {
     RowKey k;
     k.w[0] = k.w[1] = k.w[2] = 0;
     k.special = -1;
     if (kind == KEY_SINGLE) {
         const KeyCol &c = ks.cols[0];
-        if (NullRO(b.nulls[c.input], row)) {
+        if (src.Null(c.input)) {
             k.special = kNullSlotOffset;
             k.hash = 0;
             return k;
         }
-        uint64_t v = static_cast<uint64_t>(SignExtend(LoadBitsRO(b.cols[c.input], row, c.width), c.width));
+        uint64_t v = static_cast<uint64_t>(SignExtend(src.Bits(c.input, c.width), c.width));
         k.w[0] = v;
         if (v == kEmptyKey) {
             k.special = kSentinelSlotOffset;
@@ -41,30 +71,170 @@ __device__ __forceinline__ RowKey ReadKey(const KeySpec &ks, const BatchDesc &b,
         k.hash = Mix64(v);
         return k;
     }
+    // The loops are unrolled over constant word indices, so the words stay in registers.
     uint32_t mask = 0;
-    for (int ci = 0; ci < ks.nCols; ++ci) {
+#pragma unroll
+    for (int ci = 0; ci < kMaxKeyCols; ++ci) {
+        if (ci >= ks.nCols) {
+            break;
+        }
         const KeyCol &c = ks.cols[ci];
-        if (NullRO(b.nulls[c.input], row)) {
+        if (src.Null(c.input)) {
             mask |= 1u << ci;
             continue;
         }
         const int wi = c.byteOffset >> 3;
         const int sh = (c.byteOffset & 7) * 8;
+        uint64_t lo, hi = 0;
         if (c.width == 16) {
-            const uint64_t *p = static_cast<const uint64_t *>(b.cols[c.input]) + 2 * row;
-            k.w[wi] = p[0];
-            k.w[wi + 1] = p[1];
+            const uint64_t *p = src.Wide(c.input);
+            lo = p[0];
+            hi = p[1];
         } else {
-            k.w[wi] |= LoadBitsRO(b.cols[c.input], row, c.width) << sh;
+            lo = src.Bits(c.input, c.width) << sh;
+        }
+        OrKeyWord(k, wi, lo);
+        OrKeyWord(k, wi + 1, hi);
+    }
+    OrKeyWord(k, ks.maskByte >> 3, static_cast<uint64_t>(mask) << ((ks.maskByte & 7) * 8));
+    k.hash = KeyWordsHash(k, ks.words);
+    return k;
+}
+
+__device__ __forceinline__ RowKey ReadKey(const KeySpec &ks, const BatchDesc &b, int64_t row, int kind)
+{
+    return ReadKeyOf(ks, BatchRow{b, row}, kind);
+}
+
+// ---- several rows at once
+// A load is only in flight with another row's if nothing between them waits for it or branches on it, so
+// the loads of a value of N rows come first, under one branch on its width, and what uses them after.
+// at(j): the address of row j's value; bit j of `use`: row j exists.
+template <int N, class At>
+__device__ __forceinline__ void LoadBitsRows(At at, int width, uint32_t use, uint64_t (&v)[N])
+{
+    switch (width) {
+        case 1:
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                v[j] = ((use >> j) & 1u) != 0 ? __ldg(reinterpret_cast<const unsigned char *>(at(j))) : 0;
+            }
+            break;
+        case 2:
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                v[j] = ((use >> j) & 1u) != 0 ? __ldg(reinterpret_cast<const unsigned short *>(at(j))) : 0;
+            }
+            break;
+        case 4:
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                v[j] = ((use >> j) & 1u) != 0 ? __ldg(reinterpret_cast<const unsigned int *>(at(j))) : 0;
+            }
+            break;
+        default:
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                v[j] = ((use >> j) & 1u) != 0 ? __ldg(reinterpret_cast<const unsigned long long *>(at(j))) : 0;
+            }
+            break;
+    }
+}
+
+// Rows row0 + j * kStep of a batch.
+template <int kStep> struct BatchRows {
+    const BatchDesc &b;
+    int64_t row0;
+    __device__ __forceinline__ const char *At(int input, int width, int j) const
+    {
+        return static_cast<const char *>(b.cols[input]) + (row0 + j * kStep) * width;
+    }
+    __device__ __forceinline__ bool Nullable(int input) const { return b.nulls[input] != nullptr; }
+    template <int N> __device__ __forceinline__ uint32_t Nulls(int input, uint32_t use) const
+    {
+        const unsigned char *nulls = reinterpret_cast<const unsigned char *>(b.nulls[input]);
+        unsigned int byte[N];
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            byte[j] = ((use >> j) & 1u) != 0 ? __ldg(nulls + ((row0 + j * kStep) >> 3)) : 0u;
+        }
+        uint32_t m = 0;
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            m |= ((byte[j] >> ((row0 + j * kStep) & 7)) & 1u) << j;
+        }
+        return m;
+    }
+};
+
+// ReadKey of N rows (bit j of `use`; the others' keys are meaningless).
+template <int kKind, int N, class Rows>
+__device__ __forceinline__ void ReadKeys(const KeySpec &ks, const Rows &rows, uint32_t use, RowKey (&k)[N])
+{
+    if constexpr (kKind == KEY_SINGLE) {
+        const KeyCol &c = ks.cols[0];
+        uint64_t raw[N];
+        LoadBitsRows<N>([&](int j) { return rows.At(c.input, c.width, j); }, c.width, use, raw);
+        const uint32_t null = rows.Nullable(c.input) ? rows.template Nulls<N>(c.input, use) : 0u;
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const uint64_t v = static_cast<uint64_t>(SignExtend(raw[j], c.width));
+            const bool isNull = ((null >> j) & 1u) != 0;
+            k[j].w[0] = isNull ? 0ull : v;
+            k[j].w[1] = k[j].w[2] = 0;
+            k[j].special = isNull ? kNullSlotOffset : (v == kEmptyKey ? kSentinelSlotOffset : -1);
+            k[j].hash = isNull ? 0ull : Mix64(v);
+        }
+    } else {
+        // Two columns at a time: both columns' loads are in flight together.
+        uint32_t nulls[N];
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            k[j].w[0] = k[j].w[1] = k[j].w[2] = 0;
+            k[j].special = -1;
+            nulls[j] = 0;
+        }
+        for (int c0 = 0; c0 < ks.nCols; c0 += 2) {
+            uint64_t raw[2][N];
+            uint32_t null[2] = {0, 0};
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                if (c0 + i < ks.nCols) {
+                    const KeyCol &c = ks.cols[c0 + i];
+                    LoadBitsRows<N>([&](int j) { return rows.At(c.input, c.width, j); }, c.width, use, raw[i]);
+                    null[i] = rows.Nullable(c.input) ? rows.template Nulls<N>(c.input, use) : 0u;
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                if (c0 + i >= ks.nCols) {
+                    break;
+                }
+                const KeyCol &c = ks.cols[c0 + i];
+                const int wi = c.byteOffset >> 3;
+                const int sh = (c.byteOffset & 7) * 8;
+                if (c.width == 16) {
+                    uint64_t hi[N];
+                    LoadBitsRows<N>([&](int j) { return rows.At(c.input, c.width, j) + 8; }, 8, use & ~null[i], hi);
+#pragma unroll
+                    for (int j = 0; j < N; ++j) {
+                        OrKeyWord(k[j], wi + 1, hi[j]);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < N; ++j) {
+                    const bool isNull = ((null[i] >> j) & 1u) != 0;
+                    OrKeyWord(k[j], wi, isNull ? 0ull : raw[i][j] << sh);
+                    nulls[j] |= (isNull ? 1u : 0u) << (c0 + i);
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            OrKeyWord(k[j], ks.maskByte >> 3, static_cast<uint64_t>(nulls[j]) << ((ks.maskByte & 7) * 8));
+            k[j].hash = KeyWordsHash(k[j], ks.words);
         }
     }
-    k.w[ks.maskByte >> 3] |= static_cast<uint64_t>(mask) << ((ks.maskByte & 7) * 8);
-    uint64_t h = 0x9e3779b97f4a7c15ull;
-    for (int i = 0; i < ks.words; ++i) {
-        h = Mix64(h ^ k.w[i]);
-    }
-    k.hash = h;
-    return k;
 }
 
 // Published tag of a packed slot: never 0 (free) or 1 (locked).
@@ -459,8 +629,11 @@ __device__ __forceinline__ int64_t GlobalFind(const AggTable &t, const KeySpec &
             unsigned long long prev =
                 atomicCAS(reinterpret_cast<unsigned long long *>(slot), 0ull, static_cast<unsigned long long>(kTagLocked));
             if (prev == 0) {
-                for (int j = 0; j < ks.words; ++j) {
-                    slot[1 + j] = k.w[j];
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    if (j < ks.words) {
+                        slot[1 + j] = k.w[j];
+                    }
                 }
                 StoreRelease(slot, tag);
                 *inserted = true;
@@ -480,8 +653,9 @@ __device__ __forceinline__ int64_t GlobalFind(const AggTable &t, const KeySpec &
         }
         if (cur == tag) {
             bool eq = true;
-            for (int j = 0; j < ks.words; ++j) {
-                eq = eq && (slot[1 + j] == k.w[j]);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                eq = eq && (j >= ks.words || slot[1 + j] == k.w[j]);
             }
             if (eq) {
                 return static_cast<int64_t>(i);
@@ -496,11 +670,11 @@ __device__ __forceinline__ int64_t GlobalFind(const AggTable &t, const KeySpec &
 // Same layout as the global table (slotWords words per slot), nSlots slots, no special
 // slots (those rows go straight to the global table).  Returns the slot or -1.
 __device__ __forceinline__ int SmemFind(uint64_t *sm, int nSlots, int slotWords, const KeySpec &ks, const RowKey &k,
-    int kind)
+    int kind, int maxProbe = kSmemProbe)
 {
     int i = static_cast<int>((static_cast<uint64_t>(static_cast<uint32_t>(k.hash >> 32)) * nSlots) >> 32);
     if (kind == KEY_SINGLE) {
-        for (int probe = 0; probe < kSmemProbe; ++probe) {
+        for (int probe = 0; probe < maxProbe; ++probe) {
             unsigned long long *kp = reinterpret_cast<unsigned long long *>(sm + static_cast<int64_t>(i) * slotWords);
             unsigned long long cur = *reinterpret_cast<volatile unsigned long long *>(kp);
             if (cur == k.w[0]) {
@@ -519,7 +693,7 @@ __device__ __forceinline__ int SmemFind(uint64_t *sm, int nSlots, int slotWords,
         return -1;
     }
     const uint64_t tag = PublishedTag(k.hash);
-    for (int probe = 0; probe < kSmemProbe; ++probe) {
+    for (int probe = 0; probe < maxProbe; ++probe) {
         uint64_t *slot = sm + static_cast<int64_t>(i) * slotWords;
         volatile uint64_t *vs = slot;
         uint64_t cur = vs[0];
@@ -527,8 +701,11 @@ __device__ __forceinline__ int SmemFind(uint64_t *sm, int nSlots, int slotWords,
             unsigned long long prev =
                 atomicCAS(reinterpret_cast<unsigned long long *>(slot), 0ull, static_cast<unsigned long long>(kTagLocked));
             if (prev == 0) {
-                for (int j = 0; j < ks.words; ++j) {
-                    vs[1 + j] = k.w[j];
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    if (j < ks.words) {
+                        vs[1 + j] = k.w[j];
+                    }
                 }
                 __threadfence_block();
                 vs[0] = tag;
@@ -547,8 +724,9 @@ __device__ __forceinline__ int SmemFind(uint64_t *sm, int nSlots, int slotWords,
         if (cur == tag) {
             __threadfence_block();
             bool eq = true;
-            for (int j = 0; j < ks.words; ++j) {
-                eq = eq && (vs[1 + j] == k.w[j]);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                eq = eq && (j >= ks.words || vs[1 + j] == k.w[j]);
             }
             if (eq) {
                 return i;
@@ -623,12 +801,11 @@ __device__ __forceinline__ void MergeRecord(const AggLaunch &p, const SpillArgs 
         k.w[0] = rec[0];
         k.hash = Mix64(k.w[0]);
     } else {
-        uint64_t h = 0x9e3779b97f4a7c15ull;
-        for (int i = 0; i < p.key.words; ++i) {
-            k.w[i] = rec[1 + i];
-            h = Mix64(h ^ k.w[i]);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            k.w[j] = j < p.key.words ? rec[1 + j] : 0ull;
         }
-        k.hash = h;
+        k.hash = KeyWordsHash(k, p.key.words);
     }
     bool inserted = false;
     int64_t g = GlobalFind(p.table, p.key, k, p.maxProbe, p.error, &inserted, p.waitBudget, kKind);

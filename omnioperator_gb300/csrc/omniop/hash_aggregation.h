@@ -144,8 +144,11 @@ public:
 private:
     struct Impl;
     struct PartBuffers;
+    struct RadixRun;
     void Decide(omg::BatchTable &bt, cudaStream_t s);
     void Partition(omg::BatchTable &bt, omg::AggLaunch &p, PartBuffers &pb, cudaStream_t s);
+    bool PlanRadix(omg::BatchTable &bt, RadixRun &run, cudaStream_t s);
+    void FoldDense(cudaStream_t s);
     void Flush();
     void EncodeStrings(omg::BatchTable &bt, cudaStream_t s);
     void BindStrings(omg::AggLaunch &p) const;
