@@ -303,11 +303,6 @@ constexpr int kRadixThreads = 512;
 constexpr int kRadixRows = 4;  // rows per thread per step
 constexpr int kStepRows = kRadixThreads * kRadixRows;
 constexpr size_t kRadixSmemBytes = 112 * 1024;  // two CTAs per SM
-constexpr int kSpecialSlots = 2;  // slots 0 and 1: the NULL and the EMPTY key
-constexpr unsigned int kIndexLocked = 0xffffffffu;
-constexpr unsigned int kIndexFull = 0xfffffffeu;
-
-__device__ __forceinline__ unsigned int *LowHalf(uint64_t *w) { return reinterpret_cast<unsigned int *>(w); }
 
 // A step: its records, where the thread's own rows (row k * kRadixThreads + threadIdx.x of the step) go in slot
 // order, and the exchange buffers.
@@ -404,17 +399,6 @@ __device__ __forceinline__ void AddWord(uint64_t *w, uint64_t v, bool shared)
     } else {
         *w += v;
     }
-}
-
-__device__ __forceinline__ double AsDouble(uint64_t bits, int inKind, int width)
-{
-    if (inKind == IN_DOUBLE) {
-        return __longlong_as_double(static_cast<long long>(bits));
-    }
-    if (inKind == IN_FLOAT) {
-        return static_cast<double>(__int_as_float(static_cast<int>(bits)));
-    }
-    return static_cast<double>(SignExtend(bits, width));
 }
 
 __device__ __forceinline__ void ApplyInt(const AccSpec &s, const Run &run, const uint64_t (&bits)[kRadixRows],
@@ -704,85 +688,6 @@ __device__ __noinline__ void GlobalRecord(const AggLaunch &p, const RecLayout &l
         }
     }
     UpdateStates(p, b, 0, in, p.table.slots + g * p.table.slotWords + p.table.keyWords);
-}
-
-__device__ __forceinline__ void InitSlot(const AggLaunch &p, uint64_t *slot)
-{
-    slot[0] = (p.key.kind == KEY_SINGLE) ? kEmptyKey : 0ull;
-    for (int j = 1; j < p.table.keyWords; ++j) {
-        slot[j] = 0;
-    }
-    InitStates(p.accs, p.nAccs, p.stateWords, slot + p.table.keyWords);
-}
-
-// The slot of key k among the groups (kSpecialSlots and up), taking a new one if need be, or -1: the
-// table is full (a key that once misses then misses every time: the entry it would take stays full).
-__device__ __forceinline__ int FindGroup(uint64_t *sm, unsigned int *index, unsigned int indexMask, unsigned int *used,
-    unsigned int nSlots, int sw, const KeySpec &ks, const RowKey &k, int kind)
-{
-    const unsigned int tag = static_cast<unsigned int>(k.hash >> 48) << 16;
-    unsigned int i = static_cast<unsigned int>(k.hash >> 32) & indexMask;
-    for (unsigned int probe = 0; probe <= indexMask; ++probe) {
-        volatile unsigned int *ve = index + i;
-        unsigned int e = *ve;
-        if (e == 0) {
-            e = atomicCAS(index + i, 0u, kIndexLocked);
-            if (e == 0) {
-                const unsigned int slot = atomicAdd(used, 1u);
-                if (slot >= nSlots) {
-                    *ve = kIndexFull;
-                    return -1;
-                }
-                volatile uint64_t *to = sm + static_cast<int64_t>(slot + kSpecialSlots) * sw;
-                if (kind == KEY_SINGLE) {
-                    to[0] = k.w[0];
-                } else {
-                    to[0] = PublishedTag(k.hash);
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) {
-                        if (j < ks.words) {
-                            to[1 + j] = k.w[j];
-                        }
-                    }
-                }
-                __threadfence_block();
-                *ve = tag | (slot + kSpecialSlots);
-                return static_cast<int>(slot + kSpecialSlots);
-            }
-        }
-        if (e == kIndexLocked) {
-            // Another thread is writing this entry's key: a handful of instructions, then it publishes.
-            int spins = 0;
-            while ((e = *ve) == kIndexLocked) {
-                if (++spins > (1 << 20)) {
-                    return -2;
-                }
-            }
-        }
-        if (e == kIndexFull) {
-            return -1;
-        }
-        if ((e & 0xffff0000u) == tag) {
-            __threadfence_block();
-            const int slot = static_cast<int>(e & 0xffffu);
-            const volatile uint64_t *at = sm + static_cast<int64_t>(slot) * sw;
-            bool eq;
-            if (kind == KEY_SINGLE) {
-                eq = at[0] == k.w[0];
-            } else {
-                eq = true;
-#pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    eq = eq && (j >= ks.words || at[1 + j] == k.w[j]);
-                }
-            }
-            if (eq) {
-                return slot;
-            }
-        }
-        i = (i + 1) & indexMask;
-    }
-    return -1;
 }
 
 // Exclusive scan of cnt[0, n) in place, by the whole CTA; returns the total.  Each slot's count is added
