@@ -25,15 +25,20 @@ void BatchTable::Build(const std::vector<VectorBatch *> &batches, const std::vec
     if (inputCols.size() > static_cast<size_t>(kMaxInputs)) {
         throw OmniException("UNSUPPORTED_ERROR", "too many input columns for one kernel", -2);
     }
-    descs_.Reset(batches.size());
     anyNulls_.assign(inputCols.size(), false);
     allDevice_.assign(inputCols.size(), true);
     size_t nTiles = 0;
     for (auto *b : batches) {
         nTiles += (static_cast<size_t>(b->GetRowCount()) + tileRows - 1) / tileRows;
     }
-    tiles_.Reset(nTiles);
-    tileOut_.Reset(nTiles);
+    nBatches_ = batches.size();
+    nTiles_ = nTiles;
+    tilesAt_ = sizeof(BatchDesc) * nBatches_;
+    tileOutAt_ = tilesAt_ + sizeof(TileDesc) * nTiles_;
+    host_.Reset(tileOutAt_ + sizeof(int64_t) * nTiles_);
+    descs_ = reinterpret_cast<BatchDesc *>(host_.Get());
+    tiles_ = reinterpret_cast<TileDesc *>(host_.Get() + tilesAt_);
+    tileOut_ = reinterpret_cast<int64_t *>(host_.Get() + tileOutAt_);
     totalRows_ = 0;
     size_t t = 0;
     for (size_t bi = 0; bi < batches.size(); ++bi) {
@@ -198,29 +203,19 @@ void BatchTable::Upload(cudaStream_t s)
         CudaCheck(LaunchMaskNulls(dMaskJobs_.Get(), static_cast<int32_t>(maskJobs_.size()), s), "mask NULL bitmaps");
         masksDone_ = true;
     }
-    dBatches_.Reset(std::max<size_t>(descs_.Size(), 1), s);
-    dTiles_.Reset(std::max<size_t>(tiles_.Size(), 1), s);
-    dTileOut_.Reset(std::max<size_t>(tileOut_.Size(), 1), s);
-    if (descs_.Size() > 0) {
-        CudaCheck(cudaMemcpyAsync(dBatches_.Get(), descs_.Get(), sizeof(BatchDesc) * descs_.Size(),
-                      cudaMemcpyHostToDevice, s),
-            "upload batch descriptors");
-    }
-    if (tiles_.Size() > 0) {
-        CudaCheck(cudaMemcpyAsync(dTiles_.Get(), tiles_.Get(), sizeof(TileDesc) * tiles_.Size(),
-                      cudaMemcpyHostToDevice, s),
-            "upload tile descriptors");
-        CudaCheck(cudaMemcpyAsync(dTileOut_.Get(), tileOut_.Get(), sizeof(int64_t) * tileOut_.Size(),
-                      cudaMemcpyHostToDevice, s),
-            "upload tile offsets");
+    const size_t bytes = tileOutAt_ + sizeof(int64_t) * nTiles_;
+    device_.Reset(bytes, s);
+    if (bytes > 0) {
+        CudaCheck(cudaMemcpyAsync(device_.Get(), host_.Get(), bytes, cudaMemcpyHostToDevice, s),
+            "upload batch and tile descriptors");
     }
 }
 
 std::vector<int64_t> BatchTable::RegionRows(int32_t nRegions) const
 {
     std::vector<int64_t> rows(static_cast<size_t>(nRegions > 0 ? nRegions : 1), 0);
-    const TileDesc *t = tiles_.Get();
-    for (size_t i = 0; i < tiles_.Size(); ++i) {
+    const TileDesc *t = tiles_;
+    for (size_t i = 0; i < nTiles_; ++i) {
         rows[i % rows.size()] += t[i].rows;
     }
     return rows;

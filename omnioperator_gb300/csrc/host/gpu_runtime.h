@@ -184,11 +184,11 @@ public:
     void SetInputNulls(size_t batch, int32_t input, const uint8_t *nulls) { descs_[batch].nulls[input] = nulls; }
     int64_t BatchRows(size_t batch) { return descs_[batch].rows; }
     int64_t BatchRowBase(size_t batch) { return descs_[batch].rowBase; }
-    size_t NumBatches() const { return descs_.Size(); }
-    const BatchDesc *DeviceBatches() const { return dBatches_.Get(); }
-    const TileDesc *DeviceTiles() const { return dTiles_.Get(); }
-    const int64_t *DeviceTileOutRows() const { return dTileOut_.Get(); }
-    int32_t NumTiles() const { return static_cast<int32_t>(tiles_.Size()); }
+    size_t NumBatches() const { return nBatches_; }
+    const BatchDesc *DeviceBatches() const { return reinterpret_cast<const BatchDesc *>(device_.Get()); }
+    const TileDesc *DeviceTiles() const { return reinterpret_cast<const TileDesc *>(device_.Get() + tilesAt_); }
+    const int64_t *DeviceTileOutRows() const { return reinterpret_cast<const int64_t *>(device_.Get() + tileOutAt_); }
+    int32_t NumTiles() const { return static_cast<int32_t>(nTiles_); }
     // Rows of the tiles t with t % nRegions == r, per r.
     std::vector<int64_t> RegionRows(int32_t nRegions) const;
     int64_t TotalRows() const { return totalRows_; }
@@ -212,12 +212,13 @@ private:
     DevArray<uint32_t> maskBits_;
     PinnedArray<MaskJob> hMaskJobs_;
     DevArray<MaskJob> dMaskJobs_;
-    PinnedArray<BatchDesc> descs_;
-    PinnedArray<TileDesc> tiles_;
-    PinnedArray<int64_t> tileOut_;
-    DevArray<BatchDesc> dBatches_;
-    DevArray<TileDesc> dTiles_;
-    DevArray<int64_t> dTileOut_;
+    // One block, so that one copy uploads it: the batch descriptors, the tiles, the tiles' output rows.
+    PinnedArray<char> host_;
+    DevArray<char> device_;
+    size_t nBatches_ = 0, nTiles_ = 0, tilesAt_ = 0, tileOutAt_ = 0;
+    BatchDesc *descs_ = nullptr;
+    TileDesc *tiles_ = nullptr;
+    int64_t *tileOut_ = nullptr;
     std::vector<bool> anyNulls_;
     std::vector<bool> allDevice_;
     int64_t totalRows_ = 0;

@@ -791,14 +791,34 @@ struct StringDict {
 };
 }  // namespace
 
+struct HashAggregationOperator::ExtractRun {
+    bool launched = false;
+    bool onHost = false;
+    std::vector<omg::OutColumn> cols;
+    omg::AggExtract e;
+};
+
+namespace {
+constexpr size_t kStatsWords = 16;
+constexpr size_t kExtractStats = 8;  // first of the extraction's words
+// Output columns of up to this many bytes for a host caller are written straight to pinned host memory
+// by the extraction, without a copy behind it.
+constexpr size_t kHostDirectBytes = size_t(4) << 20;
+// Tables of up to this many slots are extracted without waiting for the group count.
+constexpr uint64_t kAheadSlots = uint64_t(1) << 16;
+}  // namespace
+
 struct HashAggregationOperator::Impl {
     omg::OpStream stream;
     omg::KernelTimer timer;
     DevArray<uint64_t> slots;
     DevArray<uint32_t> special;
     // stats[0] = groupCount, [1] = nRetry, [2] = nSpill, [3] = error; radix aggregation: [4] = groups
-    // appended to `dense`, [5] = unit counter
+    // appended to `dense`, [5] = unit counter; extraction: [8] = rows, [9] = error, [10] = nAmbiguous
     DevArray<unsigned long long> stats;
+    omg::PinnedArray<unsigned long long> hostStats{kStatsWords};
+    // The extraction that a last flush launched behind its own kernels, valid unless rows were left over.
+    ExtractRun ahead;
     uint64_t capacity = 0;
     uint64_t groups = 0;  // in the table
     // Finished groups of a radix aggregation (slots without free ones between them, in no hash
@@ -1071,18 +1091,21 @@ void HashAggregationOperator::Decide(omg::BatchTable &bt, cudaStream_t s)
         im.plainEstimate = omg::HllGroupEstimate(h.data(), rows);
         im.estimate = im.plainEstimate;
     } else if (rows >= kSketchMinRows && (strategy_ == 0 || strategy_ == 3)) {
-        DevArray<unsigned long long> tabKeys(omg::kSketchCap, s);
-        DevArray<unsigned int> tabCounts(omg::kSketchCap, s);
-        DevArray<unsigned long long> st(omg::kSketchStats, s);
+        // The sketch's statistics, keys and counts, in one block.
+        DevArray<unsigned long long> sk(omg::kSketchStats + omg::kSketchCap + omg::kSketchCap / 2, s);
+        unsigned long long *tabKeys = sk.Get() + omg::kSketchStats;
+        unsigned int *tabCounts = reinterpret_cast<unsigned int *>(tabKeys + omg::kSketchCap);
+        omg::PinnedArray<unsigned long long> st(omg::kSketchStats);
         omg::AggLaunch p = MakeLaunch(plan_, nullptr, 0, nullptr, nullptr);
         p.batches = bt.DeviceBatches();
         p.tiles = bt.DeviceTiles();
         p.nTiles = bt.NumTiles();
         const int32_t n = static_cast<int32_t>(std::min<int64_t>(rows, kSketchSample));
-        CudaCheck(omg::LaunchAggSketch(p, n, tabKeys.Get(), tabCounts.Get(), st.Get(), s), "key sketch");
+        CudaCheck(omg::LaunchAggSketch(p, n, tabKeys, tabCounts, sk.Get(), s), "key sketch");
         ++counters_[0];
-        CudaCheck(cudaMemcpyAsync(im.sketch, st.Get(), sizeof(im.sketch), cudaMemcpyDeviceToHost, s), "read sketch");
+        CudaCheck(cudaMemcpyAsync(st.Get(), sk.Get(), sizeof(im.sketch), cudaMemcpyDeviceToHost, s), "read sketch");
         im.stream.Sync();
+        std::memcpy(im.sketch, st.Get(), sizeof(im.sketch));
         im.sketchRows = rows;
         im.plainEstimate = omg::PlainGroupEstimate(im.sketch, rows);
         im.estimate = im.plainEstimate;
@@ -1476,7 +1499,7 @@ void HashAggregationOperator::EncodeStrings(omg::BatchTable &bt, cudaStream_t s)
     }
 }
 
-void HashAggregationOperator::Flush()
+void HashAggregationOperator::Flush(bool last)
 {
     if (pending_.empty()) {
         return;
@@ -1487,8 +1510,9 @@ void HashAggregationOperator::Flush()
         im.stream.SetUser(userStream_);
     }
     cudaStream_t s = im.stream.Get();
-    if (im.stats.Get() == nullptr) {
-        im.stats.Reset(8, s, true);
+    const bool freshStats = im.stats.Get() == nullptr;
+    if (freshStats) {
+        im.stats.Reset(kStatsWords, s, true);
     }
     omg::BatchTable bt;
     bt.Build(pending_, plan_.inputCols, omg::kTileRows, &plan_.inputMasks);
@@ -1510,10 +1534,11 @@ void HashAggregationOperator::Flush()
     // Create the table on first use, sized for the group estimate (load factor <= 1/2).
     if (im.capacity == 0) {
         uint64_t cap = radix ? NextPow2(radixRun.tableGroups * 2)
-                             : (im.estimate > 0 ? NextPow2(im.estimate * 2) : kDefaultCapacity);
+                             : (im.estimate > 0 ? NextPow2(im.estimate * 2)
+                                                : std::min(kDefaultCapacity, NextPow2(static_cast<uint64_t>(rows) * 2)));
         cap = std::max<uint64_t>(cap, 1024);
         im.slots.Reset((cap + 2) * plan_.slotWords, s);
-        im.special.Reset(2, s, true);
+        im.special.Reset(2, s);
         im.capacity = cap;
         omg::AggLaunch init = MakeLaunch(plan_, im.slots.Get(), cap, im.special.Get(), im.stats.Get());
         CudaCheck(omg::LaunchAggInitTable(init, s), "init aggregation table");
@@ -1561,9 +1586,14 @@ void HashAggregationOperator::Flush()
     const size_t spillCap = radix ? radixRun.spillCap
                                   : (few ? static_cast<size_t>(fewLayout.maxGroups) * omg::LaunchAggFewGrid()
                                          : static_cast<size_t>(smemSlots) * maxGrid);
-    DevArray<uint64_t> spillA(std::max<size_t>(spillCap, 1) * plan_.slotWords, s);
+    DevArray<uint64_t> spillA;
+    if (spillCap > 0) {
+        spillA.Reset(spillCap * plan_.slotWords, s);
+    }
     DevArray<uint64_t> spillB;
-    CudaCheck(cudaMemsetAsync(im.stats.Get() + 1, 0, 5 * sizeof(unsigned long long), s), "reset stats");
+    if (!freshStats) {
+        CudaCheck(cudaMemsetAsync(im.stats.Get() + 1, 0, 5 * sizeof(unsigned long long), s), "reset stats");
+    }
     p.retry = retryA.Get();
     p.retryCap = static_cast<uint32_t>(rows);
     p.smemSlots = smemSlots;
@@ -1595,8 +1625,12 @@ void HashAggregationOperator::Flush()
     }
     im.timer.Stop(s);
     ++counters_[0];
-    unsigned long long h[5];
-    CudaCheck(cudaMemcpyAsync(h, im.stats.Get(), sizeof(h), cudaMemcpyDeviceToHost, s), "read stats");
+    if (last && im.capacity <= kAheadSlots && !radix && im.denseGroups == 0 && plan_.dictInputs.empty()) {
+        // The groups out, without waiting to hear how many there are: at most one per slot, or per row.
+        LaunchExtract(im.ahead, std::min<uint64_t>(im.capacity, im.groups + static_cast<uint64_t>(rows)) + 2, s);
+    }
+    unsigned long long *h = im.hostStats.Get();
+    CudaCheck(cudaMemcpyAsync(h, im.stats.Get(), kStatsWords * sizeof(*h), cudaMemcpyDeviceToHost, s), "read stats");
     im.stream.Sync();
     counters_[6] += im.timer.ElapsedNs();
     ++counters_[7];
@@ -1614,6 +1648,7 @@ void HashAggregationOperator::Flush()
     }
     // Exact resize path: grow the table and re-run the rows (and partial states) that could
     // not be placed.  Each round at least doubles the capacity.
+    im.ahead.launched = im.ahead.launched && nRetry == 0 && nSpillH == 0;
     while (nRetry > 0 || nSpillH > 0) {
         const uint64_t need = NextPow2(std::max<uint64_t>(im.capacity * 2, 2 * (im.groups + nRetry + nSpillH)));
         DevArray<uint64_t> newSlots((need + 2) * plan_.slotWords, s);
@@ -1645,7 +1680,7 @@ void HashAggregationOperator::Flush()
                               spillA.Get(), static_cast<uint32_t>(nSpillH), rgrid, s),
             "aggregation retry kernel");
         ++counters_[0];
-        CudaCheck(cudaMemcpyAsync(h, im.stats.Get(), sizeof(h), cudaMemcpyDeviceToHost, s), "read stats");
+        CudaCheck(cudaMemcpyAsync(h, im.stats.Get(), kStatsWords * sizeof(*h), cudaMemcpyDeviceToHost, s), "read stats");
         im.stream.Sync();
         std::swap(retryA, retryB);
         std::swap(spillA, spillB);
@@ -1658,7 +1693,7 @@ void HashAggregationOperator::Flush()
         }
     }
     // Keep the load factor under one half for the next batches (the reference grows x4).
-    if (im.groups * 2 > im.capacity) {
+    if (im.groups * 2 > im.capacity && !im.ahead.launched) {
         const uint64_t need = NextPow2(im.groups * 4);
         DevArray<uint64_t> newSlots((need + 2) * plan_.slotWords, s);
         DevArray<uint32_t> newSpecial(2, s, true);
@@ -1809,7 +1844,7 @@ bool HashAggregationOperator::ExtractSpilled()
     }
     cudaStream_t s = im.stream.Get();
     if (im.stats.Get() == nullptr) {
-        im.stats.Reset(8, s, true);
+        im.stats.Reset(kStatsWords, s, true);
     }
     const size_t slotBytes = static_cast<size_t>(plan_.slotWords) * sizeof(uint64_t);
     uint64_t estimate = 0;
@@ -2010,12 +2045,91 @@ bool HashAggregationOperator::ExtractSpilled()
     return true;
 }
 
+// Output columns for up to `bound` groups in one block, and the extraction of the table and the dense groups
+// into them.  Its counters are the words of stats from kExtractStats.
+void HashAggregationOperator::LaunchExtract(ExtractRun &x, uint64_t bound, cudaStream_t s)
+{
+    Impl &im = *impl_;
+    const size_t nOut = plan_.outs.size();
+    x.launched = true;
+    x.cols.assign(nOut, omg::OutColumn{});
+    auto up = [](size_t n) { return (n + 255) / 256 * 256; };
+    const size_t nullBytes = up(omg::NullBitmapBytes(static_cast<int64_t>(bound)));
+    size_t values = 0;
+    for (const OutSpec &os : plan_.outs) {
+        values += up(bound * os.outWidth + 16);
+    }
+    const size_t bytes = values + nOut * nullBytes;
+    x.onHost = !deviceOutput_ && plan_.dictInputs.empty() && bytes <= kHostDirectBytes;
+    omg::BufferPtr block = x.onHost ? omg::Buffer::NewHost(bytes, false) : omg::Buffer::NewDevice(bytes, s, false);
+    size_t at = 0;
+    for (size_t o = 0; o < nOut; ++o) {
+        const OutSpec &os = plan_.outs[o];
+        x.cols[o].type = plan_.outTypes[o]->GetId();
+        x.cols[o].width = os.outWidth;
+        x.cols[o].values = omg::Buffer::Slice(block, at, bound * os.outWidth + 16);
+        x.cols[o].nulls = omg::Buffer::Slice(block, values + o * nullBytes, nullBytes);
+        x.cols[o].hasNull = os.kind != omg::OUT_COUNT && os.kind != omg::OUT_IS_EMPTY;
+        at += up(bound * os.outWidth + 16);
+    }
+    for (size_t o = 0; o < nOut && o < plan_.outContainer.size(); ++o) {
+        // A container's fields (a partial AVG's sum and count) are never NULL.
+        x.cols[o].containerFields = plan_.outContainer[o];
+        for (int32_t f = 0; f < plan_.outContainer[o]; ++f) {
+            x.cols[o + f].hasNull = false;
+        }
+    }
+    omg::AggExtract &e = x.e;
+    std::memset(&e, 0, sizeof(e));
+    e.table = MakeLaunch(plan_, im.slots.Get(), im.capacity, im.special.Get(), im.stats.Get()).table;
+    e.key = plan_.key;
+    e.nAccs = static_cast<int32_t>(plan_.accs.size());
+    for (int i = 0; i < e.nAccs; ++i) {
+        e.accs[i] = plan_.accs[i];
+    }
+    e.nOut = static_cast<int32_t>(nOut);
+    for (size_t o = 0; o < nOut; ++o) {
+        e.out[o] = plan_.outs[o];
+        e.out[o].values = x.cols[o].values->Data();
+        e.out[o].nulls = static_cast<uint8_t *>(x.cols[o].nulls->Data());
+    }
+    e.overflowAsNull = plan_.overflowAsNull ? 1 : 0;
+    unsigned long long *cnt = im.stats.Get() + kExtractStats;
+    e.outCount = cnt;
+    e.error = reinterpret_cast<int32_t *>(cnt + 1);
+    e.nAmbiguous = cnt + 2;
+    RunExtract(x, s);
+}
+
+// Clears the NULL bitmaps and the counters, and extracts the table's and the dense groups.
+void HashAggregationOperator::RunExtract(ExtractRun &x, cudaStream_t s)
+{
+    Impl &im = *impl_;
+    char *nulls = static_cast<char *>(x.cols[0].nulls->Data());
+    const size_t bytes = x.cols.size() * x.cols[0].nulls->Bytes();  // one after another
+    if (x.onHost) {
+        std::memset(nulls, 0, bytes);
+    } else {
+        CudaCheck(cudaMemsetAsync(nulls, 0, bytes, s), "reset nulls");
+    }
+    CudaCheck(cudaMemsetAsync(im.stats.Get() + kExtractStats, 0, 3 * sizeof(unsigned long long), s), "reset counters");
+    CudaCheck(omg::LaunchAggExtract(x.e, s), "extract groups");
+    ++counters_[0];
+    if (im.denseGroups > 0) {
+        DevArray<uint32_t> noSpecial(2, s, true);
+        omg::AggExtract d = x.e;
+        d.table = MakeLaunch(plan_, im.dense.Get(), im.denseGroups, noSpecial.Get(), im.stats.Get()).table;
+        CudaCheck(omg::LaunchAggExtract(d, s), "extract dense groups");
+        ++counters_[0];
+    }
+}
+
 void HashAggregationOperator::Extract()
 {
     if (spillEnabled_ && ExtractSpilled()) {
         return;
     }
-    Flush();
+    Flush(true);
     Impl &im = *impl_;
     if (im.capacity == 0) {
         uniqueKeys_ = 0;
@@ -2026,84 +2140,42 @@ void HashAggregationOperator::Extract()
     }
     cudaStream_t s = im.stream.Get();
     omg::AggLaunch base = MakeLaunch(plan_, im.slots.Get(), im.capacity, im.special.Get(), im.stats.Get());
-    DevArray<unsigned long long> cnt(4, s, true);
-    CudaCheck(omg::LaunchAggCount(base.table, plan_.key.kind, cnt.Get(), s), "count groups");
-    unsigned long long nGroups = 0;
-    CudaCheck(cudaMemcpyAsync(&nGroups, cnt.Get(), sizeof(nGroups), cudaMemcpyDeviceToHost, s), "read group count");
-    im.stream.Sync();
-    nGroups += im.denseGroups;
-    uniqueKeys_ = nGroups;
-    counters_[3] = static_cast<int64_t>(nGroups);
-    if (nGroups == 0) {
-        return;
-    }
     const size_t nOut = plan_.outs.size();
-    std::vector<omg::OutColumn> cols(nOut);
-    for (size_t o = 0; o < nOut; ++o) {
-        const OutSpec &os = plan_.outs[o];
-        cols[o].type = plan_.outTypes[o]->GetId();
-        cols[o].width = os.outWidth;
-        cols[o].values = omg::Buffer::NewDevice(static_cast<size_t>(nGroups) * os.outWidth + 16, s, false);
-        cols[o].nulls = omg::Buffer::NewDevice(omg::NullBitmapBytes(static_cast<int64_t>(nGroups)), s, true);
-        cols[o].hasNull = os.kind != omg::OUT_COUNT && os.kind != omg::OUT_IS_EMPTY;
+    const unsigned long long *hc = im.hostStats.Get() + kExtractStats;
+    auto readCounters = [&] {
+        CudaCheck(cudaMemcpyAsync(im.hostStats.Get() + kExtractStats, im.stats.Get() + kExtractStats,
+                      3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s),
+            "read extract counters");
+        im.stream.Sync();
+    };
+    ExtractRun &x = im.ahead;
+    std::vector<omg::OutColumn> &cols = x.cols;
+    omg::AggExtract &e = x.e;
+    DevArray<unsigned long long> ambSlots;
+    // At most the inserted groups and the two special ones.
+    const uint64_t bound = im.groups + im.denseGroups + 2;
+    const uint32_t ambCap = static_cast<uint32_t>(std::min<uint64_t>(bound, 1ull << 22));
+    if (!x.launched) {
+        LaunchExtract(x, bound, s);
+        readCounters();
     }
-    for (size_t o = 0; o < nOut && o < plan_.outContainer.size(); ++o) {
-        // A container's fields (a partial AVG's sum and count) are never NULL.
-        cols[o].containerFields = plan_.outContainer[o];
-        for (int32_t f = 0; f < plan_.outContainer[o]; ++f) {
-            cols[o + f].hasNull = false;
+    if (hc[2] > 0) {
+        // Groups whose sticky-overflow outcome depends on row order: extract again, naming them.
+        ambSlots.Reset(ambCap, s);
+        e.ambiguousSlots = ambSlots.Get();
+        e.ambiguousCap = ambCap;
+        if (im.denseGroups == 0) {
+            RunExtract(x, s);
+            readCounters();
         }
     }
-    omg::AggExtract e;
-    std::memset(&e, 0, sizeof(e));
-    e.table = base.table;
-    e.key = plan_.key;
-    e.nAccs = static_cast<int32_t>(plan_.accs.size());
-    for (int i = 0; i < e.nAccs; ++i) {
-        e.accs[i] = plan_.accs[i];
-    }
-    e.nOut = static_cast<int32_t>(nOut);
-    for (size_t o = 0; o < nOut; ++o) {
-        e.out[o] = plan_.outs[o];
-        e.out[o].values = cols[o].values->Data();
-        e.out[o].nulls = static_cast<uint8_t *>(cols[o].nulls->Data());
-    }
-    e.overflowAsNull = plan_.overflowAsNull ? 1 : 0;
-    // cnt[0] = nGroups (reused as outCount after reset), cnt[1] = error, cnt[2] = nAmbiguous
-    const uint32_t ambCap = static_cast<uint32_t>(std::min<unsigned long long>(nGroups, 1ull << 22));
-    DevArray<unsigned long long> ambSlots(ambCap, s);
-    CudaCheck(cudaMemsetAsync(cnt.Get(), 0, 4 * sizeof(unsigned long long), s), "reset counters");
-    e.outCount = cnt.Get();
-    e.error = reinterpret_cast<int32_t *>(cnt.Get() + 1);
-    e.nAmbiguous = cnt.Get() + 2;
-    e.ambiguousSlots = ambSlots.Get();
-    e.ambiguousCap = ambCap;
-    CudaCheck(omg::LaunchAggExtract(e, s), "extract groups");
-    ++counters_[0];
-    DevArray<uint32_t> noSpecial;
-    if (im.denseGroups > 0) {
-        noSpecial.Reset(2, s, true);
-        omg::AggExtract d = e;
-        d.table = MakeLaunch(plan_, im.dense.Get(), im.denseGroups, noSpecial.Get(), im.stats.Get()).table;
-        CudaCheck(omg::LaunchAggExtract(d, s), "extract dense groups");
-        ++counters_[0];
-    }
-    unsigned long long hc[4];
-    CudaCheck(cudaMemcpyAsync(hc, cnt.Get(), sizeof(hc), cudaMemcpyDeviceToHost, s), "read extract counters");
-    im.stream.Sync();
     if (hc[2] > 0 && im.denseGroups > 0) {
         // The ordered replay finds its groups in the table: everything into the table, and again.
         FoldDense(s);
         base = MakeLaunch(plan_, im.slots.Get(), im.capacity, im.special.Get(), im.stats.Get());
         e.table = base.table;
-        for (size_t o = 0; o < nOut; ++o) {
-            CudaCheck(cudaMemsetAsync(cols[o].nulls->Data(), 0, cols[o].nulls->Bytes(), s), "reset nulls");
-        }
-        CudaCheck(cudaMemsetAsync(cnt.Get(), 0, 4 * sizeof(unsigned long long), s), "reset counters");
-        CudaCheck(omg::LaunchAggExtract(e, s), "extract groups");
-        ++counters_[0];
-        CudaCheck(cudaMemcpyAsync(hc, cnt.Get(), sizeof(hc), cudaMemcpyDeviceToHost, s), "read extract counters");
-        im.stream.Sync();
+        RunExtract(x, s);
+        readCounters();
     }
     if (hc[2] > 0) {
         // Some groups' sticky-overflow outcome depends on row order: replay those groups in
@@ -2130,27 +2202,29 @@ void HashAggregationOperator::Extract()
         CudaCheck(omg::LaunchAggOrdered(p, static_cast<int32_t>(im.retained.size()), e, ambSlots.Get(),
                       static_cast<uint32_t>(hc[2]), forced.Get(), s),
             "ordered overflow replay");
-        for (size_t o = 0; o < nOut; ++o) {
-            CudaCheck(cudaMemsetAsync(cols[o].nulls->Data(), 0, cols[o].nulls->Bytes(), s), "reset nulls");
-        }
-        CudaCheck(cudaMemsetAsync(cnt.Get(), 0, 4 * sizeof(unsigned long long), s), "reset counters");
         e.forcedOverflow = forced.Get();
-        CudaCheck(omg::LaunchAggExtract(e, s), "extract groups");
-        counters_[0] += 2;
-        CudaCheck(cudaMemcpyAsync(hc, cnt.Get(), sizeof(hc), cudaMemcpyDeviceToHost, s), "read extract counters");
-        im.stream.Sync();
+        ++counters_[0];
+        RunExtract(x, s);
+        readCounters();
     }
     if (hc[1] != 0) {
         throw OmniException("OPERATOR_RUNTIME_ERROR", "sum_aggregator overflow.", -5);
     }
     const int64_t rows = static_cast<int64_t>(hc[0]);
+    uniqueKeys_ = hc[0];
+    counters_[3] = rows;
+    if (rows == 0) {
+        return;
+    }
     if (!plan_.dictInputs.empty()) {
         DecodeStrings(cols, rows, s);
     }
     std::vector<omg::OutColumn> outCols = cols;
     if (!deviceOutput_) {
-        outCols = omg::CopyColumnsToHost(cols, rows, s);
-        im.stream.Sync();
+        if (!x.onHost) {
+            outCols = omg::CopyColumnsToHost(cols, rows, s);
+            im.stream.Sync();
+        }
         for (auto &c : outCols) {
             c.hasNull = false;  // host vectors: HasNull() scans the bitmap
         }
@@ -2158,6 +2232,7 @@ void HashAggregationOperator::Extract()
     for (auto *b : omg::CarveBatches(outCols, rows, plan_.rowsPerBatch)) {
         outputs_.push_back(b);
     }
+    cols.clear();
     counters_[5] = rows;
 }
 

@@ -149,7 +149,11 @@ private:
     void Partition(omg::BatchTable &bt, omg::AggLaunch &p, PartBuffers &pb, cudaStream_t s);
     bool PlanRadix(omg::BatchTable &bt, RadixRun &run, cudaStream_t s);
     void FoldDense(cudaStream_t s);
-    void Flush();
+    struct ExtractRun;
+    // last: no more rows will come.
+    void Flush(bool last = false);
+    void LaunchExtract(ExtractRun &x, uint64_t bound, cudaStream_t s);
+    void RunExtract(ExtractRun &x, cudaStream_t s);
     void EncodeStrings(omg::BatchTable &bt, cudaStream_t s);
     void BindStrings(omg::AggLaunch &p) const;
     void DecodeStrings(std::vector<omg::OutColumn> &cols, int64_t rows, cudaStream_t s);

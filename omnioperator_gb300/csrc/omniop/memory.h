@@ -52,6 +52,15 @@ public:
         return std::make_shared<Buffer>(Kind::DEVICE_VIEW, ptr, bytes);
     }
 
+    // `bytes` bytes from byte `offset` of `whole`, which lives as long as its slices.
+    static std::shared_ptr<Buffer> Slice(const std::shared_ptr<Buffer> &whole, size_t offset, size_t bytes)
+    {
+        auto b = std::make_shared<Buffer>(whole->IsDevice() ? Kind::DEVICE_VIEW : Kind::HOST_VIEW,
+            static_cast<char *>(whole->ptr_) + offset, bytes);
+        b->whole_ = whole;
+        return b;
+    }
+
     void *Data() const { return ptr_; }
     size_t Bytes() const { return bytes_; }
     bool IsDevice() const { return kind_ == Kind::DEVICE || kind_ == Kind::DEVICE_VIEW; }
@@ -62,6 +71,7 @@ private:
     void *ptr_;
     size_t bytes_;
     void *stream_;  // device buffers are freed in order on the stream they were allocated on
+    std::shared_ptr<Buffer> whole_;
 };
 using BufferPtr = std::shared_ptr<Buffer>;
 
