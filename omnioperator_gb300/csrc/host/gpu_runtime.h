@@ -185,6 +185,7 @@ public:
     int64_t BatchRows(size_t batch) { return descs_[batch].rows; }
     int64_t BatchRowBase(size_t batch) { return descs_[batch].rowBase; }
     size_t NumBatches() const { return nBatches_; }
+    const BatchDesc *HostBatches() const { return descs_; }  // pinned; as built
     const BatchDesc *DeviceBatches() const { return reinterpret_cast<const BatchDesc *>(device_.Get()); }
     const TileDesc *DeviceTiles() const { return reinterpret_cast<const TileDesc *>(device_.Get() + tilesAt_); }
     const int64_t *DeviceTileOutRows() const { return reinterpret_cast<const int64_t *>(device_.Get() + tileOutAt_); }

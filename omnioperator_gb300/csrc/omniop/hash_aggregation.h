@@ -152,7 +152,10 @@ private:
     struct ExtractRun;
     // last: no more rows will come.
     void Flush(bool last = false);
+    void AllocOutputs(ExtractRun &x, uint64_t bound, cudaStream_t s);
     void LaunchExtract(ExtractRun &x, uint64_t bound, cudaStream_t s);
+    bool ExtractSmall();
+    void EmitOutputs(ExtractRun &x, int64_t rows, cudaStream_t s);
     void RunExtract(ExtractRun &x, cudaStream_t s);
     void EncodeStrings(omg::BatchTable &bt, cudaStream_t s);
     void BindStrings(omg::AggLaunch &p) const;
