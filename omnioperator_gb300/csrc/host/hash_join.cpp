@@ -79,8 +79,9 @@ struct JoinBuildState {
     std::vector<bool> colHasNull;
     std::vector<DevArray<int64_t>> colOffs;  // VARCHAR/CHAR columns: rows + 1 offsets into colValues
     DevArray<int64_t> entries;
-    DevArray<uint64_t> hashKeys;
+    DevArray<uint64_t> hashSlots;  // {key, entry} pairs
     DevArray<int32_t> csr;
+    int64_t csrCount = 0;
     omg::JoinTable table{};
     uint32_t maxDup = 0;
     DevArray<uint8_t> visited;  // BUILD_OUTER / FULL: one byte per build row, set by the probes
@@ -192,7 +193,13 @@ void JoinBuildState::Build()
     const int32_t keyWidth = multiKey ? 8 : buildTypes.GetType(keyCol)->ByteWidth();
     table.keyWidth = keyWidth;
     // Gather every build column into one contiguous HBM array (reading host-pinned or
-    // device batches directly).
+    // device batches directly).  The batch tables' staging outlives the copies (the key statistics are
+    // waited for).
+    std::vector<omg::BatchTable> tables(static_cast<size_t>(nCols));
+    struct Wait {  // before the staging goes, also when a column throws
+        cudaStream_t s;
+        ~Wait() { cudaStreamSynchronize(s); }
+    } wait{s};
     for (int c = 0; c < nCols; ++c) {
         const bool varlen = Varlen(buildTypes.GetType(c));
         const int w = buildTypes.GetType(c)->ByteWidth();
@@ -208,7 +215,7 @@ void JoinBuildState::Build()
         if (rows == 0) {
             continue;
         }
-        omg::BatchTable bt;
+        omg::BatchTable &bt = tables[static_cast<size_t>(c)];
         bt.Build(batches, {c});
         bt.Upload(s);
         if (bt.AnyNulls(0)) {
@@ -230,7 +237,6 @@ void JoinBuildState::Build()
         CudaCheck(omg::LaunchGatherColumn(bt.DeviceBatches(), bt.DeviceTiles(), bt.NumTiles(), bt.DeviceTileOutRows(),
                       0, w, colValues[c].Get(), colHasNull[c] ? colNulls[c].Get() : nullptr, s),
             "gather build column");
-        stream.Sync();  // the batch table's staging must outlive the copy
     }
     if (rows == 0) {
         built = true;
@@ -295,11 +301,11 @@ void JoinBuildState::Build()
         table.mode = omg::JOIN_HASH;
         table.capacity = std::max<uint64_t>(NextPow2(2 * static_cast<uint64_t>(nonNull)), 1024);
         n = table.capacity;
-        hashKeys.Reset(n, s);
-        CudaCheck(omg::LaunchFillU64(hashKeys.Get(), omg::kEmptyKey, static_cast<int64_t>(n), s), "init hash keys");
+        hashSlots.Reset(2 * n, s);
+        CudaCheck(omg::LaunchFillHashSlots(hashSlots.Get(), static_cast<int64_t>(n), s), "init hash slots");
     }
     DevArray<uint32_t> counts(n, s, true);
-    CudaCheck(omg::LaunchBuildCount(table, keys, keyNulls, rows, keyWidth, hashKeys.Get(), counts.Get(), sentinelCount,
+    CudaCheck(omg::LaunchBuildCount(table, keys, keyNulls, rows, keyWidth, hashSlots.Get(), counts.Get(), sentinelCount,
                   maxCount, err.Get(), s),
         "build count");
     long long h2[3];
@@ -313,8 +319,11 @@ void JoinBuildState::Build()
     maxDup = static_cast<uint32_t>(h2[0] & 0xffffffffll);
     const uint32_t nSentinel = static_cast<uint32_t>(h2[1] & 0xffffffffll);
     table.unique = (maxDup <= 1 && nSentinel <= 1) ? 1 : 0;
-    entries.Reset(n, s);
-    CudaCheck(omg::LaunchFillI64(entries.Get(), -1, static_cast<int64_t>(n), s), "init entries");
+    if (arrayMode) {
+        entries.Reset(n, s);
+        CudaCheck(omg::LaunchFillI64(entries.Get(), -1, static_cast<int64_t>(n), s), "init entries");
+    }
+    int64_t *entryWords = arrayMode ? entries.Get() : reinterpret_cast<int64_t *>(hashSlots.Get()) + 1;
     DevArray<int64_t> offsets;
     DevArray<uint32_t> cursor;
     int64_t total = 0;
@@ -328,14 +337,14 @@ void JoinBuildState::Build()
         CudaCheck(cudaMemcpyAsync(&ht, tot.Get(), sizeof(ht), cudaMemcpyDeviceToHost, s), "read total");
         stream.Sync();
         total = ht;
-        csr.Reset(static_cast<size_t>(total + nSentinel + 1), s);
+        csrCount = total + static_cast<int64_t>(nSentinel);
+        csr.Reset(static_cast<size_t>(csrCount + 1), s);
         cursor.Reset(n, s, true);
     }
     table.arrayEntries = entries.Get();
-    table.hashEntries = entries.Get();
-    table.hashKeys = hashKeys.Get();
+    table.hashSlots = hashSlots.Get();
     CudaCheck(omg::LaunchBuildFill(table, keys, keyNulls, rows, keyWidth, counts.Get(), offsets.Get(), cursor.Get(),
-                  entries.Get(), csr.Get(), nSentinel, total, sentinelCursor, sentinelEntry, err.Get(), s),
+                  entryWords, csr.Get(), nSentinel, total, sentinelCursor, sentinelEntry, err.Get(), s),
         "build fill");
     int64_t hs = -1;
     CudaCheck(cudaMemcpyAsync(&hs, sentinelEntry, sizeof(hs), cudaMemcpyDeviceToHost, s), "read sentinel");
@@ -1380,7 +1389,7 @@ std::unique_ptr<LookupJoinOperator::ProbeCall> LookupJoinOperator::LaunchBatches
     // Unique build keys and <= 8 bytes of NULL-free build output per row: fetch the build
     // values with the table entry from a per-slot packed copy (built once per factory).
     {
-        bool eligible = b.table.unique && nOut > nProbeOut && b.kind != omg::JOIN_KIND_EXISTENCE && !b.multiKey;
+        bool eligible = (b.table.unique || b.csrCount > 0) && nOut > nProbeOut && b.kind != omg::JOIN_KIND_EXISTENCE && !b.multiKey;
         int shift = 0;
         for (size_t o = nProbeOut; o < nOut && eligible; ++o) {
             const int w = p.out[o].width;
@@ -1389,7 +1398,13 @@ std::unique_ptr<LookupJoinOperator::ProbeCall> LookupJoinOperator::LaunchBatches
             shift += 8 * w;
         }
         std::lock_guard<std::mutex> g(f_.payloadMu);
-        if (eligible && !f_.payloadDecided) {
+        if (eligible && !f_.payloadDecided && !b.table.unique) {
+            f_.slotPayload = omg::Buffer::NewDevice(static_cast<size_t>(b.csrCount) * sizeof(uint64_t), s, false);
+            CudaCheck(omg::LaunchBuildCsrPayload(p, b.csrCount, static_cast<uint64_t *>(f_.slotPayload->Data()), s),
+                "build CSR payload");
+            impl_->stream.Sync();
+            f_.payloadDecided = true;
+        } else if (eligible && !f_.payloadDecided) {
             const uint64_t nSlots = b.table.mode == omg::JOIN_ARRAY ? b.table.range : b.table.capacity;
             f_.slotPayload = omg::Buffer::NewDevice((nSlots + 1) * sizeof(uint64_t), s, false);
             CudaCheck(omg::LaunchBuildSlotPayload(p, nSlots, static_cast<uint64_t *>(f_.slotPayload->Data()), s),
@@ -1407,7 +1422,9 @@ std::unique_ptr<LookupJoinOperator::ProbeCall> LookupJoinOperator::LaunchBatches
                 "build slot bitmap");
             impl_->stream.Sync();
         }
-        if (eligible && f_.slotPayload) {
+        if (eligible && f_.slotPayload && !b.table.unique) {
+            p.table.csrPayload = static_cast<const uint64_t *>(f_.slotPayload->Data());
+        } else if (eligible && f_.slotPayload) {
             p.table.slotPayload = static_cast<const uint64_t *>(f_.slotPayload->Data());
             // Filter operands that are build output columns packed into the payload.
             for (int32_t i = 0; i < p.nFilter; ++i) {
@@ -1434,7 +1451,14 @@ std::unique_ptr<LookupJoinOperator::ProbeCall> LookupJoinOperator::LaunchBatches
         regionCap = std::max<uint64_t>(regionCap, static_cast<uint64_t>(r));
     }
     if (!b.table.unique) {
-        regionCap *= std::min<uint32_t>(b.maxDup, 2);
+        // Room for every key's duplicates while that is at most a gigabyte (64 MiB of pinned memory): a
+        // region that overflows costs the probe a second run.
+        uint64_t rowBytes = 0;
+        for (const omg::OutColumn &c : cols) {
+            rowBytes += c.width == 0 ? 8 : static_cast<uint64_t>(c.width);
+        }
+        const uint64_t bytes = regionCap * static_cast<uint64_t>(nRegions) * rowBytes * b.maxDup;
+        regionCap *= bytes <= (uint64_t(1) << (deviceOutput_ ? 30 : 26)) ? b.maxDup : std::min<uint32_t>(b.maxDup, 2);
     }
     regionCap = (regionCap + 63) / 64 * 64;
     // The region counters, then one more 128-byte line whose first word is the kernel's error.

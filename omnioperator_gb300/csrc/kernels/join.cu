@@ -144,12 +144,12 @@ __global__ void KeyStatsKernel(const void *keys, const uint8_t *nulls, int64_t n
 }
 
 // Find the hash slot of `key` (inserting it when `insert`), -1 if absent.
-__device__ __forceinline__ int64_t HashSlot(uint64_t *keys, uint64_t capacity, uint64_t key, bool insert)
+__device__ __forceinline__ int64_t HashSlot(uint64_t *slots, uint64_t capacity, uint64_t key, bool insert)
 {
     const uint64_t mask = capacity - 1;
     uint64_t i = Mix64(key) & mask;
     for (uint64_t probe = 0; probe < capacity; ++probe) {
-        unsigned long long *kp = reinterpret_cast<unsigned long long *>(keys + i);
+        unsigned long long *kp = reinterpret_cast<unsigned long long *>(slots + 2 * i);
         unsigned long long cur = *reinterpret_cast<volatile unsigned long long *>(kp);
         if (cur == key) {
             return static_cast<int64_t>(i);
@@ -169,8 +169,9 @@ __device__ __forceinline__ int64_t HashSlot(uint64_t *keys, uint64_t capacity, u
 }
 
 __global__ void BuildCountKernel(JoinTable t, const void *keys, const uint8_t *nulls, int64_t n, int32_t width,
-    uint64_t *hashKeys, uint32_t *counts, uint32_t *sentinelCount, unsigned int *maxCount, int32_t *error)
+    uint64_t *hashSlots, uint32_t *counts, uint32_t *sentinelCount, unsigned int *maxCount, int32_t *error)
 {
+    uint32_t most = 0;  // the largest count this thread saw: one atomic per warp, not one per duplicate
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         if (RowIsNull(nulls, i)) {
@@ -183,16 +184,18 @@ __global__ void BuildCountKernel(JoinTable t, const void *keys, const uint8_t *n
         } else if (key == kEmptyKey) {
             old = atomicAdd(sentinelCount, 1u);
         } else {
-            const int64_t s = HashSlot(hashKeys, t.capacity, key, true);
+            const int64_t s = HashSlot(hashSlots, t.capacity, key, true);
             if (s < 0) {
                 SetError(error, 4);
                 continue;
             }
             old = atomicAdd(&counts[s], 1u);
         }
-        if (old >= 1) {
-            atomicMax(maxCount, old + 1);
-        }
+        most = max(most, old + 1);
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((threadIdx.x & 31) == 0 && most > 1) {
+        atomicMax(maxCount, most);
     }
 }
 
@@ -201,6 +204,7 @@ __global__ void BuildFillKernel(JoinTable t, const void *keys, const uint8_t *nu
     uint32_t sentinelCount, int64_t sentinelOffset, unsigned int *sentinelCursor, int64_t *sentinelEntryOut,
     int32_t *error)
 {
+    const int step = t.mode == JOIN_ARRAY ? 1 : 2;  // words from one slot's entry to the next
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         if (RowIsNull(nulls, i)) {
@@ -213,7 +217,7 @@ __global__ void BuildFillKernel(JoinTable t, const void *keys, const uint8_t *nu
         } else if (key == kEmptyKey) {
             slot = -2;
         } else {
-            slot = HashSlot(const_cast<uint64_t *>(t.hashKeys), t.capacity, key, false);
+            slot = HashSlot(const_cast<uint64_t *>(t.hashSlots), t.capacity, key, false);
             if (slot < 0) {
                 SetError(error, 4);
                 continue;
@@ -221,7 +225,7 @@ __global__ void BuildFillKernel(JoinTable t, const void *keys, const uint8_t *nu
         }
         if (t.unique) {
             if (slot >= 0) {
-                entries[slot] = i;
+                entries[slot * step] = i;
             } else {
                 *sentinelEntryOut = i;
             }
@@ -236,7 +240,7 @@ __global__ void BuildFillKernel(JoinTable t, const void *keys, const uint8_t *nu
         const int64_t off = offsets[slot];
         csrRows[off + c] = static_cast<int32_t>(i);
         if (c == 0) {
-            entries[slot] = (off << 32) | static_cast<int64_t>(counts[slot]);
+            entries[slot * step] = (off << 32) | static_cast<int64_t>(counts[slot]);
         }
     }
 }
@@ -249,11 +253,11 @@ __global__ void FillI64Kernel(int64_t *p, int64_t v, int64_t n)
     }
 }
 
-__global__ void FillU64Kernel(uint64_t *p, uint64_t v, int64_t n)
+__global__ void FillHashSlotsKernel(ulonglong2 *p, int64_t n)
 {
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        p[i] = v;
+        p[i] = make_ulonglong2(kEmptyKey, ~0ull);
     }
 }
 
@@ -281,15 +285,38 @@ __global__ void ScanBlockSumsKernel(const uint32_t *counts, int64_t n, int64_t *
     }
 }
 
-__global__ void ScanSumsKernel(int64_t *blockSums, int64_t nBlocks, long long *total)
+// One block; each thread takes consecutive sums (one thread alone took 138 us for 2048 of them).
+__global__ void __launch_bounds__(kScanThreads) ScanSumsKernel(int64_t *blockSums, int64_t nBlocks, long long *total)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        long long run = 0;
-        for (int64_t b = 0; b < nBlocks; ++b) {
-            const long long v = blockSums[b];
-            blockSums[b] = run;
-            run += v;
-        }
+    __shared__ long long warpSums[32];
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const int64_t per = (nBlocks + kScanThreads - 1) / kScanThreads;
+    const int64_t first = min(static_cast<int64_t>(threadIdx.x) * per, nBlocks);
+    const int64_t end = min(first + per, nBlocks);
+    long long mine = 0;
+    for (int64_t i = first; i < end; ++i) {
+        mine += blockSums[i];
+    }
+    long long inc = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long y = __shfl_up_sync(0xffffffffu, inc, o);
+        inc += lane >= o ? y : 0;
+    }
+    if (lane == 31) {
+        warpSums[warp] = inc;
+    }
+    __syncthreads();
+    long long run = inc - mine;
+    for (int w = 0; w < warp; ++w) {
+        run += warpSums[w];
+    }
+    for (int64_t i = first; i < end; ++i) {
+        const long long v = blockSums[i];
+        blockSums[i] = run;
+        run += v;
+    }
+    if (threadIdx.x == kScanThreads - 1) {
         *total = run;
     }
 }
@@ -350,13 +377,13 @@ __device__ __forceinline__ Match Lookup(const JoinTable &t, uint64_t key)
         const uint64_t mask = t.capacity - 1;
         uint64_t i = Mix64(key) & mask;
         for (uint64_t probe = 0; probe < t.capacity; ++probe) {
-            const uint64_t k = __ldg(reinterpret_cast<const unsigned long long *>(t.hashKeys) + i);
-            if (k == key) {
-                e = __ldg(reinterpret_cast<const long long *>(t.hashEntries) + i);
+            const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(t.hashSlots) + i);
+            if (v.x == key) {
+                e = static_cast<int64_t>(v.y);
                 m.slot = i;
                 break;
             }
-            if (k == kEmptyKey) {
+            if (v.x == kEmptyKey) {
                 break;
             }
             i = (i + 1) & mask;
@@ -374,6 +401,51 @@ __device__ __forceinline__ Match Lookup(const JoinTable &t, uint64_t key)
     return m;
 }
 
+__device__ __forceinline__ void SetMatch(const JoinTable &t, int64_t e, uint64_t slot, Match &m)
+{
+    m.slot = slot;
+    if (e >= 0) {
+        m.entry = t.unique ? e : e >> 32;
+        m.count = t.unique ? 1u : static_cast<uint32_t>(e & 0xffffffffll);
+    }
+}
+
+// Lookup of N keys (bit j of live) in a HASH table.  The first slots of all keys are loaded before any is
+// looked at, so that their latencies overlap; a key whose first slot holds another key goes on alone.
+template <int N>
+__device__ __forceinline__ void LookupHash(const JoinTable &t, const int64_t (&key)[N], uint32_t live, Match (&m)[N])
+{
+    const uint64_t mask = t.capacity - 1;
+    const ulonglong2 *slots = reinterpret_cast<const ulonglong2 *>(t.hashSlots);
+    ulonglong2 v[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        v[j] = ((live >> j) & 1u) != 0 ? __ldg(slots + (Mix64(static_cast<uint64_t>(key[j])) & mask))
+                                       : make_ulonglong2(kEmptyKey, ~0ull);
+    }
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        m[j] = Match{0, 0, 0};
+        if (((live >> j) & 1u) == 0) {
+            continue;
+        }
+        const uint64_t k = static_cast<uint64_t>(key[j]);
+        if (k == kEmptyKey) {
+            SetMatch(t, t.sentinelEntry, t.capacity, m[j]);
+            continue;
+        }
+        uint64_t i = Mix64(k) & mask;
+        ulonglong2 w = v[j];
+        for (uint64_t probe = 1; w.x != k && w.x != kEmptyKey && probe < t.capacity; ++probe) {
+            i = (i + 1) & mask;
+            w = __ldg(slots + i);
+        }
+        if (w.x == k) {
+            SetMatch(t, static_cast<int64_t>(w.y), i, m[j]);
+        }
+    }
+}
+
 // Read-only loads (non-coherent path): the probe never writes what it reads, so these may be
 // issued ahead of the output stores.
 __device__ __forceinline__ int64_t LoadIntRO(const void *col, int64_t row, int width)
@@ -388,6 +460,58 @@ __device__ __forceinline__ int64_t LoadIntRO(const void *col, int64_t row, int w
         default:
             return __ldg(static_cast<const long long *>(col) + row);
     }
+}
+
+// Keys of rows row0 + 32 j (j < n), zero-extended rows past `rows` included as 0: the loads of all N rows are in
+// flight together, under one branch on the width.
+template <int N>
+__device__ __forceinline__ void LoadKeysRO(const void *col, int64_t row0, int64_t rows, int width, int64_t (&key)[N])
+{
+    switch (width) {
+        case 1:
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                key[j] = row0 + 32 * j < rows ? LoadIntRO(col, row0 + 32 * j, 1) : 0;
+            }
+            break;
+        case 2:
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                key[j] = row0 + 32 * j < rows ? LoadIntRO(col, row0 + 32 * j, 2) : 0;
+            }
+            break;
+        case 4:
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                key[j] = row0 + 32 * j < rows ? LoadIntRO(col, row0 + 32 * j, 4) : 0;
+            }
+            break;
+        default:
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                key[j] = row0 + 32 * j < rows ? LoadIntRO(col, row0 + 32 * j, 8) : 0;
+            }
+            break;
+    }
+}
+
+// Bit j: row row0 + 32 j exists (it is below `rows`) and is NULL.
+template <int N> __device__ __forceinline__ uint32_t NullRowsRO(const uint8_t *nulls, int64_t row0, int64_t rows)
+{
+    if (nulls == nullptr) {
+        return 0;
+    }
+    unsigned int byte[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        byte[j] = row0 + 32 * j < rows ? __ldg(reinterpret_cast<const unsigned char *>(nulls) + ((row0 + 32 * j) >> 3)) : 0u;
+    }
+    uint32_t m = 0;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        m |= ((byte[j] >> ((row0 + 32 * j) & 7)) & 1u) << j;
+    }
+    return m;
 }
 
 __device__ __forceinline__ bool RowIsNullRO(const uint8_t *nulls, int64_t row)
@@ -487,25 +611,40 @@ __device__ __forceinline__ void WriteJoinRowPayload(const ProbeLaunch &p, const 
     }
 }
 
+__device__ __forceinline__ uint64_t PackBuildRow(const ProbeLaunch &p, int64_t row)
+{
+    uint64_t v = 0;
+    for (int o = 0; o < p.nOut; ++o) {
+        const JoinOutCol &oc = p.out[o];
+        if (oc.side == 1) {
+            const uint64_t bits = LoadBits(oc.buildValues, row, oc.width);
+            const uint64_t mask = oc.width >= 8 ? ~0ull : ((1ull << (8 * oc.width)) - 1);
+            v |= (bits & mask) << oc.shift;
+        }
+    }
+    return v;
+}
+
 // Packs the build output values of every unique-table slot (<= 8 bytes in total).
-__global__ void BuildSlotPayloadKernel(const int64_t *entries, uint64_t nSlots, int64_t sentinelEntry,
+// (step: words from one slot's entry to the next.)
+__global__ void BuildSlotPayloadKernel(const int64_t *entries, int step, uint64_t nSlots, int64_t sentinelEntry,
     const __grid_constant__ ProbeLaunch p, uint64_t *payload)
 {
     for (uint64_t s = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; s <= nSlots;
          s += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        const int64_t row = s < nSlots ? entries[s] : sentinelEntry;
-        uint64_t v = 0;
-        if (row >= 0) {
-            for (int o = 0; o < p.nOut; ++o) {
-                const JoinOutCol &oc = p.out[o];
-                if (oc.side == 1) {
-                    const uint64_t bits = LoadBits(oc.buildValues, row, oc.width);
-                    const uint64_t mask = oc.width >= 8 ? ~0ull : ((1ull << (8 * oc.width)) - 1);
-                    v |= (bits & mask) << oc.shift;
-                }
-            }
-        }
-        payload[s] = v;
+        const int64_t row = s < nSlots ? entries[s * step] : sentinelEntry;
+        payload[s] = row >= 0 ? PackBuildRow(p, row) : 0;
+    }
+}
+
+// The same for the CSR of a table with duplicates: a key's build rows' values lie side by side, so that a
+// match takes one load of a line where it took the row number and a gather per column.
+__global__ void BuildCsrPayloadKernel(const int32_t *csrRows, int64_t n, const __grid_constant__ ProbeLaunch p,
+    uint64_t *payload)
+{
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        payload[i] = PackBuildRow(p, csrRows[i]);
     }
 }
 
@@ -568,8 +707,11 @@ __device__ __forceinline__ uint32_t EmitCount(int kind, bool exists, uint32_t cn
 // rows base + 32r + i (coalesced), looks the keys up, reserves its output range with one
 // atomicAdd, and writes its matches compacted in row order.  kUnique: every key has at most one
 // build row, so a ballot gives the compaction; otherwise counts are prefix-summed per round.
-constexpr int kWarpRounds = 16;
+// (Four rounds: with sixteen a small launch was one CTA of eight warps, and the arrays of a lane's rows did not fit
+// the registers.)
+constexpr int kWarpRounds = 4;
 constexpr int kRowsPerWarp = kWarpRounds * 32;
+constexpr int kSegsPerTile = kTileRows / kRowsPerWarp;
 
 // kKinds: any join kind (p.joinKind) -- the rows each probe row yields follow EmitCount, rows
 // without a match get NULL build columns, and matched build rows are marked visited when the
@@ -584,9 +726,12 @@ __global__ void __launch_bounds__(kProbeThreads, 3) ProbeKernel(const __grid_con
     const int kind = kKinds ? p.joinKind : static_cast<int>(JOIN_KIND_INNER);
     const bool emitMatches = kind == JOIN_KIND_INNER || kind == JOIN_KIND_PROBE_OUTER ||
         kind == JOIN_KIND_BUILD_OUTER || kind == JOIN_KIND_FULL;
-    for (int t = blockIdx.x; t < p.nTiles; t += gridDim.x) {
+    const int64_t nItems = static_cast<int64_t>(p.nTiles) * kSegsPerTile;
+    for (int64_t item = static_cast<int64_t>(blockIdx.x) * (kProbeThreads / 32) + warp; item < nItems;
+         item += static_cast<int64_t>(gridDim.x) * (kProbeThreads / 32)) {
+        const int t = static_cast<int>(item / kSegsPerTile);
         const TileDesc tile = p.tiles[t];
-        const int w0 = warp * kRowsPerWarp;
+        const int w0 = static_cast<int>(item % kSegsPerTile) * kRowsPerWarp;
         if (w0 >= tile.rows) {
             continue;
         }
@@ -594,23 +739,17 @@ __global__ void __launch_bounds__(kProbeThreads, 3) ProbeKernel(const __grid_con
         const void *keyCol = b.cols[p.keyInput];
         const uint8_t *keyNulls = b.nulls[p.keyInput];
         const int64_t base = static_cast<int64_t>(tile.row0) + w0;
-        const int nRows = min(kRowsPerWarp, tile.rows - w0);
+        const int64_t endRow = static_cast<int64_t>(tile.row0) + tile.rows;
         // Phase 1: all keys and validity bits of the warp's rows (independent loads).
         int64_t key[kWarpRounds];
-        uint32_t live = 0;   // bit i: this lane's row of round i exists and its key is not NULL
+        LoadKeysRO<kWarpRounds>(keyCol, base + lane, endRow, p.keyWidth, key);
         uint32_t exist = 0;  // bit i: this lane's row of round i exists
 #pragma unroll
         for (int i = 0; i < kWarpRounds; ++i) {
-            const int r = i * 32 + lane;
-            key[i] = 0;
-            if (r < nRows) {
-                exist |= 1u << i;
-                key[i] = LoadIntRO(keyCol, base + r, p.keyWidth);
-                if (!RowIsNullRO(keyNulls, base + r)) {
-                    live |= 1u << i;
-                }
-            }
+            exist |= base + i * 32 + lane < endRow ? 1u << i : 0u;
         }
+        // bit i: this lane's row of round i exists and its key is not NULL
+        const uint32_t live = exist & ~NullRowsRO<kWarpRounds>(keyNulls, base + lane, endRow);
         // Phase 2: table lookups (independent of each other).
         int32_t entry[kWarpRounds];
         uint32_t cnt[kWarpRounds];
@@ -624,7 +763,7 @@ __global__ void __launch_bounds__(kProbeThreads, 3) ProbeKernel(const __grid_con
                 payload[i] = 0;
                 if (((live >> i) & 1u) && key[i] >= p.table.minKey && d < p.table.range) {
                     e = __ldg(reinterpret_cast<const long long *>(p.table.arrayEntries) + d);
-                    if (kPayload) {
+                    if (kUnique && kPayload) {
                         payload[i] = __ldg(reinterpret_cast<const unsigned long long *>(p.table.slotPayload) + d);
                     }
                 }
@@ -633,19 +772,16 @@ __global__ void __launch_bounds__(kProbeThreads, 3) ProbeKernel(const __grid_con
                 hit |= (cnt[i] != 0 ? 1u : 0u) << i;
             }
         } else {
+            Match m[kWarpRounds];
+            LookupHash<kWarpRounds>(p.table, key, live, m);
 #pragma unroll
             for (int i = 0; i < kWarpRounds; ++i) {
-                Match m{0, 0, 0};
-                payload[i] = 0;
-                if ((live >> i) & 1u) {
-                    m = Lookup(p.table, static_cast<uint64_t>(key[i]));
-                    if (kPayload && m.count != 0) {
-                        payload[i] = __ldg(reinterpret_cast<const unsigned long long *>(p.table.slotPayload) + m.slot);
-                    }
-                }
-                entry[i] = static_cast<int32_t>(m.entry);
-                cnt[i] = m.count;
-                hit |= (m.count != 0 ? 1u : 0u) << i;
+                payload[i] = kUnique && kPayload && m[i].count != 0
+                    ? __ldg(reinterpret_cast<const unsigned long long *>(p.table.slotPayload) + m[i].slot)
+                    : 0ull;
+                entry[i] = static_cast<int32_t>(m[i].entry);
+                cnt[i] = m[i].count;
+                hit |= (m[i].count != 0 ? 1u : 0u) << i;
             }
         }
         if (kKinds && p.visited != nullptr) {
@@ -707,8 +843,7 @@ __global__ void __launch_bounds__(kProbeThreads, 3) ProbeKernel(const __grid_con
                 if (e) {
                     const uint64_t at = pos + __popc(m & lanesBelow);
                     if (at < p.regionCap) {
-                        // The key is re-read (an L1/L2 hit) rather than kept live in registers.
-                        const int64_t k = LoadIntRO(keyCol, row, p.keyWidth);
+                        const int64_t k = key[i];
                         if (kKinds && !(matched && emitMatches)) {
                             WriteProbeOnlyRow(p, b, row, k, matched, regionBase + at);
                         } else if (kPayload) {
@@ -732,15 +867,20 @@ __global__ void __launch_bounds__(kProbeThreads, 3) ProbeKernel(const __grid_con
                 const uint64_t at = pos + inc - e;
                 if (kKinds && e != 0 && !(matched && emitMatches)) {
                     if (at < p.regionCap) {
-                        WriteProbeOnlyRow(p, b, row, LoadIntRO(keyCol, row, p.keyWidth), matched, regionBase + at);
+                        WriteProbeOnlyRow(p, b, row, key[i], matched, regionBase + at);
                     }
                 } else {
                     for (uint32_t k = 0; k < e; ++k) {
                         if (at + k >= p.regionCap) {
                             break;
                         }
-                        WriteJoinRow(p, b, row, LoadIntRO(keyCol, row, p.keyWidth),
-                            __ldg(p.table.csrRows + entry[i] + k), regionBase + at + k);
+                        if (kPayload) {
+                            WriteJoinRowPayload(p, b, row, key[i],
+                                __ldg(reinterpret_cast<const unsigned long long *>(p.table.csrPayload) + entry[i] + k),
+                                regionBase + at + k);
+                        } else {
+                            WriteJoinRow(p, b, row, key[i], __ldg(p.table.csrRows + entry[i] + k), regionBase + at + k);
+                        }
                     }
                 }
                 pos += __shfl_sync(0xffffffffu, inc, 31);
@@ -1673,9 +1813,12 @@ __global__ void __launch_bounds__(kProbeThreads, 3) ProbeFastKernel(const __grid
         shift[o] = p.out[o].shift;
         isKey[o] = p.out[o].side == 0;
     }
-    for (int t = blockIdx.x; t < p.nTiles; t += gridDim.x) {
+    const int64_t nItems = static_cast<int64_t>(p.nTiles) * kSegsPerTile;
+    for (int64_t item = static_cast<int64_t>(blockIdx.x) * (kProbeThreads / 32) + warp; item < nItems;
+         item += static_cast<int64_t>(gridDim.x) * (kProbeThreads / 32)) {
+        const int t = static_cast<int>(item / kSegsPerTile);
         const TileDesc tile = p.tiles[t];
-        const int w0 = warp * kRowsPerWarp;
+        const int w0 = static_cast<int>(item % kSegsPerTile) * kRowsPerWarp;
         if (w0 >= tile.rows) {
             continue;
         }
@@ -1683,20 +1826,16 @@ __global__ void __launch_bounds__(kProbeThreads, 3) ProbeFastKernel(const __grid
         const long long *keyCol = static_cast<const long long *>(b.cols[p.keyInput]);
         const uint8_t *keyNulls = b.nulls[p.keyInput];
         const int64_t base = static_cast<int64_t>(tile.row0) + w0;
-        const int nRows = min(kRowsPerWarp, tile.rows - w0);
+        const int64_t endRow = static_cast<int64_t>(tile.row0) + tile.rows;
         int64_t key[kWarpRounds];
         uint32_t live = 0;
 #pragma unroll
         for (int i = 0; i < kWarpRounds; ++i) {
-            const int r = i * 32 + lane;
-            key[i] = 0;
-            if (r < nRows) {
-                key[i] = __ldg(keyCol + base + r);
-                if (!RowIsNullRO(keyNulls, base + r)) {
-                    live |= 1u << i;
-                }
-            }
+            const int64_t row = base + i * 32 + lane;
+            key[i] = row < endRow ? __ldg(keyCol + row) : 0;
+            live |= row < endRow ? 1u << i : 0u;
         }
+        live &= ~NullRowsRO<kWarpRounds>(keyNulls, base + lane, endRow);
         uint64_t payload[kWarpRounds];
         uint32_t hit = 0;
         if (arrayMode) {
@@ -1711,16 +1850,12 @@ __global__ void __launch_bounds__(kProbeThreads, 3) ProbeFastKernel(const __grid
                 }
             }
         } else {
+            Match m[kWarpRounds];
+            LookupHash<kWarpRounds>(p.table, key, live, m);
 #pragma unroll
             for (int i = 0; i < kWarpRounds; ++i) {
-                payload[i] = 0;
-                if ((live >> i) & 1u) {
-                    const Match m = Lookup(p.table, static_cast<uint64_t>(key[i]));
-                    if (m.count != 0) {
-                        payload[i] = __ldg(payloadTab + m.slot);
-                        hit |= 1u << i;
-                    }
-                }
+                payload[i] = m[i].count != 0 ? __ldg(payloadTab + m[i].slot) : 0ull;
+                hit |= (m[i].count != 0 ? 1u : 0u) << i;
             }
         }
         uint32_t total = 0;
@@ -1745,8 +1880,7 @@ __global__ void __launch_bounds__(kProbeThreads, 3) ProbeFastKernel(const __grid
                 const uint64_t rat = pos + __popc(m & lanesBelow);
                 if (rat < p.regionCap) {
                     const uint64_t at = regionBase + rat;
-                    // Re-read the key (an L1 hit) rather than keeping 16 keys live in registers.
-                    const int64_t kv = __ldg(keyCol + base + i * 32 + lane);
+                    const int64_t kv = key[i];
 #pragma unroll
                     for (int o = 0; o < kNumOut; ++o) {
                         const int64_t v = isKey[o] ? kv : static_cast<int64_t>(payload[i] >> shift[o]);
@@ -2913,13 +3047,13 @@ cudaError_t LaunchKeyStats(const void *keys, const uint8_t *nulls, int64_t n, in
 }
 
 cudaError_t LaunchBuildCount(JoinTable t, const void *keys, const uint8_t *nulls, int64_t n, int32_t width,
-    uint64_t *hashKeysMutable, uint32_t *counts, uint32_t *sentinelCount, unsigned int *maxCount, int32_t *error,
+    uint64_t *hashSlotsMutable, uint32_t *counts, uint32_t *sentinelCount, unsigned int *maxCount, int32_t *error,
     cudaStream_t stream)
 {
     if (n == 0) {
         return cudaSuccess;
     }
-    BuildCountKernel<<<GridFor(n, 256, 8), 256, 0, stream>>>(t, keys, nulls, n, width, hashKeysMutable, counts,
+    BuildCountKernel<<<GridFor(n, 256, 8), 256, 0, stream>>>(t, keys, nulls, n, width, hashSlotsMutable, counts,
         sentinelCount, maxCount, error);
     return cudaGetLastError();
 }
@@ -2932,7 +3066,7 @@ cudaError_t LaunchScanCounts(const uint32_t *counts, int64_t n, int64_t *offsets
         return cudaMemsetAsync(total, 0, sizeof(long long), stream);
     }
     ScanBlockSumsKernel<<<static_cast<unsigned>(nBlocks), kScanThreads, 0, stream>>>(counts, n, blockSums);
-    ScanSumsKernel<<<1, 32, 0, stream>>>(blockSums, nBlocks, total);
+    ScanSumsKernel<<<1, kScanThreads, 0, stream>>>(blockSums, nBlocks, total);
     ScanApplyKernel<<<static_cast<unsigned>(nBlocks), kScanThreads, 0, stream>>>(counts, n, blockSums, offsets);
     return cudaGetLastError();
 }
@@ -3224,16 +3358,19 @@ cudaError_t LaunchProbe(const ProbeLaunch &p, cudaStream_t stream)
         g_lastProbeKernel.store(PROBE_KERNEL_BITS);
         return cudaLaunchKernel(kernel, dim3(grid), dim3(kBitsThreads), args, static_cast<size_t>(bitsBytes), stream);
     }
+    const int64_t warpCtas = static_cast<int64_t>(p.nTiles) * kSegsPerTile / (kProbeThreads / 32);
     if (p.nKeyCols == 0 && p.joinKind != JOIN_KIND_INNER) {
-        auto kk = !p.table.unique ? ProbeKernel<false, false, true>
+        auto kk = !p.table.unique ? (p.table.csrPayload != nullptr ? ProbeKernel<false, true, true>
+                                                                   : ProbeKernel<false, false, true>)
                                   : (p.table.slotPayload != nullptr ? ProbeKernel<true, true, true>
                                                                     : ProbeKernel<true, false, true>);
         const int maxGrid = SMs() * BlocksPerSM(reinterpret_cast<const void *>(kk), kProbeThreads, 0);
         g_lastProbeKernel.store(PROBE_KERNEL_GENERAL);
-        kk<<<p.nTiles < maxGrid ? p.nTiles : maxGrid, kProbeThreads, 0, stream>>>(p);
+        kk<<<warpCtas < maxGrid ? static_cast<int>(warpCtas) : maxGrid, kProbeThreads, 0, stream>>>(p);
         return cudaGetLastError();
     }
-    auto kernel = !p.table.unique ? ProbeKernel<false, false, false>
+    auto kernel = !p.table.unique ? (p.table.csrPayload != nullptr ? ProbeKernel<false, true, false>
+                                                                   : ProbeKernel<false, false, false>)
                                   : (p.table.slotPayload != nullptr ? ProbeKernel<true, true, false>
                                                                     : ProbeKernel<true, false, false>);
     if (fast) {
@@ -3243,7 +3380,7 @@ cudaError_t LaunchProbe(const ProbeLaunch &p, cudaStream_t stream)
         kernel = reinterpret_cast<decltype(kernel)>(fk[p.nOut - 1]);
     }
     const int maxGrid = SMs() * BlocksPerSM(reinterpret_cast<const void *>(kernel), kProbeThreads, 0);
-    const int grid = p.nTiles < maxGrid ? p.nTiles : maxGrid;
+    const int grid = warpCtas < maxGrid ? static_cast<int>(warpCtas) : maxGrid;
     g_lastProbeKernel.store(fast ? PROBE_KERNEL_FAST : PROBE_KERNEL_GENERAL);
     kernel<<<grid, kProbeThreads, 0, stream>>>(p);
     return cudaGetLastError();
@@ -3319,8 +3456,19 @@ cudaError_t LaunchBuildSlotBits(const int64_t *arrayEntries, uint64_t range, uin
 cudaError_t LaunchBuildSlotPayload(const ProbeLaunch &p, uint64_t nSlots, uint64_t *payload, cudaStream_t stream)
 {
     const int64_t n = static_cast<int64_t>(nSlots) + 1;
-    const int64_t *entries = p.table.mode == JOIN_ARRAY ? p.table.arrayEntries : p.table.hashEntries;
-    BuildSlotPayloadKernel<<<GridFor(n, 256, 8), 256, 0, stream>>>(entries, nSlots, p.table.sentinelEntry, p, payload);
+    const bool array = p.table.mode == JOIN_ARRAY;
+    const int64_t *entries = array ? p.table.arrayEntries : reinterpret_cast<const int64_t *>(p.table.hashSlots) + 1;
+    BuildSlotPayloadKernel<<<GridFor(n, 256, 8), 256, 0, stream>>>(entries, array ? 1 : 2, nSlots,
+        p.table.sentinelEntry, p, payload);
+    return cudaGetLastError();
+}
+
+cudaError_t LaunchBuildCsrPayload(const ProbeLaunch &p, int64_t n, uint64_t *payload, cudaStream_t stream)
+{
+    if (n == 0) {
+        return cudaSuccess;
+    }
+    BuildCsrPayloadKernel<<<GridFor(n, 256, 8), 256, 0, stream>>>(p.table.csrRows, n, p, payload);
     return cudaGetLastError();
 }
 
@@ -3333,12 +3481,12 @@ cudaError_t LaunchFillI64(int64_t *p, int64_t v, int64_t n, cudaStream_t stream)
     return cudaGetLastError();
 }
 
-cudaError_t LaunchFillU64(uint64_t *p, uint64_t v, int64_t n, cudaStream_t stream)
+cudaError_t LaunchFillHashSlots(uint64_t *slots, int64_t n, cudaStream_t stream)
 {
     if (n == 0) {
         return cudaSuccess;
     }
-    FillU64Kernel<<<GridFor(n, 256, 8), 256, 0, stream>>>(p, v, n);
+    FillHashSlotsKernel<<<GridFor(n, 256, 8), 256, 0, stream>>>(reinterpret_cast<ulonglong2 *>(slots), n);
     return cudaGetLastError();
 }
 

@@ -90,7 +90,7 @@ cudaError_t LaunchKeyStats(const void *keys, const uint8_t *nulls, int64_t n, in
     long long *stats, cudaStream_t stream);
 // ARRAY mode: counts[key - min] += 1; HASH mode: insert keys, counts per slot.
 cudaError_t LaunchBuildCount(JoinTable t, const void *keys, const uint8_t *nulls, int64_t n, int32_t width,
-    uint64_t *hashKeysMutable, uint32_t *counts, uint32_t *sentinelCount, unsigned int *maxCount,
+    uint64_t *hashSlotsMutable, uint32_t *counts, uint32_t *sentinelCount, unsigned int *maxCount,
     int32_t *error, cudaStream_t stream);
 // Exclusive scan of uint32 counts into int64 offsets; total written to *total.
 cudaError_t LaunchScanCounts(const uint32_t *counts, int64_t n, int64_t *offsets, int64_t *blockSums,
@@ -176,11 +176,14 @@ cudaError_t LaunchGatherRows(const void *src, const uint8_t *srcNulls, const int
 // Packs the build output columns named by p.out (side 1, with shifts set) per table slot into
 // payload[nSlots + 1] (the last slot holds the EMPTY-key row of a HASH table).
 cudaError_t LaunchBuildSlotPayload(const ProbeLaunch &p, uint64_t nSlots, uint64_t *payload, cudaStream_t stream);
+// The same for the n positions of p.table.csrRows.
+cudaError_t LaunchBuildCsrPayload(const ProbeLaunch &p, int64_t n, uint64_t *payload, cudaStream_t stream);
 // Occupancy bitmap of an ARRAY table (bit d set iff arrayEntries[d] >= 0) into a buffer of
 // SlotBitsBytes(range) bytes.
 uint64_t SlotBitsBytes(uint64_t range);
 cudaError_t LaunchBuildSlotBits(const int64_t *arrayEntries, uint64_t range, uint32_t *bits, cudaStream_t stream);
 cudaError_t LaunchFillI64(int64_t *p, int64_t v, int64_t n, cudaStream_t stream);
-cudaError_t LaunchFillU64(uint64_t *p, uint64_t v, int64_t n, cudaStream_t stream);
+// n free {key, entry} pairs.
+cudaError_t LaunchFillHashSlots(uint64_t *slots, int64_t n, cudaStream_t stream);
 
 }  // namespace omg

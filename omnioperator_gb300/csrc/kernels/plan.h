@@ -343,8 +343,8 @@ struct JoinTable {
     uint64_t range;           // ARRAY: number of entries
     uint64_t capacity;        // HASH: power of two
     const int64_t *arrayEntries;   // ARRAY: entry per key - minKey, -1 = none
-    const uint64_t *hashKeys;      // HASH: keys, kEmptyKey = free
-    const int64_t *hashEntries;    // HASH: entry per slot
+    // HASH: {key, entry} pairs, so that a lookup's one 16-byte load brings both; key kEmptyKey = free.
+    const uint64_t *hashSlots;
     int64_t sentinelEntry;         // entry of the key equal to kEmptyKey (-1 = none)
     const int32_t *csrRows;        // build rows grouped by key
     int32_t keyWidth;              // probe key width in bytes
@@ -353,6 +353,8 @@ struct JoinTable {
     // packed per table slot (ARRAY: key - minKey; HASH: slot; the EMPTY-key row at `capacity`),
     // so the probe fetches them with the entry instead of gathering by build row afterwards.
     const uint64_t *slotPayload;
+    // Tables with duplicates, under the same conditions: those values packed per position of csrRows.
+    const uint64_t *csrPayload;
     // ARRAY tables with a slot payload: bit d set iff slot d holds a build row.
     const uint32_t *slotBits;
 };

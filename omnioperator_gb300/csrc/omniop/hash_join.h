@@ -111,7 +111,7 @@ public:
     std::string filterText;
     // Build output values packed per table slot, built by the first probe that can use it.
     mutable std::mutex payloadMu;
-    mutable omg::BufferPtr slotPayload;
+    mutable omg::BufferPtr slotPayload;  // or, of a table with duplicates, the CSR payload
     mutable omg::BufferPtr slotBits;  // ARRAY tables: occupancy bitmap of the slots
     mutable bool payloadDecided = false;
     // Partitioned builds, one per partition function (kind, bits, splits), made by the first

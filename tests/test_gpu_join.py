@@ -354,3 +354,58 @@ def test_worker_pipeline_error_reaches_the_caller(gpu):
     pf.close()
     bop.delete()
     bf.close()
+
+
+def _dup_join(rng, nb, npb, dup, sparse, kind, pay2_null=False):
+    """Build rows with 1 to `dup` rows a key; probe keys of which a fifth match none, some NULL."""
+    keys = np.arange(nb, dtype=np.int64)
+    if sparse:
+        keys = keys * 1_000_003 - 5 * 10**11
+    count = rng.integers(1, dup + 1, nb)
+    bkey = np.repeat(keys, count)
+    order = rng.permutation(len(bkey))
+    bkey = bkey[order]
+    p1 = rng.integers(-2**31, 2**31, len(bkey)).astype(np.int32)
+    p2 = rng.integers(-2**31, 2**31, len(bkey)).astype(np.int32)
+    m2 = rng.random(len(bkey)) < 0.1 if pay2_null else None
+    pkey = np.where(rng.random(npb) < 0.8, keys[rng.integers(0, nb, npb)], keys[-1] + 1 + rng.integers(0, 50, npb))
+    pnull = rng.random(npb) < 0.02
+    return bkey, p1, p2, m2, pkey.astype(np.int64), pnull
+
+
+@pytest.mark.parametrize("npb", [1, 31, 127, 128, 129, 4096, 4097, 40_000])
+@pytest.mark.parametrize("dup,sparse,pay2_null", [(1, True, False), (3, True, False), (3, False, False), (70, True, True)])
+def test_probe_segments_and_duplicates(gpu, npb, dup, sparse, pay2_null):
+    """Probe sizes around a warp's 128-row segment and a tile, hash and array tables, unique keys, keys with a
+    few build rows (their payload read in CSR order) and with many (NULL payloads: gathered by row)."""
+    rng = np.random.default_rng(npb + dup)
+    bkey, p1, p2, m2, pkey, pnull = _dup_join(rng, 300, npb, dup, sparse, "inner", pay2_null)
+    I = omg.IntType()
+    for jt in (omg.OMNI_JOIN_TYPE_INNER, omg.OMNI_JOIN_TYPE_LEFT):
+        bf = omg.HashBuilderOperatorFactory(jt, [omg.LongType(), I, I], [0])
+        bop = bf.create_operator()
+        bop.add_input(omg.make_batch([omg.LongType(), I, I], [bkey, p1, p2], [None, None, m2]))
+        bop.get_output()
+        pf = omg.LookupJoinOperatorFactory([omg.LongType()], [0], [0], [1, 2], [I, I], bf)
+        op = pf.create_operator()
+        op.add_input(omg.make_batch([omg.LongType()], [pkey], [pnull]))
+        got = []
+        for b in op.drain():
+            cols = omg.batch_to_numpy(b)
+            omg.free_batch(b)
+            got += list(zip(*[np.where(m, None, v.astype(object)) for v, m in cols]))
+        op.delete()
+        pf.close()
+        bop.delete()
+        bf.close()
+        rows_of = {}
+        for r, k in enumerate(bkey):
+            rows_of.setdefault(int(k), []).append(r)
+        want = []
+        for k, n in zip(pkey, pnull):
+            hits = [] if n else rows_of.get(int(k), [])
+            want += [(int(k), int(p1[r]), None if m2 is not None and m2[r] else int(p2[r])) for r in hits]
+            if not hits and jt == omg.OMNI_JOIN_TYPE_LEFT:
+                want.append((None if n else int(k), None, None))
+        key = lambda t: tuple((x is None, x or 0) for x in t)  # noqa: E731
+        assert sorted(got, key=key) == sorted(want, key=key)
