@@ -3128,10 +3128,21 @@ bool HostSimpleFilterShape(const ProbeLaunch &p)
         p.filter[2].op <= FOP_GTE;
 }
 
-// Only the bitmap kernel packs multi-column keys as it reads them (keys of up to two parts).
+// Two key parts of 4 bytes each.
+bool TwoParts32(const ProbeLaunch &p)
+{
+    return p.pack.nParts == 2 && p.pack.width[0] == 4 && p.pack.width[1] == 4;
+}
+
+// Only the bitmap kernel packs multi-column keys as it reads them (keys of up to two parts). With a filter, its
+// kernels are there for one comparison on two 4-byte parts: a packing pass of its own took 124 us for 2^24
+// probe rows and left the probe to read the 8-byte keys back; together they took 615 us from call to result,
+// the one kernel 383 us.
 bool ProbePacksKeys(const ProbeLaunch &p)
 {
-    return p.pack.nParts <= kFusedPackParts && p.nFilter == 0 && BitsProbeEligible(p, nullptr);
+    const bool filter = p.nFilter > 0;
+    return p.pack.nParts <= kFusedPackParts && (!filter || (TwoParts32(p) && HostSimpleFilterShape(p))) &&
+        BitsProbeEligible(p, nullptr);
 }
 
 cudaError_t LaunchProbe(const ProbeLaunch &p, cudaStream_t stream)
@@ -3218,8 +3229,17 @@ cudaError_t LaunchProbe(const ProbeLaunch &p, cudaStream_t stream)
             OMG_FILTER_INST(4, 0, true, 2),
         };
         static const Inst cmpKeyInst = OMG_FILTER_INST(3, OutLayout(kW8, kW4, kW4), false, 2);
+#define OMG_PACK_FILTER_INST(n, layout)                                                                      \
+    {layout, n, reinterpret_cast<const void *>(ProbeBitsKernel<n, layout, true, true, 2, 2>),               \
+        reinterpret_cast<const void *>(ProbeBitsKernel<n, layout, false, true, 2, 2>)}
+        // One comparison on a key of two 4-byte parts: as two32Insts.
+        static const Inst two32CmpInsts[] = {
+            OMG_PACK_FILTER_INST(4, OutLayout(kW4, kW4, kW4, kW4)), OMG_PACK_FILTER_INST(1, 0),
+            OMG_PACK_FILTER_INST(2, 0), OMG_PACK_FILTER_INST(3, 0), OMG_PACK_FILTER_INST(4, 0),
+        };
 #undef OMG_BITS_INST
 #undef OMG_FILTER_INST
+#undef OMG_PACK_FILTER_INST
         constexpr int kInsts = static_cast<int>(sizeof(insts) / sizeof(insts[0]));
         int pick = -1;
         for (int i = 0; i < kInsts && pick < 0; ++i) {
@@ -3236,8 +3256,8 @@ cudaError_t LaunchProbe(const ProbeLaunch &p, cudaStream_t stream)
         const int single = p.singleBatch ? 0 : 1;
         if (probeCols || p.pack.nParts > 0 || p.nFilter > 0) {
             const bool filter = p.nFilter > 0;
-            const bool packed = p.pack.nParts > 0 && !filter;
-            const bool two32 = packed && p.pack.nParts == 2 && p.pack.width[0] == 4 && p.pack.width[1] == 4;
+            const bool packed = p.pack.nParts > 0;
+            const bool two32 = packed && TwoParts32(p);
             bool cmp = filter && HostSimpleFilterShape(p);
             const Inst *ci = filter ? (cmp ? &cmpInsts[p.nOut - 1] : &filterInsts[p.nOut - 1])
                                     : (packed ? &packedInsts[p.nOut - 1] : &colInsts[p.nOut - 1]);
@@ -3249,7 +3269,8 @@ cudaError_t LaunchProbe(const ProbeLaunch &p, cudaStream_t stream)
                 for (int o = 0; w4 && o < p.nOut; ++o) {
                     w4 = p.out[o].width == 4;
                 }
-                ci = w4 ? &two32Insts[0] : &two32Insts[p.nOut];
+                ci = filter ? (w4 ? &two32CmpInsts[0] : &two32CmpInsts[p.nOut])
+                            : (w4 ? &two32Insts[0] : &two32Insts[p.nOut]);
             }
             const void *ck = single == 0 ? ci->single : ci->tiled;
             cudaError_t cerr = EnsureDynamicSmem(ck, kBitsMaxSmem);

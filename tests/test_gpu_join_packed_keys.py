@@ -167,3 +167,67 @@ def test_keys_too_wide_to_pack_keep_the_tuple_hash(gpu):
     kernel = _check("INNER", [L, L, L], bcols, bmasks, 2, [L, L], pcols, pmasks, [0, 1], [2],
                     batch_sizes=(4096, 3000))
     assert kernel == KIND_KERNEL
+
+
+@pytest.mark.parametrize("kind", ["inner", "left", "semi", "anti"])
+@pytest.mark.parametrize("against", ["literal", "probe", "key"])
+def test_two_int32_keys_with_one_comparison(gpu, kind, against):
+    """The bitmap probe that packs two 4-byte key parts as it reads them and tests one comparison: a payload
+    field with a literal, with another probe column (NULLs in it), and a key part with a literal; ragged
+    batches, NULL parts, parts outside the build's ranges."""
+    rng = np.random.default_rng(len(kind) + len(against))
+    nb, n = 40_000, 300_000
+    code = rng.permutation(nb * 2)[:nb]
+    b1, b2 = (code >> 8).astype(np.int32) - 70, (code & 255).astype(np.int32)
+    q1 = rng.integers(-1000, 1000, nb).astype(np.int32)
+    q2 = rng.integers(-2**31, 2**31, nb).astype(np.int32)
+    pc = rng.integers(-500, 2 * nb + 500, n)
+    p1, p2 = (pc >> 8).astype(np.int32) - 70, (pc & 255).astype(np.int32)
+    x = rng.integers(-1000, 1000, n).astype(np.int32)
+    m1, m2, mx = rng.random(n) < 0.01, rng.random(n) < 0.01, rng.random(n) < 0.05
+    # Joined columns: probe 0..2 (two key parts and x), build 3..6.
+    if against == "literal":
+        filt = omg.Binary(omg.EXPR_GTE, omg.Field(5, I), omg.Literal(0, I))
+    elif against == "probe":
+        filt = omg.Binary(omg.EXPR_LT, omg.Field(2, I), omg.Field(5, I))
+    else:
+        filt = omg.Binary(omg.EXPR_NEQ, omg.Field(1, I), omg.Literal(7, I))
+    jt = {"inner": omg.OMNI_JOIN_TYPE_INNER, "left": omg.OMNI_JOIN_TYPE_LEFT, "semi": omg.OMNI_JOIN_TYPE_LEFT_SEMI,
+          "anti": omg.OMNI_JOIN_TYPE_LEFT_ANTI}[kind]
+    emits = kind in ("inner", "left")
+    bf = omg.HashBuilderOperatorFactory(jt, [I] * 4, [0, 1])
+    bop = bf.create_operator()
+    bop.add_input(omg.make_batch([I] * 4, [b1, b2, q1, q2]))
+    bop.get_output()
+    pf = omg.LookupJoinOperatorFactory([I] * 3, [0, 1], [0, 1], [2, 3] if emits else [], [I, I] if emits else [], bf,
+                                       filter_expr=filt)
+    op = pf.create_operator()
+    op.set_no_more_input(False)
+    for s, e in split(n, [4096, 1000, 50_000]):
+        op.add_input(omg.make_batch([I] * 3, [p1[s:e], p2[s:e], x[s:e]], [m1[s:e], m2[s:e], mx[s:e]]))
+    op.no_more_input()
+    outs = op.drain()
+    assert omg.lib().omg_debug_last_probe_kernel() == BITS_KERNEL
+    parts = [omg.batch_to_numpy(b) for b in outs]
+    omg.free_batches(outs)
+    op.delete()
+    pf.close()
+    bop.delete()
+    bf.close()
+    got = np.stack([np.concatenate([np.where(p[c][1], -2**40, p[c][0].astype(np.int64)) for p in parts])
+                    for c in range(4 if emits else 2)], axis=1)
+    row = np.full(2 * nb, -1)
+    row[code] = np.arange(nb)
+    hit = (pc >= 0) & (pc < 2 * nb) & ~m1 & ~m2
+    br = np.where(hit, row[np.clip(pc, 0, 2 * nb - 1)], -1)
+    hit &= br >= 0
+    f1 = q1[np.clip(br, 0, None)]
+    ok = {"literal": f1 >= 0, "probe": ~mx & (x < f1), "key": p2 != 7}[against]
+    hit &= ok
+    a, b = np.where(m1, -2**40, p1.astype(np.int64)), np.where(m2, -2**40, p2.astype(np.int64))
+    v1 = np.where(hit, f1.astype(np.int64), -2**40)
+    v2 = np.where(hit, q2[np.clip(br, 0, None)].astype(np.int64), -2**40)
+    keep = {"inner": hit, "left": np.ones(n, bool), "semi": hit, "anti": ~hit}[kind]
+    want = np.stack([a, b, v1, v2] if emits else [a, b], axis=1)[keep]
+    assert got.shape == want.shape
+    assert np.array_equal(got[np.lexsort(got.T)], want[np.lexsort(want.T)])
