@@ -585,6 +585,27 @@ __device__ __forceinline__ void InitStates(const AccSpec *accs, int nAccs, int s
     }
 }
 
+// A decimal128 value into an exact sum or a min / max.
+__device__ __forceinline__ void ApplyWide(const AccSpec &s, const char *at, uint64_t *w)
+{
+    const unsigned long long *v = reinterpret_cast<const unsigned long long *>(at);
+    uint64_t lo = __ldg(v);
+    uint64_t hi = __ldg(v + 1);
+    if (s.kind != ACC_WSUM3) {
+        AtomicMinMax128(w, lo, hi, s.kind == ACC_XMIN);
+        return;
+    }
+    if (static_cast<int64_t>(hi) < 0) {  // magnitude = -(hi:lo)
+        lo = ~lo + 1;
+        hi = ~hi + (lo == 0 ? 1u : 0u);
+        w += 4;
+    }
+    Red(w, lo & 0xffffffffull);
+    Red(w + 1, lo >> 32);
+    Red(w + 2, hi & 0xffffffffull);
+    Red(w + 3, hi >> 32);
+}
+
 // ------------------------------------------------------------------ global table
 // Returns the slot index or -1 when no slot was found within maxProbe probes.
 __device__ __forceinline__ int64_t GlobalFind(const AggTable &t, const KeySpec &ks, const RowKey &k, int maxProbe,
@@ -912,8 +933,6 @@ __device__ __forceinline__ void InitSlot(const AggLaunch &p, uint64_t *slot)
     }
     InitStates(p.accs, p.nAccs, p.stateWords, slot + p.table.keyWords);
 }
-
-__device__ __forceinline__ unsigned int *LowHalf(uint64_t *w) { return reinterpret_cast<unsigned int *>(w); }
 
 __device__ __forceinline__ double AsDouble(uint64_t bits, int inKind, int width)
 {

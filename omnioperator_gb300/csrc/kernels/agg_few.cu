@@ -32,9 +32,7 @@ __device__ __forceinline__ void AddTwoSum(double &s, double &c, double x)
 {
     const double sum = __dadd_rn(s, x);
     if (isfinite(sum)) {
-        const double bv = __dsub_rn(sum, s);
-        const double av = __dsub_rn(sum, bv);
-        c = __dadd_rn(c, __dadd_rn(__dsub_rn(s, av), __dsub_rn(x, bv)));
+        c = __dadd_rn(c, SumError(s, x, sum));
     }
     s = sum;
 }
@@ -95,8 +93,8 @@ __device__ __forceinline__ void ApplyFew(const AggLaunch &p, const FewLayout &l,
                     const int64_t x = SignExtend(in.bits[k], s.inWidth);
                     const uint64_t m = x >= 0 ? static_cast<uint64_t>(x) : 0ull - static_cast<uint64_t>(x);
                     if ((m >> 57) != 0) {
-                        Red(to + (x >= 0 ? 0 : 2), m & 0xffffffffull);
-                        Red(to + (x >= 0 ? 1 : 3), m >> 32);
+                        SharedAdd(to + (x >= 0 ? 0 : 2), m & 0xffffffffull);
+                        SharedAdd(to + (x >= 0 ? 1 : 3), m >> 32);
                     } else {
                         (x >= 0 ? pos : neg)[at[k]] += m;
                     }
@@ -104,10 +102,10 @@ __device__ __forceinline__ void ApplyFew(const AggLaunch &p, const FewLayout &l,
                 if ((fold >> k) & 1u) {
                     const uint64_t u = pos[at[k]];
                     const uint64_t v = neg[at[k]];
-                    Red(to, u & 0xffffffffull);
-                    Red(to + 1, u >> 32);
-                    Red(to + 2, v & 0xffffffffull);
-                    Red(to + 3, v >> 32);
+                    SharedAdd(to, u & 0xffffffffull);
+                    SharedAdd(to + 1, u >> 32);
+                    SharedAdd(to + 2, v & 0xffffffffull);
+                    SharedAdd(to + 3, v >> 32);
                     pos[at[k]] = 0;
                     neg[at[k]] = 0;
                 }
@@ -134,7 +132,7 @@ __device__ __forceinline__ void ApplyFew(const AggLaunch &p, const FewLayout &l,
                             e = j == k ? at[j] : e;
                             to = j == k ? states[j] : to;
                         }
-                        AtomicAddCompensated(to + s.word, d[e], 0.0);
+                        SharedAddCompensated(to + s.word, d[e]);
                         d[e] = 0.0;
                     }
                 }

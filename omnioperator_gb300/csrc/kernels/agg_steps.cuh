@@ -196,27 +196,6 @@ __device__ __forceinline__ void ApplyInt(const AccSpec &s, const Run &run, const
     }
 }
 
-// A decimal128 value into an exact sum or a min / max.
-__device__ __forceinline__ void ApplyWide(const AccSpec &s, const char *at, uint64_t *w)
-{
-    const unsigned long long *v = reinterpret_cast<const unsigned long long *>(at);
-    uint64_t lo = __ldg(v);
-    uint64_t hi = __ldg(v + 1);
-    if (s.kind != ACC_WSUM3) {
-        AtomicMinMax128(w, lo, hi, s.kind == ACC_XMIN);
-        return;
-    }
-    if (static_cast<int64_t>(hi) < 0) {  // magnitude = -(hi:lo)
-        lo = ~lo + 1;
-        hi = ~hi + (lo == 0 ? 1u : 0u);
-        w += 4;
-    }
-    Red(w, lo & 0xffffffffull);
-    Red(w + 1, lo >> 32);
-    Red(w + 2, hi & 0xffffffffull);
-    Red(w + 3, hi >> 32);
-}
-
 // Add x to the compensated sum at w (AtomicAddCompensated without the atomics).  A sum of at most
 // 8 + 5 plain additions (a thread's rows, a warp's threads) comes in; every one after that is
 // compensated.

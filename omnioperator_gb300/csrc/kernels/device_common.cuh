@@ -179,6 +179,16 @@ __device__ __forceinline__ void AtomicAddU192(uint64_t *w, uint64_t lo, uint64_t
     }
 }
 
+// The rounding error of sum = fl(a + x), exact while sum is finite (Dekker's Fast2Sum).  Two FP64
+// subtractions, where Knuth's TwoSum takes five: an SM does two FP64 operations a cycle.
+__device__ __forceinline__ double SumError(double a, double x, double sum)
+{
+    constexpr unsigned long long kAbs = 0x7fffffffffffffffull;
+    const bool aLarger = (static_cast<unsigned long long>(__double_as_longlong(a)) & kAbs) >=
+        (static_cast<unsigned long long>(__double_as_longlong(x)) & kAbs);
+    return __dsub_rn(aLarger ? x : a, __dsub_rn(sum, aLarger ? a : x));
+}
+
 // Compensated atomic double sum.  atomicAdd(double) stores fl(old + x) (round to nearest
 // even) and returns `old`, so the adding thread can form the exact rounding error of its own
 // addition with Knuth's TwoSum and push it into the companion word.  s + c then carries the
@@ -196,6 +206,39 @@ __device__ __forceinline__ void AtomicAddCompensated(uint64_t *w, double x, doub
     }
     if (err != 0.0) {
         atomicAdd(s + 1, err);
+    }
+}
+
+// The low 32 bits of a little-endian 64-bit state word.
+__device__ __forceinline__ unsigned int *LowHalf(uint64_t *w) { return reinterpret_cast<unsigned int *>(w); }
+
+// Add to a 64-bit word in shared memory that nobody reads before a barrier: two native 32-bit additions
+// (the second for a high half or a carry only) where the 64-bit one is a compare-and-swap loop.
+__device__ __forceinline__ void SharedAdd(uint64_t *w, uint64_t v)
+{
+    const unsigned int lo = static_cast<unsigned int>(v);
+    unsigned int hi = static_cast<unsigned int>(v >> 32);
+    if (lo != 0) {
+        const unsigned int old = atomicAdd(LowHalf(w), lo);
+        hi += old + lo < lo ? 1u : 0u;
+    }
+    if (hi != 0) {
+        atomicAdd(LowHalf(w) + 1, hi);
+    }
+}
+
+// AtomicAddCompensated on a sum in shared memory.  (A compare-and-swap loop of its own, whose addition is the
+// sum wanted, was twice as slow where groups are contended for as the one that atomicAdd compiles to.)
+__device__ __forceinline__ void SharedAddCompensated(uint64_t *w, double x)
+{
+    double *s = reinterpret_cast<double *>(w);
+    const double old = atomicAdd(s, x);
+    const double sum = __dadd_rn(old, x);
+    if (isfinite(sum)) {
+        const double err = SumError(old, x, sum);
+        if (err != 0.0) {
+            atomicAdd(s + 1, err);
+        }
     }
 }
 
