@@ -707,7 +707,12 @@ OmniStatus HashAggregationOperatorFactory::Init()
             break;
         }
     }
-    p.smemSlots = static_cast<int32_t>(kSmemBudget / (p.slotWords * sizeof(uint64_t)));
+    // Slots in shared memory lie an odd number of words apart: 16 words put a state of every slot on the same
+    // bank.  16-byte states keep the even stride.
+    p.smemStride = std::any_of(p.accs.begin(), p.accs.end(), [](const AccSpec &a) {
+        return a.kind == omg::ACC_XMIN || a.kind == omg::ACC_XMAX;
+    }) ? p.slotWords : (p.slotWords | 1);
+    p.smemSlots = static_cast<int32_t>(kSmemBudget / (p.smemStride * sizeof(uint64_t)));
     p.rowsPerBatch = GetMaxRowCount(rowBytes);
     p.outContainer.assign(p.outs.size(), 0);
     for (size_t i : containerAt) {
@@ -927,6 +932,7 @@ omg::AggLaunch MakeAggLaunch(const AggPlan &plan, uint64_t *slots, uint64_t capa
     p.table.slots = slots;
     p.table.capacity = capacity;
     p.table.slotWords = plan.slotWords;
+    p.smemStride = plan.smemStride;
     p.table.keyWords = plan.keyWords;
     p.table.specialUsed = special;
     p.table.groupCount = stats;
@@ -1127,7 +1133,7 @@ void HashAggregationOperator::Decide(omg::BatchTable &bt, cudaStream_t s)
     // Partitions: enough that one partition's groups fill a CTA's shared table to kPartLoad.
     const bool wantPart = strategy_ == 3 || (strategy_ == 0 && rows >= kSketchMinRows);
     if (wantPart && im.estimate > 0) {
-        const double perCta = kPartLoad * omg::AggPartSmemSlots(plan_.slotWords);
+        const double perCta = kPartLoad * omg::AggPartSmemSlots(plan_.smemStride);
         const uint64_t need = NextPow2(static_cast<uint64_t>(std::ceil(static_cast<double>(im.estimate) / perCta)));
         if (need <= static_cast<uint64_t>(omg::kMaxParts) && perCta >= 1.0) {
             int bits = 0;
@@ -1207,10 +1213,10 @@ struct HashAggregationOperator::RadixRun {
 };
 
 namespace {
-// Rows of a unit, and of the largest partition that is one unit: a hot key's partition is spread over
-// several CTAs, and the merge of a unit's table (some thousand slots) stays small beside its rows.
+// Most rows of a unit (partitions of up to two units' rows stay whole): a hot key's partition is spread over
+// several CTAs, and the merge of a unit's table (some thousand slots) stays small beside its rows.  Fewer
+// rows make smaller units, down to one step, until every CTA has one.
 constexpr uint64_t kRadixUnitRows = 1 << 14;
-constexpr uint64_t kRadixWholeRows = 1 << 15;
 // Target fill of a unit's slots: the partitions' group counts vary by a few percent, and the estimate by
 // 1.6 (one standard error of 2^12 registers); groups beyond the slots go to the global table.
 constexpr double kRadixLoad = 0.85;
@@ -1263,7 +1269,7 @@ bool HashAggregationOperator::PlanRadix(omg::BatchTable &bt, RadixRun &run, cuda
 {
     Impl &im = *impl_;
     const uint64_t rows = static_cast<uint64_t>(bt.TotalRows());
-    const int32_t nSlots = omg::AggRadixSlots(plan_.slotWords, &run.indexSize);
+    const int32_t nSlots = omg::AggRadixSlots(plan_.smemStride, &run.indexSize);
     if (nSlots < 64 || rows >= (uint64_t(1) << 32) || !LayoutRecord(plan_, bt, run.layout)) {
         return false;
     }
@@ -1295,6 +1301,8 @@ bool HashAggregationOperator::PlanRadix(omg::BatchTable &bt, RadixRun &run, cuda
         const uint64_t unitSlots = static_cast<uint64_t>(nSlots) << run.passBits;
         std::vector<unsigned int> start(nParts);
         std::vector<omg::RadixUnit> whole;
+        const uint64_t perCta = (rows / (2 * omg::DeviceSMCount()) + omg::kRadixStepRows) / omg::kRadixStepRows;
+        const uint64_t unitRows = std::min<uint64_t>(kRadixUnitRows, perCta * omg::kRadixStepRows);
         uint64_t first = 0;
         uint64_t multi = 0;
         for (uint32_t q = 0; q < nParts; ++q) {
@@ -1303,10 +1311,10 @@ bool HashAggregationOperator::PlanRadix(omg::BatchTable &bt, RadixRun &run, cuda
                 n += h[f];
             }
             start[q] = static_cast<unsigned int>(first);
-            if (n > kRadixWholeRows) {
+            if (n > 2 * unitRows) {
                 ++multi;
-                for (uint64_t r = 0; r < n; r += kRadixUnitRows) {
-                    const uint64_t m = std::min(kRadixUnitRows, n - r);
+                for (uint64_t r = 0; r < n; r += unitRows) {
+                    const uint64_t m = std::min(unitRows, n - r);
                     run.units.push_back(omg::RadixUnit{static_cast<uint32_t>(first + r), static_cast<uint32_t>(m), 1, 0});
                     run.spillCap += std::min(m, unitSlots);
                 }
@@ -1580,7 +1588,7 @@ void HashAggregationOperator::Flush(bool last)
     if (few) {
         smemSlots = 0;
     } else if (im.partBits >= 0) {
-        smemSlots = omg::AggPartSmemSlots(plan_.slotWords);
+        smemSlots = omg::AggPartSmemSlots(plan_.smemStride);
         Partition(bt, p, part, s);
         rowBatches = p.batches;
     }
@@ -1613,7 +1621,7 @@ void HashAggregationOperator::Flush(bool last)
         ra.dense = radixRun.dense.Get();
         ra.denseCount = im.stats.Get() + 4;
         ra.denseCap = radixRun.denseCap;
-        p.smemSlots = omg::AggRadixSlots(plan_.slotWords, &ra.indexSize);
+        p.smemSlots = omg::AggRadixSlots(plan_.smemStride, &ra.indexSize);
         CudaCheck(omg::LaunchRadixAgg(p, radixRun.layout, ra, spillA.Get(), nSpill, static_cast<uint32_t>(spillCap), s),
             "radix aggregation");
         ++counters_[0];
@@ -2164,7 +2172,7 @@ bool HashAggregationOperator::ExtractSmall()
         im.stream.SetUser(userStream_);
     }
     cudaStream_t s = im.stream.Get();
-    const int32_t nSlots = omg::AggSmallSlots(plan_.slotWords, &a.indexSize);
+    const int32_t nSlots = omg::AggSmallSlots(plan_.smemStride, &a.indexSize);
     if (nSlots < 64) {
         return false;
     }

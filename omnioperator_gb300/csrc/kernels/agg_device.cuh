@@ -782,9 +782,9 @@ __device__ __forceinline__ void ProcessRow(const AggLaunch &p, int32_t batchIdx,
     const int sw = p.table.slotWords;
     const int kw = p.table.keyWords;
     if (smSlots > 0 && in.k.special < 0) {
-        int i = SmemFind(sm, smSlots, sw, p.key, in.k, kKind);
+        int i = SmemFind(sm, smSlots, p.smemStride, p.key, in.k, kKind);
         if (i >= 0) {
-            UpdateStates(p, b, row, in, sm + static_cast<int64_t>(i) * sw + kw);
+            UpdateStates(p, b, row, in, sm + static_cast<int64_t>(i) * p.smemStride + kw);
             return;
         }
     }

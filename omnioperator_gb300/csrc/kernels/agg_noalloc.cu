@@ -190,6 +190,7 @@ NoAllocStatus RunAggNoAlloc(const NoAllocPlan &plan, const void *const *cols, co
     p.tiles = tiles;
     p.nTiles = nTiles;
     p.smemSlots = plan.smemSlots;
+    p.smemStride = plan.slotWords;
     if ((err = LaunchAggInitTable(p, stream)) != cudaSuccess) {
         return fail(err, "init table");
     }

@@ -322,6 +322,8 @@ __device__ __noinline__ void GlobalRecord(const AggLaunch &p, const RecLayout &l
     UpdateStates(p, b, 0, in, p.table.slots + g * p.table.slotWords + p.table.keyWords);
 }
 
+static_assert(kStepRows == kRadixStepRows, "units are whole steps");
+
 template <int kKind>
 __global__ void __launch_bounds__(kStepThreads, 2) RadixAggKernel(const __grid_constant__ AggLaunch p,
     const __grid_constant__ RecLayout l, const __grid_constant__ RadixAgg a, const __grid_constant__ SpillArgs sp)
@@ -335,10 +337,11 @@ __global__ void __launch_bounds__(kStepThreads, 2) RadixAggKernel(const __grid_c
     __shared__ unsigned int warpSums[kStepThreads / 32];
     __shared__ unsigned long long denseBase;
     const int sw = p.table.slotWords;
+    const int ss = p.smemStride;
     const int kw = p.table.keyWords;
     const unsigned int nSlots = static_cast<unsigned int>(p.smemSlots);
     const int nAll = static_cast<int>(nSlots) + kSpecialSlots;
-    const StepTable tab = MakeStepTable(smem, nAll, sw, kw, nSlots, a.indexSize, &used, warpSums);
+    const StepTable tab = MakeStepTable(smem, nAll, ss, kw, nSlots, a.indexSize, &used, warpSums);
     InitStepTable(p, tab);
     if (threadIdx.x == 0) {
         newGroups = 0;
@@ -371,17 +374,17 @@ __global__ void __launch_bounds__(kStepThreads, 2) RadixAggKernel(const __grid_c
             const unsigned int groups = min(used, nSlots);
             if (threadIdx.x < kSpecialSlots) {
                 const int s = threadIdx.x;
-                uint64_t *slot = smem + static_cast<int64_t>(s) * sw;
+                uint64_t *slot = smem + static_cast<int64_t>(s) * ss;
                 if (slot[kw + p.accs[0].word] != 0) {
                     atomicExch(&p.table.specialUsed[s], 1u);
                     MergeStates(p, p.accs, p.nAccs, slot + kw, p.table.slots + (p.table.capacity + s) * sw + kw);
                     InitSlot(p, slot);
                 }
             }
-            uint64_t *first = smem + static_cast<int64_t>(kSpecialSlots) * sw;
+            uint64_t *first = smem + static_cast<int64_t>(kSpecialSlots) * ss;
             if (unit.multi != 0) {
                 for (unsigned int i = threadIdx.x; i < groups; i += kStepThreads) {
-                    MergeRecord<kKind>(p, sp, first + static_cast<int64_t>(i) * sw, &newGroups);
+                    MergeRecord<kKind>(p, sp, first + static_cast<int64_t>(i) * ss, &newGroups);
                 }
             } else {
                 // A whole partition: append its groups.
@@ -394,13 +397,14 @@ __global__ void __launch_bounds__(kStepThreads, 2) RadixAggKernel(const __grid_c
                 } else {
                     uint64_t *dst = a.dense + denseBase * sw;
                     for (unsigned int w = threadIdx.x; w < groups * sw; w += kStepThreads) {
-                        dst[w] = first[w];
+                        const unsigned int g = w / sw;
+                        dst[w] = first[g * ss + (w - g * sw)];
                     }
                 }
             }
             __syncthreads();
             for (unsigned int i = threadIdx.x; i < groups; i += kStepThreads) {
-                InitSlot(p, first + static_cast<int64_t>(i) * sw);
+                InitSlot(p, first + static_cast<int64_t>(i) * ss);
             }
             for (int i = threadIdx.x; i < a.indexSize; i += kStepThreads) {
                 tab.index[i] = 0;
@@ -443,9 +447,9 @@ __global__ void __launch_bounds__(512) RadixRetryKernel(const __grid_constant__ 
 
 }  // namespace
 
-int32_t AggRadixSlots(int32_t slotWords, int32_t *indexSize)
+int32_t AggRadixSlots(int32_t smemStride, int32_t *indexSize)
 {
-    return StepTableSlots(slotWords, kRadixSmemBytes, indexSize);
+    return StepTableSlots(smemStride, kRadixSmemBytes, indexSize);
 }
 
 cudaError_t LaunchRadixKeys(const AggLaunch &p, unsigned int *hist, unsigned int *regs, cudaStream_t stream)

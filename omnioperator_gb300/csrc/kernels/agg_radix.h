@@ -17,6 +17,7 @@ constexpr int kRadixFineBits = 14;
 constexpr int kRadixFineParts = 1 << kRadixFineBits;
 constexpr int kRadixShift = 18;
 constexpr int kRadixMaxPassBits = 4;
+constexpr int kRadixStepRows = 2048;  // rows that a CTA sorts and adds up at a time
 constexpr int kRadixHllBits = 12;
 constexpr int kRadixHllRegs = 1 << kRadixHllBits;
 
@@ -64,7 +65,7 @@ struct RadixAgg {
 };
 
 // Groups that a CTA's shared table holds, and the size of its index.
-int32_t AggRadixSlots(int32_t slotWords, int32_t *indexSize);
+int32_t AggRadixSlots(int32_t smemStride, int32_t *indexSize);
 // One pass over the keys of p's tiles: rows per fine partition, hist[kRadixFineParts], and HyperLogLog
 // registers of the key hashes, regs[kRadixHllRegs] (both zeroed by the caller).
 cudaError_t LaunchRadixKeys(const AggLaunch &p, unsigned int *hist, unsigned int *regs, cudaStream_t stream);

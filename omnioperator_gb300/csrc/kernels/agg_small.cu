@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) AggSmallKernel(const __grid_c
     __shared__ unsigned int used;
     __shared__ unsigned int missed;
     __shared__ unsigned int warpSums[kStepThreads / 32];
-    const int sw = p.table.slotWords;
+    const int sw = p.smemStride;
     const int kw = p.table.keyWords;
     const unsigned int nSlots = static_cast<unsigned int>(p.smemSlots);
     const int nAll = static_cast<int>(nSlots) + kSpecialSlots;
@@ -111,9 +111,9 @@ __global__ void __launch_bounds__(kStepThreads, 1) AggSmallKernel(const __grid_c
 
 }  // namespace
 
-int32_t AggSmallSlots(int32_t slotWords, int32_t *indexSize)
+int32_t AggSmallSlots(int32_t smemStride, int32_t *indexSize)
 {
-    return StepTableSlots(slotWords, kSmallSmemBytes, indexSize);
+    return StepTableSlots(smemStride, kSmallSmemBytes, indexSize);
 }
 
 cudaError_t LaunchAggSmall(const AggLaunch &p, const AggExtract &e, const SmallArgs &a, cudaStream_t stream)

@@ -31,7 +31,7 @@ struct SmallArgs {
 };
 
 // Groups that the launch can hold, and the size of its index.
-int32_t AggSmallSlots(int32_t slotWords, int32_t *indexSize);
+int32_t AggSmallSlots(int32_t smemStride, int32_t *indexSize);
 // p: key, accumulators, table.slotWords / keyWords, smemSlots; e: outputs (their NULL bitmaps need not be
 // cleared), error and nAmbiguous.
 cudaError_t LaunchAggSmall(const AggLaunch &p, const AggExtract &e, const SmallArgs &a, cudaStream_t stream);

@@ -25,7 +25,7 @@ cudaError_t LaunchAgg(const AggLaunch &p, uint64_t *spill, unsigned int *nSpill,
     const uint64_t *spillIn, uint32_t nSpillIn, int gridBlocks, cudaStream_t stream);
 // Partitioned aggregation: shared slots per CTA of a partitioned launch, and the partition pass
 // (histogram, layout, scatter) over p's batches into a's buffers; a.hist must be zero.
-int32_t AggPartSmemSlots(int32_t slotWords);
+int32_t AggPartSmemSlots(int32_t smemStride);
 cudaError_t LaunchAggPartition(const AggLaunch &p, const PartArgs &a, cudaStream_t stream);
 // Key sketch of nSample rows stratified over p's tiles; stats as described at kSketchStats.
 // tabKeys / tabCounts hold kSketchCap entries.

@@ -174,6 +174,7 @@ struct AggLaunch {
     const unsigned long long *retryIn;
     uint32_t nRetryIn;
     int32_t smemSlots;  // per-CTA shared-memory pre-aggregation slots (0 = off)
+    int32_t smemStride; // words from one of them to the next (slotWords or one more)
     int32_t *error;     // sticky device error code (0 = none)
     long long waitBudget;  // clock64 ticks a thread may wait for another's slot publication
     // Partitioned launches (nParts > 0): the batches are hash partitions, tiles

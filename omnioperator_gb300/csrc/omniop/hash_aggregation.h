@@ -47,6 +47,7 @@ struct AggPlan {
     int32_t stateWords = 0;
     int32_t keyWords = 0;                  // words before the state in a table slot
     int32_t slotWords = 0;
+    int32_t smemStride = 0;                // words from a shared table's slot to the next
     std::vector<omg::OutSpec> outs;        // pointers filled at extraction
     std::vector<type::DataTypePtr> outTypes;
     int32_t rowsPerBatch = 0;
