@@ -1262,6 +1262,33 @@ bool LayoutRecord(const AggPlan &plan, const omg::BatchTable &bt, omg::RecLayout
 }
 }  // namespace
 
+// Whether the rows of a first flush, whose groups fit the partitions, are better sorted by step than added to
+// the partitions' tables row by row.
+// A double sum there is a compare-and-swap loop, and a CTA takes the rows of one group one after the other, at
+// some 0.35 us; the radix passes cost about 0.1 ms and 50 ps a row more.  4M rows in 10,000 groups, six
+// aggregates: the hottest key with a tenth of the rows 12.3 ms against 0.65, uniform 0.40 against 0.62;
+// 300,000 rows in 1,000 groups, Zipf, 0.34 against 0.33.
+// Two-column keys take the tables longer the more groups they hold: with a double sum the line is at 900
+// groups and 2^21 rows (at 2^22 rows 700 groups 0.56 ms against 0.77, 1,000 groups 0.94 against 0.73, 10,000
+// groups 1.41 against 0.77; at 2^20 rows 1,000 groups 0.39 against 0.45), and without one at 2^22 rows in
+// several partitions (10,000 groups 0.70 against 0.58, 1,000 in one partition 0.44 against 0.57).
+bool HashAggregationOperator::RadixBeatsPartitions(int64_t rows) const
+{
+    const Impl &im = *impl_;
+    const bool doubles = std::any_of(plan_.accs.begin(), plan_.accs.end(),
+        [](const AccSpec &a) { return a.kind == omg::ACC_DSUM; });
+    if (plan_.key.kind == omg::KEY_PACKED &&
+        (doubles ? im.estimate >= 900 && rows >= (int64_t(1) << 21) : im.partBits > 0 && rows >= (int64_t(1) << 22))) {
+        return true;
+    }
+    if (!doubles || im.sketch[0] == 0) {
+        return false;
+    }
+    const double hottest = static_cast<double>(std::max(im.sketch[1], im.sketch[8])) / static_cast<double>(im.sketch[0]);
+    const double perCta = hottest * static_cast<double>(rows) * (1 << im.partBits) / omg::DeviceSMCount();
+    return perCta * 0.35 > 100.0 + static_cast<double>(rows) * 50e-6;
+}
+
 // The key pass and what follows from it: how many partitions, their records and units, and every
 // buffer of the run.  False (nothing changed): the plan's rows do not fit a record, there are more
 // groups than the passes hold, or the device has no memory for the records.
@@ -1534,12 +1561,24 @@ void HashAggregationOperator::Flush(bool last)
         Decide(bt, s);
     }
     FoldDense(s);
-    // More groups than the partitions of the partitioned strategy hold: the radix aggregation, on the
-    // operator's first rows (later ones go to the table).  The line is where the estimate leaves the
-    // partitioned strategy; the global table it replaces there was behind at every size measured.
+    // As few groups as fit every thread's own states: no partitions and no atomics (0.15 ms against 1.22 ms
+    // for 2^22 rows of 6 groups).  A group that the estimate missed goes to the global table.
+    omg::FewLayout fewLayout;
+    bool few = false;
+    if (strategy_ == 0 && im.partBits >= 0) {
+        uint32_t nullable = 0;
+        for (size_t i = 0; i < plan_.inputCols.size(); ++i) {
+            nullable |= bt.AnyNulls(static_cast<int32_t>(i)) ? 1u << i : 0u;
+        }
+        few = omg::LayoutAggFew(MakeLaunch(plan_, nullptr, 0, nullptr, nullptr), nullable, &fewLayout) &&
+            im.estimate + 2 <= static_cast<uint64_t>(fewLayout.maxGroups + fewLayout.firstSlot);
+    }
+    // The radix aggregation, on the operator's first rows (later ones go to the table): more groups than the
+    // partitions of the partitioned strategy hold (the global table it replaces there was behind at every
+    // size measured), or rows that those take longer for.
     RadixRun radixRun;
-    const bool radix = strategy_ == 0 && im.capacity == 0 && im.partBits < 0 && im.estimate > 0 &&
-        rows >= kSketchMinRows && PlanRadix(bt, radixRun, s);
+    const bool radix = strategy_ == 0 && im.capacity == 0 && im.estimate > 0 && rows >= kSketchMinRows && !few &&
+        (im.partBits < 0 || RadixBeatsPartitions(rows)) && PlanRadix(bt, radixRun, s);
     // Create the table on first use, sized for the group estimate (load factor <= 1/2).
     if (im.capacity == 0) {
         uint64_t cap = radix ? NextPow2(radixRun.tableGroups * 2)
@@ -1573,19 +1612,7 @@ void HashAggregationOperator::Flush(bool last)
     p.batches = bt.DeviceBatches();
     p.tiles = bt.DeviceTiles();
     p.nTiles = bt.NumTiles();
-    // As few groups as fit every thread's own states: no partitions and no atomics (0.15 ms against 1.22 ms
-    // for 2^22 rows of 6 groups).  A group that the estimate missed goes to the global table.
-    omg::FewLayout fewLayout;
-    bool few = false;
-    if (strategy_ == 0 && im.partBits >= 0) {
-        uint32_t nullable = 0;
-        for (size_t i = 0; i < plan_.inputCols.size(); ++i) {
-            nullable |= bt.AnyNulls(static_cast<int32_t>(i)) ? 1u << i : 0u;
-        }
-        few = omg::LayoutAggFew(p, nullable, &fewLayout) &&
-            im.estimate + 2 <= static_cast<uint64_t>(fewLayout.maxGroups + fewLayout.firstSlot);
-    }
-    if (few) {
+    if (few || radix) {
         smemSlots = 0;
     } else if (im.partBits >= 0) {
         smemSlots = omg::AggPartSmemSlots(plan_.smemStride);

@@ -149,6 +149,7 @@ private:
     void Decide(omg::BatchTable &bt, cudaStream_t s);
     void Partition(omg::BatchTable &bt, omg::AggLaunch &p, PartBuffers &pb, cudaStream_t s);
     bool PlanRadix(omg::BatchTable &bt, RadixRun &run, cudaStream_t s);
+    bool RadixBeatsPartitions(int64_t rows) const;
     void FoldDense(cudaStream_t s);
     struct ExtractRun;
     // last: no more rows will come.

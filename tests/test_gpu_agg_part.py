@@ -54,3 +54,43 @@ def test_word_sums_in_halves(gpu, groups, rows, sign):
         x = d[live & (inv == g)]
         if len(x):
             assert abs(cols[5][0][order][g] - math.fsum(x)) <= 130 * 2.0**-53 * np.abs(x).sum()
+
+
+@pytest.mark.parametrize("keys", [1, 2])
+@pytest.mark.parametrize("share", [0.02, 0.3, 0.95])
+@pytest.mark.parametrize("groups", [500, 9000])
+def test_hot_groups_with_double_sums(gpu, keys, share, groups):
+    """Groups that fit the partitions, some of whose rows are one key's (or the NULL key's): AUTO takes the
+    partitions or the radix passes, by the share of the hottest key and the width of the key."""
+    rng = np.random.default_rng(groups + keys)
+    rows = 400_003
+    key = rng.integers(0, groups, rows)
+    hot = rng.random(rows)
+    key[hot < share] = 3
+    km = hot < share / 3
+    v = rng.integers(-2**40, 2**40, rows)
+    d = rng.standard_normal(rows)
+    dm = rng.random(rows) < 0.05
+    kcols, ktypes = ([key], [L]) if keys == 1 else ([key, (key % 7).astype(np.int32)], [L, I])
+    k = len(kcols)
+    cols, _ = run_agg(list(range(k)), ktypes, [[k], [k + 1], [k + 1], []], [[L], [D], [D], []], [[L], [D], [D], [L]],
+                      [SUM, SUM, MIN, CALL], kcols + [v, d], ktypes + [L, D],
+                      nulls=[km] + [None] * k + [dm], batch_sizes=(100_000, 4096))
+    code = np.where(km, groups + (key % 7 if keys == 2 else 0), key)
+    uniq, inv = np.unique(code, return_inverse=True)
+    got = np.where(cols[0][1], groups + (cols[1][0] if keys == 2 else 0), cols[0][0])
+    order = np.argsort(got)
+    assert np.array_equal(got[order], uniq)
+    want = np.zeros(len(uniq), np.int64)
+    np.add.at(want, inv, v)
+    assert np.array_equal(cols[k][0][order], want)
+    low = np.full(len(uniq), np.inf)
+    np.minimum.at(low, inv[~dm], d[~dm])
+    some = np.bincount(inv[~dm], minlength=len(uniq)) > 0
+    assert np.array_equal(cols[k + 2][0][order][some], low[some])
+    assert np.array_equal(cols[k + 3][0][order], np.bincount(inv, minlength=len(uniq)))
+    mass = np.bincount(inv[~dm], weights=np.abs(d[~dm]), minlength=len(uniq))
+    for g in list(range(0, len(uniq), 97)) + [3, len(uniq) - 1]:
+        # Each partial table leaves at most 64 plain additions of its own rows: 64 * 2^-53 of the group's mass.
+        exact = math.fsum(d[~dm & (inv == g)])
+        assert abs(cols[k + 1][0][order][g] - exact) <= 66 * 2.0**-53 * mass[g]
