@@ -3137,12 +3137,18 @@ bool TwoParts32(const ProbeLaunch &p)
 // Only the bitmap kernel packs multi-column keys as it reads them (keys of up to two parts). With a filter, its
 // kernels are there for one comparison on two 4-byte parts: a packing pass of its own took 124 us for 2^24
 // probe rows and left the probe to read the 8-byte keys back; together they took 615 us from call to result,
-// the one kernel 383 us.
+// the one kernel 383 us.  With 8-byte outputs the widths are run-time ones there, and it was behind (1.97 ms
+// against 1.89 for 28M rows).
 bool ProbePacksKeys(const ProbeLaunch &p)
 {
-    const bool filter = p.nFilter > 0;
-    return p.pack.nParts <= kFusedPackParts && (!filter || (TwoParts32(p) && HostSimpleFilterShape(p))) &&
-        BitsProbeEligible(p, nullptr);
+    bool fused = true;
+    if (p.nFilter > 0) {
+        fused = TwoParts32(p) && HostSimpleFilterShape(p);
+        for (int o = 0; o < p.nOut; ++o) {
+            fused = fused && p.out[o].width == 4;
+        }
+    }
+    return p.pack.nParts <= kFusedPackParts && fused && BitsProbeEligible(p, nullptr);
 }
 
 cudaError_t LaunchProbe(const ProbeLaunch &p, cudaStream_t stream)
