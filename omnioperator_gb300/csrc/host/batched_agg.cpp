@@ -27,6 +27,11 @@ constexpr int32_t kDefaultVariant = 1;  // 256 threads, 4 CTAs per SM
 // Probe limit of the task tables (sized for a load of 1/2 or less): a task whose rows need more
 // probes has outgrown its table and is re-run exactly.
 constexpr int32_t kTaskMaxProbe = 96;
+// Tasks of at most this load over all partitions of a shared table go by units; a table of a unit has slots for
+// twice the groups expected.  A unit has rows enough for its merge to stay small beside them.
+constexpr double kUnitLoad = 0.6;
+constexpr int32_t kUnitMinTiles = 8;
+constexpr int32_t kUnitMaxTiles = 64;
 
 uint64_t NextPow2(uint64_t v)
 {
@@ -100,6 +105,10 @@ struct BatchedAggregation::Impl {
     DevArray<int64_t> offsets;
     DevArray<omg::TaskChunk> chunks;
     int32_t nChunks = 0;
+    DevArray<omg::TaskUnit> units;
+    DevArray<uint8_t> shared;
+    DevArray<unsigned int> nextUnit;
+    int32_t nUnits = 0;
     DevArray<unsigned long long> cursor;
     DevArray<int64_t> blockSums;
     DevArray<long long> total;
@@ -150,6 +159,7 @@ struct BatchedAggregation::Impl {
         p.nTiles = bt.NumTiles();
         p.taskTables = tables.Get();
         p.taskFailed = failed.Get();
+        p.taskShared = shared.Get();
         return p;
     }
 
@@ -161,6 +171,7 @@ struct BatchedAggregation::Impl {
         CudaCheck(cudaMemsetAsync(failed.Get(), 0, sizeof(uint32_t) * n, s), "reset task flags");
         CudaCheck(omg::LaunchAggInitTable(p, s), "init task tables");
         CudaCheck(omg::LaunchAggTasks(p, variant, s), "batched aggregation");
+        CudaCheck(omg::LaunchAggTaskUnits(p, units.Get(), nUnits, nextUnit.Get(), s), "batched aggregation by units");
         CudaCheck(omg::LaunchAggTaskCount(tables.Get(), n, chunks.Get(), nChunks, plan.key.kind, groups.Get(), s), "count task groups");
         CudaCheck(omg::LaunchAggTaskPad(groups.Get(), n, counts.Get(), s), "pad task regions");
         CudaCheck(omg::LaunchScanCounts(counts.Get(), n, offsets.Get(), blockSums.Get(), total.Get(), s),
@@ -292,6 +303,43 @@ struct BatchedAggregation::Impl {
         CudaCheck(cudaMemcpyAsync(chunks.Get(), hostChunks.data(), sizeof(omg::TaskChunk) * hostChunks.size(),
                       cudaMemcpyHostToDevice, s),
             "upload task chunks");
+        std::vector<omg::TaskUnit> hostUnits;
+        std::vector<uint8_t> hostShared(n, 0);
+        const int32_t maxSlots = omg::AggPartSmemSlots(plan.smemStride);
+        // Double sums of few groups are faster in the global table, whose atomics are not compare-and-swap loops.
+        const uint64_t minGroups = std::any_of(plan.accs.begin(), plan.accs.end(),
+            [](const omg::AccSpec &a) { return a.kind == omg::ACC_DSUM; }) ? 256 : 0;
+        int32_t tile = 0;
+        for (int32_t t = 0; t < n; ++t) {
+            const int32_t tiles = static_cast<int32_t>((tasks[t]->GetRowCount() + omg::kTileRows - 1) / omg::kTileRows);
+            int32_t bits = 0;
+            while (bits <= omg::kTaskMaxPartBits &&
+                static_cast<double>(estimate[t]) > kUnitLoad * maxSlots * (1 << bits)) {
+                ++bits;
+            }
+            if (bits <= omg::kTaskMaxPartBits && estimate[t] >= minGroups) {
+                hostShared[t] = 1;
+                const int64_t slots = std::max<int64_t>(64, 2 * (static_cast<int64_t>(estimate[t]) >> bits));
+                const int64_t want = 8 * static_cast<int64_t>(estimate[t]) / omg::kTileRows + 1;
+                const int32_t step = static_cast<int32_t>(
+                    std::min<int64_t>(kUnitMaxTiles, std::max<int64_t>(kUnitMinTiles, want)));
+                for (int32_t first = 0; first < tiles; first += step) {
+                    for (int32_t part = 0; part < (1 << bits); ++part) {
+                        hostUnits.push_back(omg::TaskUnit{t, tile + first, std::min(step, tiles - first),
+                            static_cast<int32_t>(std::min<int64_t>(slots, maxSlots)), bits, part});
+                    }
+                }
+            }
+            tile += tiles;
+        }
+        nUnits = static_cast<int32_t>(hostUnits.size());
+        units.Reset(std::max<size_t>(hostUnits.size(), 1), s);
+        nextUnit.Reset(1, s);
+        shared.Reset(n, s);
+        CudaCheck(cudaMemcpyAsync(units.Get(), hostUnits.data(), sizeof(omg::TaskUnit) * hostUnits.size(),
+                      cudaMemcpyHostToDevice, s),
+            "upload task units");
+        CudaCheck(cudaMemcpyAsync(shared.Get(), hostShared.data(), n, cudaMemcpyHostToDevice, s), "upload task flags");
         cursor.Reset(n, s);
         blockSums.Reset(static_cast<size_t>(n) / 1024 + 2, s);
         total.Reset(1, s, true);
@@ -306,7 +354,7 @@ struct BatchedAggregation::Impl {
             outCols[o].nulls = omg::Buffer::NewDevice(omg::NullBitmapBytes(static_cast<int64_t>(outBound)), s, true);
             outCols[o].hasNull = plan.outs[o].kind != omg::OUT_COUNT && plan.outs[o].kind != omg::OUT_IS_EMPTY;
         }
-        CudaCheck(cudaStreamSynchronize(s), "cudaStreamSynchronize");  // hostTables and hostChunks are on the stack
+        CudaCheck(cudaStreamSynchronize(s), "cudaStreamSynchronize");  // the host vectors are on the stack
         prepareUs = NowUs() - t0;
         Tune(s);
         // Capture the per-run sequence once (a private stream is needed for capture).

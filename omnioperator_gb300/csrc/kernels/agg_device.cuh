@@ -809,12 +809,9 @@ struct SpillArgs {
     uint32_t nSpillIn;
 };
 
-template <int kKind>
-__device__ __forceinline__ void MergeRecord(const AggLaunch &p, const SpillArgs &sp, const uint64_t *rec,
-    unsigned int *newGroups)
+// The key of a record or a slot.
+template <int kKind> __device__ __forceinline__ RowKey RecordKey(const AggLaunch &p, const uint64_t *rec)
 {
-    const int sw = p.table.slotWords;
-    const int kw = p.table.keyWords;
     RowKey k;
     k.special = -1;
     k.w[0] = k.w[1] = k.w[2] = 0;
@@ -828,6 +825,16 @@ __device__ __forceinline__ void MergeRecord(const AggLaunch &p, const SpillArgs 
         }
         k.hash = KeyWordsHash(k, p.key.words);
     }
+    return k;
+}
+
+template <int kKind>
+__device__ __forceinline__ void MergeRecord(const AggLaunch &p, const SpillArgs &sp, const uint64_t *rec,
+    unsigned int *newGroups)
+{
+    const int sw = p.table.slotWords;
+    const int kw = p.table.keyWords;
+    const RowKey k = RecordKey<kKind>(p, rec);
     bool inserted = false;
     int64_t g = GlobalFind(p.table, p.key, k, p.maxProbe, p.error, &inserted, p.waitBudget, kKind);
     if (g < 0) {

@@ -40,6 +40,9 @@ cudaError_t LaunchAggTaskSketch(const AggLaunch &p, int32_t nTasks, unsigned lon
 int32_t AggTasksVariants();
 void AggTasksVariantShape(int32_t variant, int32_t *threads, int32_t *blocksPerSM);
 cudaError_t LaunchAggTasks(const AggLaunch &p, int32_t variant, cudaStream_t stream);
+// The tasks flagged in p.taskShared, by units; next: a word of scratch.
+cudaError_t LaunchAggTaskUnits(const AggLaunch &p, const TaskUnit *units, int32_t nUnits, unsigned int *next,
+    cudaStream_t stream);
 cudaError_t LaunchAggTaskCount(const AggTable *tables, int32_t nTasks, const TaskChunk *chunks, int32_t nChunks,
     int32_t keyKind, uint32_t *counts, cudaStream_t stream);
 cudaError_t LaunchAggTaskPad(const uint32_t *groups, int32_t nTasks, uint32_t *padded, cudaStream_t stream);

@@ -186,6 +186,7 @@ struct AggLaunch {
     // task whose group does not fit sets taskFailed[i] (the host re-runs it exactly).
     const AggTable *taskTables;
     uint32_t *taskFailed;
+    const uint8_t *taskShared;  // tasks whose rows AggTaskUnitsKernel takes
     // VARCHAR inputs aggregated by SMIN/SMAX: the input's string dictionary (id k's characters
     // are strChars[strOff[k], strOff[k + 1])), for comparing two ids' strings.
     const int64_t *strOff[kMaxInputs];
@@ -202,6 +203,18 @@ struct TaskChunk {
     int32_t task;
     uint32_t chunk;
 };
+
+// A run of a task's tiles that one CTA aggregates in a shared table of `slots` slots: the rows whose partition of
+// 1 << partBits is `part`.
+struct TaskUnit {
+    int32_t task;
+    int32_t firstTile;
+    int32_t nTiles;
+    int32_t slots;
+    int32_t partBits;
+    int32_t part;
+};
+constexpr int kTaskMaxPartBits = 3;
 
 // ---- hash partitioning of aggregation input -------------------------------------------------
 // Rows go to partition (hash >> kPartShift) & (nParts - 1); the shared tables index slots with

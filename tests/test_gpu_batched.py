@@ -134,3 +134,55 @@ def test_batched_tables_around_a_chunk_of_slots(gpu, groups):
         tasks.append((key, rng.integers(-10**6, 10**6, n, dtype=np.int64), rng.random(n), km, None, None))
     (per,), _ = _run(tasks)
     _check(tasks, per)
+
+
+@pytest.mark.parametrize("groups", [255, 300, 1100, 2300, 9000, 11_000, 40_000])
+def test_batched_units_and_partitions(gpu, groups):
+    """Tasks whose rows go through shared tables, by units of 8 tiles and more, in one to eight partitions, and
+    just past those: rows around a unit's end, NULL and EMPTY keys, NULL values, double sums."""
+    rng = np.random.default_rng(groups)
+    tasks = []
+    for n in (32_768, 32_769, 140_001):
+        key = rng.integers(0, groups, n) * 7919
+        key[::1009] = np.iinfo(np.int64).min
+        tasks.append((key, rng.integers(-2**40, 2**40, n, dtype=np.int64), rng.random(n), rng.random(n) < 0.02,
+                      rng.random(n) < 0.05, rng.random(n) < 0.05))
+    (per, again), _ = _run(tasks, runs=2)
+    _check(tasks, per)
+    _check(tasks, again)
+
+
+@pytest.mark.parametrize("groups", [1, 7, 3000])
+def test_batched_units_of_two_column_keys(gpu, groups):
+    """Whole-number states of few groups and a packed key in the units' shared tables, exact in numpy."""
+    rng = np.random.default_rng(groups)
+    I = omg.IntType()
+    fac = omg.HashAggregationOperatorFactory([0, 1], [I, L], [[2], [2]], [[L], [L]], [[L], [L]],
+                                             [omg.OMNI_AGGREGATION_TYPE_SUM, omg.OMNI_AGGREGATION_TYPE_COUNT_COLUMN])
+    data = []
+    for n in (1, 4097, 70_001):
+        code = rng.integers(0, groups, n)
+        data.append((code.astype(np.int32) % 13, code * 2**33, rng.integers(-2**45, 2**45, n), rng.random(n) < 0.1))
+    handles = [omg.make_batch([I, L, L], [a, b, v], [None, None, m]) for a, b, v, m in data]
+    batch = omg.AggBatch(fac, handles)
+    batch.run()
+    got = {}
+    for t, b in batch.outputs():
+        got.setdefault(t, []).append(omg.batch_to_numpy(b))
+        omg.free_batch(b)
+    batch.close()
+    omg.free_batches(handles)
+    fac.close()
+    for t, (a, b, v, m) in enumerate(data):
+        cols = [np.concatenate([p[c][0] for p in got[t]]) for c in range(4)]
+        null = np.concatenate([p[2][1] for p in got[t]])
+        code, inv = np.unique(b // 2**33, return_inverse=True)
+        order = np.argsort(cols[1])
+        assert np.array_equal(cols[1][order], code * 2**33)
+        assert np.array_equal(cols[0][order], code % 13)
+        want = np.zeros(len(code), np.int64)
+        np.add.at(want, inv[~m], v[~m])
+        count = np.bincount(inv[~m], minlength=len(code))
+        assert np.array_equal(~null[order], count > 0)
+        assert np.array_equal(cols[2][order][count > 0], want[count > 0])
+        assert np.array_equal(cols[3][order], count)
