@@ -126,8 +126,10 @@ __global__ void __launch_bounds__(kKeyThreads, 2) RadixKeyKernel(const __grid_co
 // stores each, 1.75 ms as one of 32 bytes), so records of three or more words are padded to 32 bytes and
 // stored 32 bytes at a time; columns apart would take a request each.  Every pass over rows loads several
 // rows' values before it uses any, and what must outlive a pass is in shared memory: a register spill is a
-// store request too.
-constexpr int kScatterThreads = 512;
+// store request too.  Wide records are bound by latency before that: 32 warps of 64 registers with three
+// sources in flight instead of 16 of 128 with six took 2^26 records of a two-column key from 3.10 to 2.35 ms
+// (two sources 2.69; 2^24 of 16 bytes 0.44 -> 0.36; steps of eight tiles 2.42 and 0.41).
+constexpr int kScatterThreads = 1024;
 constexpr int kScatterTiles = 4;
 constexpr int kTileThreadRows = kTileRows / kScatterThreads;
 constexpr int kScatterRows = kScatterTiles * kTileRows;
@@ -157,7 +159,7 @@ __device__ __forceinline__ void StoreWords(const RecLayout &l, int w, uint32_t u
 }
 
 // The values that rows row0 + j * kScatterThreads (bit j of `use`) put into sources [s0, s0 + kSrcBatch).
-constexpr int kSrcBatch = 6;
+constexpr int kSrcBatch = 3;
 
 __device__ __forceinline__ void LoadSources(const RecLayout &l, int s0, const BatchDesc &b, int64_t row0, uint32_t use,
     uint64_t (&x)[kSrcBatch][kMoveRows])
