@@ -601,7 +601,11 @@ __global__ void __launch_bounds__(kPartThreads, 1) AggTaskUnitsKernel(const __gr
             }
             return g >= 0 ? tab.slots + g * sw + kw : nullptr;
         };
+        const volatile uint32_t *failed = p.taskFailed + unit.task;
         for (int t = unit.firstTile; t < unit.firstTile + unit.nTiles; ++t) {
+            if (*failed != 0u) {
+                break;  // the host re-runs the task exactly
+            }
             ProcessPartTile<kKind>(p, b, p.tiles[t], smem, unit.slots,
                 [&](uint64_t hash) { return PartOf(hash, unit.partBits) == unit.part; },
                 [&](int64_t row) {
@@ -613,7 +617,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) AggTaskUnitsKernel(const __gr
                 });
         }
         __syncthreads();
-        for (int i = threadIdx.x; i < unit.slots; i += kPartThreads) {
+        for (int i = threadIdx.x; i < unit.slots && *failed == 0u; i += kPartThreads) {
             const uint64_t *slot = smem + static_cast<int64_t>(i) * ss;
             if (SlotOccupied(p.key, slot[0])) {
                 uint64_t *st = place(RecordKey<kKind>(p, slot));
