@@ -28,7 +28,8 @@ constexpr int32_t kDefaultVariant = 1;  // 256 threads, 4 CTAs per SM
 // probes has outgrown its table and is re-run exactly.
 constexpr int32_t kTaskMaxProbe = 96;
 // Tasks of at most this load over all partitions of a shared table go by units; a table of a unit has slots for
-// twice the groups expected.  A unit has rows enough for its merge to stay small beside them.
+// twice the groups expected.  A unit has rows enough for its merge to stay small beside them, but few rows in
+// all are spread over the SMs first (36 tasks of 1,000 to 20,000 rows).
 constexpr double kUnitLoad = 0.6;
 constexpr int32_t kUnitMinTiles = 8;
 constexpr int32_t kUnitMaxTiles = 64;
@@ -109,6 +110,7 @@ struct BatchedAggregation::Impl {
     DevArray<uint8_t> shared;
     DevArray<unsigned int> nextUnit;
     int32_t nUnits = 0;
+    bool anyGlobal = true;  // tasks whose rows go to their own tables at once
     DevArray<unsigned long long> cursor;
     DevArray<int64_t> blockSums;
     DevArray<long long> total;
@@ -170,7 +172,9 @@ struct BatchedAggregation::Impl {
         CudaCheck(cudaMemsetAsync(specials.Get(), 0, sizeof(uint32_t) * 2 * n, s), "reset special slots");
         CudaCheck(cudaMemsetAsync(failed.Get(), 0, sizeof(uint32_t) * n, s), "reset task flags");
         CudaCheck(omg::LaunchAggInitTable(p, s), "init task tables");
-        CudaCheck(omg::LaunchAggTasks(p, variant, s), "batched aggregation");
+        if (anyGlobal) {
+            CudaCheck(omg::LaunchAggTasks(p, variant, s), "batched aggregation");
+        }
         CudaCheck(omg::LaunchAggTaskUnits(p, units.Get(), nUnits, nextUnit.Get(), s), "batched aggregation by units");
         CudaCheck(omg::LaunchAggTaskCount(tables.Get(), n, chunks.Get(), nChunks, plan.key.kind, groups.Get(), s), "count task groups");
         CudaCheck(omg::LaunchAggTaskPad(groups.Get(), n, counts.Get(), s), "pad task regions");
@@ -309,6 +313,8 @@ struct BatchedAggregation::Impl {
         // Double sums of few groups are faster in the global table, whose atomics are not compare-and-swap loops.
         const uint64_t minGroups = std::any_of(plan.accs.begin(), plan.accs.end(),
             [](const omg::AccSpec &a) { return a.kind == omg::ACC_DSUM; }) ? 256 : 0;
+        const int32_t minTiles = std::min(kUnitMinTiles, bt.NumTiles() / (2 * omg::DeviceSMCount()) + 1);
+        anyGlobal = false;
         int32_t tile = 0;
         for (int32_t t = 0; t < n; ++t) {
             const int32_t tiles = static_cast<int32_t>((tasks[t]->GetRowCount() + omg::kTileRows - 1) / omg::kTileRows);
@@ -322,7 +328,7 @@ struct BatchedAggregation::Impl {
                 const int64_t slots = std::max<int64_t>(64, 2 * (static_cast<int64_t>(estimate[t]) >> bits));
                 const int64_t want = 8 * static_cast<int64_t>(estimate[t]) / omg::kTileRows + 1;
                 const int32_t step = static_cast<int32_t>(
-                    std::min<int64_t>(kUnitMaxTiles, std::max<int64_t>(kUnitMinTiles, want)));
+                    std::min<int64_t>(kUnitMaxTiles, std::max<int64_t>(minTiles, want)));
                 for (int32_t first = 0; first < tiles; first += step) {
                     for (int32_t part = 0; part < (1 << bits); ++part) {
                         hostUnits.push_back(omg::TaskUnit{t, tile + first, std::min(step, tiles - first),
@@ -330,6 +336,7 @@ struct BatchedAggregation::Impl {
                     }
                 }
             }
+            anyGlobal = anyGlobal || hostShared[t] == 0;
             tile += tiles;
         }
         nUnits = static_cast<int32_t>(hostUnits.size());

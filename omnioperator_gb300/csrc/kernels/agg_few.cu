@@ -467,7 +467,6 @@ bool LayoutAggFew(const AggLaunch &p, uint32_t nullable, FewLayout *l)
     }
     const int nAll = l->maxGroups + l->firstSlot;
     l->smemBytes = (at + nAll * slotBytes + 15) / 16 * 16;
-    l->indexSize = kFewIndex;
     return true;
 }
 

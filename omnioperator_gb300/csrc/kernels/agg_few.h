@@ -16,7 +16,6 @@ constexpr int kFewThreads = 256;
 struct FewLayout {
     int32_t maxGroups;   // with private states
     int32_t firstSlot;   // the first slot with private states: 0 when the key may be NULL, else 2
-    int32_t indexSize;
     int32_t smemBytes;
     int32_t off[kMaxAccs];
     int32_t planeStep[kMaxAccs];
