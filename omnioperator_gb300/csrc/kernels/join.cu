@@ -3037,7 +3037,8 @@ cudaError_t LaunchGatherColumn(const BatchDesc *batches, const TileDesc *tiles, 
 cudaError_t LaunchKeyStats(const void *keys, const uint8_t *nulls, int64_t n, int32_t width, long long *stats,
     cudaStream_t stream)
 {
-    const long long init[3] = {0x7fffffffffffffffll, static_cast<long long>(0x8000000000000000ull), 0};
+    // Static: the copy may still be reading it after this function has returned.
+    static const long long init[3] = {0x7fffffffffffffffll, static_cast<long long>(0x8000000000000000ull), 0};
     cudaError_t err = cudaMemcpyAsync(stats, init, sizeof(init), cudaMemcpyHostToDevice, stream);
     if (err != cudaSuccess || n == 0) {
         return err;
