@@ -1202,10 +1202,14 @@ struct HashAggregationOperator::RadixRun {
     int32_t bits = 0;
     int32_t passBits = 0;
     int32_t indexSize = 0;
-    std::vector<omg::RadixUnit> units;
+    int32_t nUnits = 0;
     uint64_t denseCap = 0;
     uint64_t tableGroups = 0;  // groups expected in the table: those of multi units
     uint64_t spillCap = 0;     // slots that the multi units could merge
+    // Pinned, and alive until the flush has waited for the kernels: an upload from other memory may still be
+    // reading its source after the call returned.
+    omg::PinnedArray<unsigned int> start;
+    omg::PinnedArray<omg::RadixUnit> units;
     DevArray<unsigned int> cursor;
     DevArray<omg::RadixUnit> dUnits;
     DevArray<uint64_t> records;
@@ -1326,7 +1330,8 @@ bool HashAggregationOperator::PlanRadix(omg::BatchTable &bt, RadixRun &run, cuda
         const uint32_t nParts = 1u << run.bits;
         const uint32_t fine = omg::kRadixFineParts >> run.bits;
         const uint64_t unitSlots = static_cast<uint64_t>(nSlots) << run.passBits;
-        std::vector<unsigned int> start(nParts);
+        run.start.Reset(nParts);
+        std::vector<omg::RadixUnit> units;
         std::vector<omg::RadixUnit> whole;
         const uint64_t perCta = (rows / (2 * omg::DeviceSMCount()) + omg::kRadixStepRows) / omg::kRadixStepRows;
         const uint64_t unitRows = std::min<uint64_t>(kRadixUnitRows, perCta * omg::kRadixStepRows);
@@ -1337,12 +1342,12 @@ bool HashAggregationOperator::PlanRadix(omg::BatchTable &bt, RadixRun &run, cuda
             for (uint32_t f = q * fine; f < (q + 1) * fine; ++f) {
                 n += h[f];
             }
-            start[q] = static_cast<unsigned int>(first);
+            run.start[q] = static_cast<unsigned int>(first);
             if (n > 2 * unitRows) {
                 ++multi;
                 for (uint64_t r = 0; r < n; r += unitRows) {
                     const uint64_t m = std::min(unitRows, n - r);
-                    run.units.push_back(omg::RadixUnit{static_cast<uint32_t>(first + r), static_cast<uint32_t>(m), 1, 0});
+                    units.push_back(omg::RadixUnit{static_cast<uint32_t>(first + r), static_cast<uint32_t>(m), 1, 0});
                     run.spillCap += std::min(m, unitSlots);
                 }
             } else if (n > 0) {
@@ -1351,14 +1356,17 @@ bool HashAggregationOperator::PlanRadix(omg::BatchTable &bt, RadixRun &run, cuda
             }
             first += n;
         }
-        run.units.insert(run.units.end(), whole.begin(), whole.end());
+        units.insert(units.end(), whole.begin(), whole.end());
+        run.nUnits = static_cast<int32_t>(units.size());
         run.tableGroups = static_cast<uint64_t>(1.1 * groups / nParts * static_cast<double>(multi)) + 64;
+        run.units.Reset(units.size());
+        std::copy(units.begin(), units.end(), run.units.Get());
         run.cursor.Reset(nParts, s);
-        CudaCheck(cudaMemcpyAsync(run.cursor.Get(), start.data(), sizeof(unsigned int) * nParts, cudaMemcpyHostToDevice,
-                      s),
+        run.dUnits.Reset(units.size(), s);
+        CudaCheck(cudaMemcpyAsync(run.cursor.Get(), run.start.Get(), sizeof(unsigned int) * nParts,
+                      cudaMemcpyHostToDevice, s),
             "upload partition starts");
-        run.dUnits.Reset(run.units.size(), s);
-        CudaCheck(cudaMemcpyAsync(run.dUnits.Get(), run.units.data(), sizeof(omg::RadixUnit) * run.units.size(),
+        CudaCheck(cudaMemcpyAsync(run.dUnits.Get(), run.units.Get(), sizeof(omg::RadixUnit) * units.size(),
                       cudaMemcpyHostToDevice, s),
             "upload radix units");
         run.records.Reset(rows * run.layout.words + 2, s);
@@ -1642,7 +1650,7 @@ void HashAggregationOperator::Flush(bool last)
         omg::RadixAgg ra;
         ra.records = radixRun.records.Get();
         ra.units = radixRun.dUnits.Get();
-        ra.nUnits = static_cast<int32_t>(radixRun.units.size());
+        ra.nUnits = radixRun.nUnits;
         ra.passBits = radixRun.passBits;
         ra.next = reinterpret_cast<unsigned int *>(im.stats.Get() + 5);
         ra.dense = radixRun.dense.Get();

@@ -8,6 +8,14 @@ import pytest
 
 CSRC = Path(__file__).resolve().parents[1] / "omnioperator_gb300" / "csrc"
 
+# Sources that live on in the caller or the factory: who waits for the copy.
+KEPT = {
+    ("sizer.cpp", "X"): "Predict and Train read results back before they return",
+    ("sizer.cpp", "T"): "Train reads the loss back before it returns",
+    ("hash_join.cpp", "f_.filterText.data()"): "a member of the factory, which outlives its operators",
+}
+
+
 def _functions(text):
     """(start, end) of top-level function bodies: from a line that is `{` to the next that is `}`."""
     opens = [m.start() for m in re.finditer(r"^\{$", text, re.M)]
@@ -15,7 +23,7 @@ def _functions(text):
 
 
 def _uploads():
-    for path in sorted((CSRC / "kernels").rglob("*.c*")):
+    for path in sorted(CSRC.rglob("*.c*")):
         text = path.read_text()
         for m in re.finditer(r"cudaMemcpyAsync\(([^;]*?),\s*cudaMemcpyHostToDevice", text, re.S):
             args = re.split(r",\s*(?![^()]*\))", m.group(1))
@@ -38,9 +46,9 @@ def test_source_outlives_the_copy(site):
     body, rest = text[start:end], text[m.end():end]
     static = re.search(r"static const[^;]*\b%s\b" % re.escape(source), body)
     waits = re.search(r"\bSync\(\)|cudaStreamSynchronize", rest)
-    assert static or waits or _pinned(body, source), f"{name}: {source}"
+    assert static or waits or _pinned(body, source) or (name, source) in KEPT, f"{name}: {source}"
 
 
 def test_every_upload_is_looked_at():
-    total = sum(p.read_text().count("cudaMemcpyHostToDevice") for p in (CSRC / "kernels").rglob("*.c*"))
-    assert total == len(list(_uploads())) > 0
+    total = sum(p.read_text().count("cudaMemcpyHostToDevice") for p in CSRC.rglob("*.c*"))
+    assert total == len(list(_uploads())) > 10
