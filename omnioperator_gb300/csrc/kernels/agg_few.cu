@@ -3,10 +3,10 @@
 // With few groups the shared tables' atomics are all on the same words: 2^22 rows of 6 groups, two INT keys
 // and six aggregates ran 1.22 ms, and 0.15 ms here (instruction issue: 480 a row, a third of them the
 // packed key).  Here every thread keeps states of its own for every group, in planes of shared
-// memory where the threads of a warp are side by side: no atomics and no bank conflicts.  Sums of
-// doubles and exact sums move to the CTA's state of the group every 64 rows (plain sums of at most 64
-// doubles, as a table slot's first 64; magnitudes of up to 64 values below 2^57), and at the end a warp
-// adds up each group's private states and the CTA's records are merged into the global table.
+// memory where the threads of a warp are side by side: no atomics and no bank conflicts.  A sum of doubles has a
+// plane for the rounding errors of its additions.  Exact sums move to the CTA's state of the group every 64
+// rows (magnitudes of up to 64 values below 2^57), and at the end a warp adds up each group's private states
+// and the CTA's records are merged into the global table.
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -113,28 +113,17 @@ __device__ __forceinline__ void ApplyFew(const AggLaunch &p, const FewLayout &l,
             break;
         }
         case ACC_DSUM: {
-            double *d = reinterpret_cast<double *>(plane);
+            double *sum = reinterpret_cast<double *>(plane);
+            double *err = reinterpret_cast<double *>(plane + l.planeStep[a]);
 #pragma unroll
             for (int k = 0; k < kFewRows; ++k) {
                 if ((has >> k) & 1u) {
-                    d[at[k]] = __dadd_rn(d[at[k]], AsDouble(in.bits[k], s.inKind, s.inWidth));
-                }
-            }
-            if (fold != 0) {
-                // A later row of the same group may already be in: at most 67 plain additions.
-#pragma unroll 1
-                for (int k = 0; k < kFewRows; ++k) {
-                    if ((fold >> k) & 1u) {
-                        int e = at[0];
-                        uint64_t *to = states[0];
-#pragma unroll
-                        for (int j = 1; j < kFewRows; ++j) {
-                            e = j == k ? at[j] : e;
-                            to = j == k ? states[j] : to;
-                        }
-                        SharedAddCompensated(to + s.word, d[e]);
-                        d[e] = 0.0;
-                    }
+                    // Once a sum is not finite it stays so, and its errors (NaN then) are not looked at.
+                    const double x = AsDouble(in.bits[k], s.inKind, s.inWidth);
+                    const double old = sum[at[k]];
+                    const double next = __dadd_rn(old, x);
+                    sum[at[k]] = next;
+                    err[at[k]] = __dadd_rn(err[at[k]], SumError(old, x, next));
                 }
             }
             break;
@@ -195,9 +184,11 @@ __device__ __forceinline__ void FoldGroup(const AggLaunch &p, const FewLayout &l
         const unsigned int *n32 = reinterpret_cast<const unsigned int *>(smem + off) + group * kFewThreads;
         const uint64_t *n64 = reinterpret_cast<const uint64_t *>(smem + off) + group * kFewThreads;
         if (s.kind == ACC_DSUM) {
+            const uint64_t *e64 = n64 + l.planeStep[a] / 8;
             double sum = 0.0, err = 0.0;
             for (int t = lane; t < kFewThreads; t += 32) {
                 AddTwoSum(sum, err, __longlong_as_double(static_cast<long long>(n64[t])));
+                err = __dadd_rn(err, __longlong_as_double(static_cast<long long>(e64[t])));
             }
             for (int o = 16; o > 0; o >>= 1) {
                 const double os = __shfl_xor_sync(0xffffffffu, sum, o);
@@ -288,7 +279,7 @@ __global__ void __launch_bounds__(kFewThreads, 2) AggFewKernel(const __grid_cons
             } else {
                 *Plane<uint64_t>(smem8, l.off[a], g) = s.kind == ACC_DSUM || s.kind == ACC_ISUM || s.kind == ACC_WSUM2
                     ? 0ull : static_cast<uint64_t>(s.init);
-                if (s.kind == ACC_WSUM2) {
+                if (s.kind == ACC_WSUM2 || s.kind == ACC_DSUM) {
                     *Plane<uint64_t>(smem8, l.off[a] + l.planeStep[a], g) = 0;
                 }
             }
@@ -408,11 +399,11 @@ bool LayoutAggFew(const AggLaunch &p, uint32_t nullable, FewLayout *l)
             case ACC_ISUM:
             case ACC_IMIN:
             case ACC_IMAX:
-            case ACC_DSUM:
             case ACC_DMIN:
             case ACC_DMAX:
                 bytes[a] = 8;
                 break;
+            case ACC_DSUM:
             case ACC_WSUM2:
                 bytes[a] = 16;
                 break;

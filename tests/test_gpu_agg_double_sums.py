@@ -1,0 +1,52 @@
+"""SUM of doubles where the order and the splitting of the additions must not show: every path carries the
+rounding errors of its additions along, so a sum is off by its own rounding and second-order terms only.
+
+With u = 2^-53 and n rows, the carried errors are at most n u sum|x| and adding those up loses at most
+n^2 u^2 sum|x|; turning sum and errors into the result rounds once more: u |sum|."""
+import math
+
+import numpy as np
+import pytest
+
+import omnioperator_gb300 as omg
+from helpers import run_agg
+
+pytestmark = pytest.mark.gpu
+
+L, I, D = omg.LongType(), omg.IntType(), omg.DoubleType()
+SUM, CALL = omg.OMNI_AGGREGATION_TYPE_SUM, omg.OMNI_AGGREGATION_TYPE_COUNT_ALL
+U = 2.0**-53
+
+
+def _values(kind, n, rng):
+    if kind == "constant":
+        return np.full(n, 0.1)
+    if kind == "thirds":
+        return rng.choice([0.1, 0.3, 1 / 3], n)
+    big = np.tile([1e16, 1.0, -1e16, 3.0], n // 4 + 1)[:n]  # cancels, but for the small ones
+    return big
+
+
+def _check(group, x, got):
+    """got: {group: sum}, for the groups to look at."""
+    for g, s in got.items():
+        v = x[group == g]
+        exact, n = math.fsum(v), len(v)
+        assert abs(s - exact) <= U * abs(exact) + n * n * U * U * np.abs(v).sum(), (g, n, s, exact)
+
+
+def _run(key, x, **kw):
+    cols, ctr = run_agg([0], [L], [[1], []], [[D], []], [[D], [L]], [SUM, CALL], [key, x], [L, D], **kw)
+    return dict(zip(cols[0][0].tolist(), cols[1][0].tolist())), ctr
+
+
+@pytest.mark.parametrize("kind", ["constant", "thirds", "cancel"])
+@pytest.mark.parametrize("n,groups", [(1 << 18, 1), (1 << 18, 5), (1_000_003, 3)])
+def test_few_groups(gpu, kind, n, groups):
+    """Thread-private states."""
+    rng = np.random.default_rng(groups)
+    key = rng.integers(0, groups, n)
+    x = _values(kind, n, rng)
+    got, ctr = _run(key, x, batch_sizes=(n,))
+    assert ctr["sizing"]["part_bits"] == 0
+    _check(key, x, got)
