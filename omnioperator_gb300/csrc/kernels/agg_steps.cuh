@@ -196,26 +196,106 @@ __device__ __forceinline__ void ApplyInt(const AccSpec &s, const Run &run, const
     }
 }
 
-// Add x to the compensated sum at w.  A sum of at most 8 + 5 plain additions (a thread's rows, a warp's
-// threads) comes in; every one after that is compensated.  FP64 operations bound it (an SM does two a cycle,
-// and a warp goes through the shared and the unshared ones for each of its threads' rows), so both kinds of
-// store take one way as far as they can: 16M rows in 100,000 groups, six aggregates, 1248 -> 1100 us in all.
-__device__ __forceinline__ void AddDouble(uint64_t *w, double x, bool shared)
+// A sum of doubles and the rounding errors of its additions (NaN once the sum is not finite: AddDouble leaves
+// them out then).
+struct Sum {
+    double sum;
+    double err;
+};
+
+__device__ __forceinline__ bool IsZero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+__device__ __forceinline__ bool IsFinite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
+
+__device__ __forceinline__ void AddTo(Sum &a, double x)
+{
+    const double next = __dadd_rn(a.sum, x);
+    a.err = __dadd_rn(a.err, SumError(a.sum, x, next));
+    a.sum = next;
+}
+
+// Add v to the compensated sum at w.  FP64 operations bound it (an SM does two a cycle, comparisons among them, and a
+// warp goes through the shared and the unshared ones for each of its threads' rows), so both kinds of store take
+// one way as far as they can, zeros are told by their bits, and nothing is compensated for on a slot's first value.
+__device__ __forceinline__ void AddDouble(uint64_t *w, const Sum &v, bool shared)
 {
     double *d = reinterpret_cast<double *>(w);
-    const double old = shared ? atomicAdd(d, x) : d[0];
-    const double sum = __dadd_rn(old, x);
+    const double old = shared ? atomicAdd(d, v.sum) : d[0];
+    double sum = v.sum;
+    double err = v.err;
+    if (!IsZero(old) || IsZero(v.sum)) {  // 0.0 + -0.0 is 0.0
+        sum = __dadd_rn(old, v.sum);
+        err = __dadd_rn(err, SumError(old, v.sum, sum));
+    }
     if (!shared) {
         d[0] = sum;
     }
-    if (isfinite(sum)) {
-        const double err = SumError(old, x, sum);
-        if (err != 0.0) {
-            if (shared) {
-                atomicAdd(d + 1, err);
+    if (!IsZero(err) && IsFinite(sum)) {
+        if (shared) {
+            atomicAdd(d + 1, err);
+        } else {
+            d[1] = __dadd_rn(d[1], err);
+        }
+    }
+}
+
+// The sum over the warp's threads, in thread 0.  Each value is cut at a bit that is the same for all of them, so far
+// below 2^8 times their largest power of two that the upper parts, 46 bits each, add up without rounding, and the
+// lower parts' roundings are of second order: 14 FP64 operations where five times AddTo and an error takes 25.
+__device__ __forceinline__ void SumWarp(Sum &v)
+{
+    const unsigned int most =
+        __reduce_max_sync(0xffffffffu, static_cast<unsigned int>(__double2hiint(v.sum)) & 0x7ff00000u);
+    if (most < (0x7ffu - 9u) << 20) {
+        const double cut = __hiloint2double(static_cast<int>(most + (8u << 20)), 0);
+        const double top = __dsub_rn(__dadd_rn(cut, v.sum), cut);
+        v.err = __dadd_rn(v.err, __dsub_rn(v.sum, top));
+        v.sum = top;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            v.sum = __dadd_rn(v.sum, __shfl_down_sync(0xffffffffu, v.sum, o));
+            v.err = __dadd_rn(v.err, __shfl_down_sync(0xffffffffu, v.err, o));
+        }
+        return;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {  // near the largest double, infinite, or not a number
+        const double sum = __shfl_down_sync(0xffffffffu, v.sum, o);
+        const double err = __shfl_down_sync(0xffffffffu, v.err, o);
+        AddTo(v, sum);
+        v.err = __dadd_rn(v.err, err);
+    }
+}
+
+// ForGroups for sums of doubles into the states at base.  A run's first value needs no addition.
+__device__ __forceinline__ void SumGroups(const Run &run, const double (&x)[kStepThreadRows], uint32_t use,
+    uint64_t *base, int sw)
+{
+    Sum v{-0.0, 0.0};  // -0.0 + x is x for every x
+    bool any = false;
+    bool shared = run.left;
+#pragma unroll
+    for (int j = 0; j < kStepThreadRows; ++j) {
+        if ((use >> j) & 1u) {
+            if (any) {
+                AddTo(v, x[j]);
             } else {
-                d[1] = __dadd_rn(d[1], err);
+                v.sum = x[j];
             }
+            any = true;
+        }
+        if (!run.uniform && ((run.ends >> j) & 1u) != 0) {
+            if (any) {
+                AddDouble(base + run.Slot(j) * sw, v, shared || (run.right && (run.live >> j) == 1u));
+            }
+            v = Sum{-0.0, 0.0};
+            any = false;
+            shared = false;
+        }
+    }
+    if (run.uniform) {
+        SumWarp(v);
+        if (__any_sync(0xffffffffu, use != 0) && (threadIdx.x & 31) == 0) {
+            AddDouble(base + run.Slot(0) * sw, v, true);
         }
     }
 }
@@ -327,9 +407,7 @@ __device__ __forceinline__ void ApplyRun(const AggLaunch &p, const Rows &rows, c
                 for (int j = 0; j < kStepThreadRows; ++j) {
                     x[j] = AsDouble(bits[j], s.inKind, s.inWidth);
                 }
-                // -0.0 + x is x for every x, so a single value passes through unchanged.
-                ForGroups(run, x, use, -0.0, [](double u, double v) { return __dadd_rn(u, v); },
-                    [&](int slot, double v, bool shared) { AddDouble(base + slot * sw, v, shared); });
+                SumGroups(run, x, use, base, sw);
                 break;
             }
             case ACC_DMIN:

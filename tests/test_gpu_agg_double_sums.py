@@ -50,3 +50,29 @@ def test_few_groups(gpu, kind, n, groups):
     got, ctr = _run(key, x, batch_sizes=(n,))
     assert ctr["sizing"]["part_bits"] == 0
     _check(key, x, got)
+
+
+@pytest.mark.parametrize("kind", ["constant", "thirds", "cancel"])
+@pytest.mark.parametrize("n,groups", [(2048, 1), (16_384, 1), (16_384, 3), (16_001, 40)])
+def test_small_calls(gpu, kind, n, groups):
+    """One launch for the whole call: rows sorted by group, runs of a thread's and a warp's rows."""
+    rng = np.random.default_rng(n + groups)
+    key = rng.integers(0, groups, n)
+    x = _values(kind, n, rng)
+    got, ctr = _run(key, x, batch_sizes=(n,))
+    assert ctr["launches"] == 1
+    _check(key, x, got)
+
+
+@pytest.mark.parametrize("kind", ["constant", "thirds", "cancel"])
+def test_radix_passes(gpu, kind):
+    """A hot group, whose partition is cut into units; groups of some hundred and of a few rows."""
+    n = 1 << 20
+    rng = np.random.default_rng(2)
+    key = 1000 + rng.integers(0, 400_000, n)
+    u = rng.random(n)
+    key[u < 0.5] = rng.integers(100, 600, int((u < 0.5).sum()))
+    key[u < 0.2] = 7
+    x = _values(kind, n, rng)
+    got, ctr = _run(key, x, batch_sizes=(n,))
+    _check(key, x, {g: s for g, s in got.items() if g < 600 or g % 4001 == 0})
