@@ -58,7 +58,8 @@ __device__ __forceinline__ void AddSharedDouble(uint64_t *w, double x, uint32_t 
 }
 
 // The rows of a tile whose key hash wants(hash) takes; elsewhere(row) takes a row without a place in the table.
-template <int kKind, class Wants, class Elsewhere>
+// kPlain: the first kPlainSumRows doubles of a slot are added plainly.
+template <int kKind, bool kPlain, class Wants, class Elsewhere>
 __device__ __forceinline__ void ProcessPartTile(const AggLaunch &p, const BatchDesc &b, const TileDesc &tile,
     uint64_t *sm, int smSlots, Wants wants, Elsewhere elsewhere)
 {
@@ -111,8 +112,8 @@ __device__ __forceinline__ void ProcessPartTile(const AggLaunch &p, const BatchD
                 if ((live >> k) & 1u) {
                     // A shared table counts the rows of one launch (< 2^32): a 32-bit add on the
                     // word's low half (little-endian) is exact and faster than a 64-bit one.
-                    arrival[k] = min(atomicAdd(LowHalf(st + slot[k] * sw + s.word), 1u),
-                        static_cast<unsigned int>(kPlainSumRows));
+                    const unsigned int n = atomicAdd(LowHalf(st + slot[k] * sw + s.word), 1u);
+                    arrival[k] = kPlain ? min(n, static_cast<unsigned int>(kPlainSumRows)) : arrival[k];
                 }
             }
             continue;
@@ -268,7 +269,7 @@ __device__ __forceinline__ void AggBody(const AggLaunch &p, const SpillArgs &sp,
             for (int t = tFirst; t < tEnd; t += tStep) {
                 const TileDesc tile = p.tiles[t];
                 const BatchDesc &b = p.batches[tile.batch];
-                ProcessPartTile<kKind>(p, b, tile, smem, smSlots, [](uint64_t) { return true; }, [&](int64_t row) {
+                ProcessPartTile<kKind, true>(p, b, tile, smem, smSlots, [](uint64_t) { return true; }, [&](int64_t row) {
                     ProcessRow<kKind>(p, tile.batch, b, row, LoadRow<kKind>(p, b, row), smem, 0, &newGroups);
                 });
             }
@@ -568,7 +569,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) AggTasksKernel(const __g
 // (5.3 ms for 58M rows in 400 tasks, at the 38 G/s that such requests go at), so here a CTA adds up a run of a
 // task's rows in a shared table and merges that: 1.0 ms, and 1.9 above for the tasks left.  More groups than a
 // table holds take up to eight runs over the keys, each for the rows of one partition; 16 runs took this
-// kernel from 0.91 to 1.36 ms and the other from 2.15 to 1.58, 32 runs 2.14 and 1.29.
+// kernel from 0.91 to 1.36 ms and the other from 2.15 to 1.58, 32 runs 2.14 and 1.29.  Doubles are compensated from
+// the first one on: a group may have a slot in every unit of its task, and 64 plain rows in each.
 template <int kKind>
 __global__ void __launch_bounds__(kPartThreads, 1) AggTaskUnitsKernel(const __grid_constant__ AggLaunch p,
     const TaskUnit *units, int32_t nUnits, unsigned int *next)
@@ -606,7 +608,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) AggTaskUnitsKernel(const __gr
             if (*failed != 0u) {
                 break;  // the host re-runs the task exactly
             }
-            ProcessPartTile<kKind>(p, b, p.tiles[t], smem, unit.slots,
+            ProcessPartTile<kKind, false>(p, b, p.tiles[t], smem, unit.slots,
                 [&](uint64_t hash) { return PartOf(hash, unit.partBits) == unit.part; },
                 [&](int64_t row) {
                     const RowIn in = LoadRow<kKind>(p, b, row);

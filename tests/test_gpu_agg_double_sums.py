@@ -76,3 +76,26 @@ def test_radix_passes(gpu, kind):
     x = _values(kind, n, rng)
     got, ctr = _run(key, x, batch_sizes=(n,))
     _check(key, x, {g: s for g, s in got.items() if g < 600 or g % 4001 == 0})
+
+
+@pytest.mark.parametrize("kind", ["constant", "thirds", "cancel"])
+def test_batched_tasks_by_units(gpu, kind):
+    """A task whose rows many CTAs add up in shared tables of their own."""
+    n, groups = 400_000, 300
+    rng = np.random.default_rng(3)
+    key = rng.integers(0, groups, n)
+    x = _values(kind, n, rng)
+    fac = omg.HashAggregationOperatorFactory([0], [L], [[1], []], [[D], []], [[D], [L]], [SUM, CALL])
+    task = omg.make_batch([L, D], [key, x])
+    batch = omg.AggBatch(fac, [task])
+    batch.run()
+    got = {}
+    for _, b in batch.outputs():
+        cols = omg.batch_to_numpy(b)
+        omg.free_batch(b)
+        got.update(zip(cols[0][0].tolist(), cols[1][0].tolist()))
+    assert batch.info()["reruns"] == 0 and len(got) == groups
+    batch.close()
+    omg.free_batch(task)
+    fac.close()
+    _check(key, x, got)
