@@ -127,6 +127,11 @@ int32_t omg_debug_set_bulk_probe(int32_t mode);
  * and stores, 5 group-staged (pinned host output), 6 bulk-copy; 0 none yet.  For tests and
  * measurements.  No reference counterpart. */
 int32_t omg_debug_last_probe_kernel(void);
+/* How the latest HashAggregation rows of this process were aggregated: out[0] = 1 one global table (with or without
+ * shared tables in front), 2 hash partitions, 3 states per thread (few groups), 4 radix passes, 5 one launch for
+ * the whole call, 0 none yet; for 4 also out[1] = passes over a partition, out[2] = units that hot partitions were
+ * cut into, out[3] = whole partitions.  For tests and measurements.  No reference counterpart. */
+int32_t omg_debug_last_agg_kernel(int64_t *out, int32_t n);
 /* Train sizing and CDF models of two hidden layers (input <= 16, hidden widths multiples of 4 up
  * to 64) with the fused kernel, all epochs in one cooperative launch (1, default), or layer by
  * layer with one launch per layer and step (0).  For tests and measurements.  No reference

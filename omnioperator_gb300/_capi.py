@@ -33,6 +33,7 @@ _SIGS = {
     "omg_debug_set_staged_probe": (I32, [I32]),
     "omg_debug_set_bulk_probe": (I32, [I32]),
     "omg_debug_last_probe_kernel": (I32, []),
+    "omg_debug_last_agg_kernel": (I32, [C.POINTER(I64), I32]),
     "omg_debug_set_fused_training": (I32, [I32]),
     "omg_op_set_agg_sizing": (I32, [P, I32]),
     "omg_debug_set_agg_flush_rows": (I32, [I64]),

@@ -167,6 +167,14 @@ int32_t omg_debug_set_staged_probe(int32_t on)
 
 int32_t omg_debug_last_probe_kernel(void) { return omg::LastProbeKernel(); }
 
+int32_t omg_debug_last_agg_kernel(int64_t *out, int32_t n)
+{
+    return Guard([&] {
+        Require(out != nullptr && n >= 0, "null output array");
+        omniruntime::op::LastAggKernel(out, n);
+    });
+}
+
 int32_t omg_debug_set_fused_training(int32_t on)
 {
     omg::SetFusedTraining(on != 0);

@@ -10,6 +10,7 @@
 #include "omniop/hash_aggregation.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cfloat>
 #include <climits>
@@ -107,11 +108,31 @@ uint64_t NextPow2(uint64_t v)
     return p;
 }
 
+// AggKernel of the latest rows, and for the radix passes: passes over a partition, units of hot partitions, whole
+// partitions.
+enum AggKernel : int64_t { AGG_TABLE = 1, AGG_PARTITIONS = 2, AGG_FEW = 3, AGG_RADIX = 4, AGG_SMALL = 5 };
+std::atomic<int64_t> g_lastAgg[4];
+
+void SetLastAgg(int64_t kernel, int64_t passes = 0, int64_t cut = 0, int64_t whole = 0)
+{
+    g_lastAgg[0] = kernel;
+    g_lastAgg[1] = passes;
+    g_lastAgg[2] = cut;
+    g_lastAgg[3] = whole;
+}
+
 constexpr uint64_t kDefaultCapacity = uint64_t(1) << 16;
 constexpr int kGlobalMaxProbe = 96;
 constexpr size_t kSmemBudget = 96 * 1024;            // shared bytes per CTA for pre-aggregation
 
 }  // namespace
+
+void LastAggKernel(int64_t *out, int32_t n)
+{
+    for (int32_t i = 0; i < n; ++i) {
+        out[i] = i < 4 ? g_lastAgg[i].load() : 0;
+    }
+}
 
 // ------------------------------------------------------------------------------ factory
 HashAggregationOperatorFactory::HashAggregationOperatorFactory(std::vector<uint32_t> &groupByCol,
@@ -1203,6 +1224,7 @@ struct HashAggregationOperator::RadixRun {
     int32_t passBits = 0;
     int32_t indexSize = 0;
     int32_t nUnits = 0;
+    int32_t nMulti = 0;  // the first of them: runs of the partitions that are cut
     uint64_t denseCap = 0;
     uint64_t tableGroups = 0;  // groups expected in the table: those of multi units
     uint64_t spillCap = 0;     // slots that the multi units could merge
@@ -1356,6 +1378,7 @@ bool HashAggregationOperator::PlanRadix(omg::BatchTable &bt, RadixRun &run, cuda
             }
             first += n;
         }
+        run.nMulti = static_cast<int32_t>(units.size());
         units.insert(units.end(), whole.begin(), whole.end());
         run.nUnits = static_cast<int32_t>(units.size());
         run.tableGroups = static_cast<uint64_t>(1.1 * groups / nParts * static_cast<double>(multi)) + 64;
@@ -1660,12 +1683,15 @@ void HashAggregationOperator::Flush(bool last)
         CudaCheck(omg::LaunchRadixAgg(p, radixRun.layout, ra, spillA.Get(), nSpill, static_cast<uint32_t>(spillCap), s),
             "radix aggregation");
         ++counters_[0];
+        SetLastAgg(AGG_RADIX, int64_t(1) << radixRun.passBits, radixRun.nMulti, radixRun.nUnits - radixRun.nMulti);
     } else if (few) {
         CudaCheck(omg::LaunchAggFew(p, fewLayout, spillA.Get(), nSpill, static_cast<uint32_t>(spillCap), s),
             "aggregation of few groups");
+        SetLastAgg(AGG_FEW);
     } else {
         CudaCheck(omg::LaunchAgg(p, spillA.Get(), nSpill, static_cast<uint32_t>(spillCap), nullptr, 0, grid, s),
             "aggregation kernel");
+        SetLastAgg(im.partBits >= 0 ? AGG_PARTITIONS : AGG_TABLE);
     }
     im.timer.Stop(s);
     ++counters_[0];
@@ -2241,6 +2267,7 @@ bool HashAggregationOperator::ExtractSmall()
     if (static_cast<int32_t>(r[1]) != 0) {
         throw OmniException("OPERATOR_RUNTIME_ERROR", "sum_aggregator overflow.", -5);
     }
+    SetLastAgg(AGG_SMALL);
     ReleasePending();
     EmitOutputs(x, static_cast<int64_t>(r[0]), s);
     return true;

@@ -35,6 +35,9 @@ namespace op {
 
 // The compiled form of a factory's aggregation: kernel inputs, key packing, accumulators
 // and output columns.
+// How the latest rows of this process were aggregated (omg_debug_last_agg_kernel): up to n words.
+void LastAggKernel(int64_t *out, int32_t n);
+
 struct AggPlan {
     std::vector<int32_t> inputCols;        // batch column of each kernel input
     std::vector<int32_t> inputWidths;      // value bytes of each kernel input
