@@ -110,6 +110,12 @@ int32_t omg_config_get_substr_rules(int32_t *negative_rule, int32_t *zero_rule);
 /* Fault injection on the host: the next `n` device allocations of this library fail
  * with OMG_ERR_OOM (0 disables).  Used by the tests; never touches the GPU. */
 int32_t omg_debug_fail_next_allocs(int32_t n);
+/* Host-side too: device allocations that would take this library's buffers beyond `bytes` fail with OMG_ERR_OOM, as on
+ * a device with less memory (0: no limit).  Used by the tests. */
+int32_t omg_debug_limit_device_memory(int64_t bytes);
+/* Bytes of this library's buffers: out[0] device memory held, out[1] the most held since the latest call of this
+ * function, out[2] pinned host memory held.  For tests and measurements. */
+int32_t omg_debug_memory(int64_t *out, int32_t n);
 /* Device-side bounded-wait budget in clock64 ticks (0 = library default). */
 int32_t omg_debug_set_wait_budget(int64_t ticks);
 /* Inner probes on a bitmap ARRAY table that write pinned host output: 1 (default) = the

@@ -29,6 +29,8 @@ _SIGS = {
     "omg_config_set_substr_rules": (I32, [I32, I32]),
     "omg_config_get_substr_rules": (I32, [C.POINTER(I32), C.POINTER(I32)]),
     "omg_debug_fail_next_allocs": (I32, [I32]),
+    "omg_debug_limit_device_memory": (I32, [I64]),
+    "omg_debug_memory": (I32, [C.POINTER(I64), I32]),
     "omg_debug_set_wait_budget": (I32, [I64]),
     "omg_debug_set_staged_probe": (I32, [I32]),
     "omg_debug_set_bulk_probe": (I32, [I32]),

@@ -153,6 +153,20 @@ int32_t omg_debug_fail_next_allocs(int32_t n)
     return OMG_OK;
 }
 
+int32_t omg_debug_limit_device_memory(int64_t bytes)
+{
+    omg::LimitDeviceMemory(bytes < 0 ? 0 : bytes);
+    return OMG_OK;
+}
+
+int32_t omg_debug_memory(int64_t *out, int32_t n)
+{
+    return Guard([&] {
+        Require(out != nullptr && n >= 0, "null output array");
+        omg::MemoryHeld(out, n);
+    });
+}
+
 int32_t omg_debug_set_wait_budget(int64_t ticks)
 {
     omg::SetWaitBudget(ticks < 0 ? 0 : ticks);

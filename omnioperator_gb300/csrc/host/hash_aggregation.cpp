@@ -1288,6 +1288,16 @@ bool LayoutRecord(const AggPlan &plan, const omg::BatchTable &bt, omg::RecLayout
 }
 }  // namespace
 
+// Whether the radix aggregation is for these rows.  It takes an operator's first rows (later ones go to the table):
+// more groups than the partitions of the partitioned strategy hold (the global table it replaces there was behind
+// at every size measured), or rows that those take longer for.
+bool HashAggregationOperator::RadixWanted(int64_t rows) const
+{
+    const Impl &im = *impl_;
+    return strategy_ == 0 && im.capacity == 0 && im.estimate > 0 && rows >= kSketchMinRows &&
+        (im.partBits < 0 || RadixBeatsPartitions(rows));
+}
+
 // Whether the rows of a first flush, whose groups fit the partitions, are better sorted by step than added to
 // the partitions' tables row by row.
 // A double sum there is a compare-and-swap loop, and a CTA takes the rows of one group one after the other, at
@@ -1315,9 +1325,9 @@ bool HashAggregationOperator::RadixBeatsPartitions(int64_t rows) const
     return perCta * 0.35 > 100.0 + static_cast<double>(rows) * 50e-6;
 }
 
-// The key pass and what follows from it: how many partitions, their records and units, and every
-// buffer of the run.  False (nothing changed): the plan's rows do not fit a record, there are more
-// groups than the passes hold, or the device has no memory for the records.
+// The key pass and what follows from it: how many partitions, their records and units, and the
+// buffers of the run.  False (nothing changed): the plan's rows do not fit a record, or there are more
+// groups than the passes hold.
 bool HashAggregationOperator::PlanRadix(omg::BatchTable &bt, RadixRun &run, cudaStream_t s)
 {
     Impl &im = *impl_;
@@ -1328,80 +1338,73 @@ bool HashAggregationOperator::PlanRadix(omg::BatchTable &bt, RadixRun &run, cuda
     }
     constexpr size_t kWords = omg::kRadixFineParts + omg::kRadixHllRegs;
     omg::PinnedArray<unsigned int> h(kWords);
-    try {
-        DevArray<unsigned int> counts(kWords, s, true);
-        omg::AggLaunch p = MakeLaunch(plan_, nullptr, 0, nullptr, nullptr);
-        p.batches = bt.DeviceBatches();
-        p.tiles = bt.DeviceTiles();
-        p.nTiles = bt.NumTiles();
-        CudaCheck(omg::LaunchRadixKeys(p, counts.Get(), counts.Get() + omg::kRadixFineParts, s), "radix key pass");
-        ++counters_[0];
-        CudaCheck(cudaMemcpyAsync(h.Get(), counts.Get(), sizeof(unsigned int) * kWords, cudaMemcpyDeviceToHost, s),
-            "read partition counts");
-        im.stream.Sync();
-        const double groups = omg::HllDistinct(h.Get() + omg::kRadixFineParts, omg::kRadixHllRegs);
-        const uint64_t tables = NextPow2(static_cast<uint64_t>(std::ceil(groups / (kRadixLoad * nSlots))));
-        while (run.bits < omg::kRadixFineBits && (uint64_t(1) << run.bits) < tables) {
-            ++run.bits;
+    DevArray<unsigned int> counts(kWords, s, true);
+    omg::AggLaunch p = MakeLaunch(plan_, nullptr, 0, nullptr, nullptr);
+    p.batches = bt.DeviceBatches();
+    p.tiles = bt.DeviceTiles();
+    p.nTiles = bt.NumTiles();
+    CudaCheck(omg::LaunchRadixKeys(p, counts.Get(), counts.Get() + omg::kRadixFineParts, s), "radix key pass");
+    ++counters_[0];
+    CudaCheck(cudaMemcpyAsync(h.Get(), counts.Get(), sizeof(unsigned int) * kWords, cudaMemcpyDeviceToHost, s),
+        "read partition counts");
+    im.stream.Sync();
+    const double groups = omg::HllDistinct(h.Get() + omg::kRadixFineParts, omg::kRadixHllRegs);
+    const uint64_t tables = NextPow2(static_cast<uint64_t>(std::ceil(groups / (kRadixLoad * nSlots))));
+    while (run.bits < omg::kRadixFineBits && (uint64_t(1) << run.bits) < tables) {
+        ++run.bits;
+    }
+    while ((uint64_t(1) << (run.bits + run.passBits)) < tables) {
+        if (++run.passBits > omg::kRadixMaxPassBits) {
+            return false;
         }
-        while ((uint64_t(1) << (run.bits + run.passBits)) < tables) {
-            if (++run.passBits > omg::kRadixMaxPassBits) {
-                return false;
+    }
+    const uint32_t nParts = 1u << run.bits;
+    const uint32_t fine = omg::kRadixFineParts >> run.bits;
+    const uint64_t unitSlots = static_cast<uint64_t>(nSlots) << run.passBits;
+    run.start.Reset(nParts);
+    std::vector<omg::RadixUnit> units;
+    std::vector<omg::RadixUnit> whole;
+    const uint64_t perCta = (rows / (2 * omg::DeviceSMCount()) + omg::kRadixStepRows) / omg::kRadixStepRows;
+    const uint64_t unitRows = std::min<uint64_t>(kRadixUnitRows, perCta * omg::kRadixStepRows);
+    uint64_t first = 0;
+    uint64_t multi = 0;
+    for (uint32_t q = 0; q < nParts; ++q) {
+        uint64_t n = 0;
+        for (uint32_t f = q * fine; f < (q + 1) * fine; ++f) {
+            n += h[f];
+        }
+        run.start[q] = static_cast<unsigned int>(first);
+        if (n > 2 * unitRows) {
+            ++multi;
+            for (uint64_t r = 0; r < n; r += unitRows) {
+                const uint64_t m = std::min(unitRows, n - r);
+                units.push_back(omg::RadixUnit{static_cast<uint32_t>(first + r), static_cast<uint32_t>(m), 1, 0});
+                run.spillCap += std::min(m, unitSlots);
             }
+        } else if (n > 0) {
+            whole.push_back(omg::RadixUnit{static_cast<uint32_t>(first), static_cast<uint32_t>(n), 0, 0});
+            run.denseCap += std::min(n, unitSlots);
         }
-        const uint32_t nParts = 1u << run.bits;
-        const uint32_t fine = omg::kRadixFineParts >> run.bits;
-        const uint64_t unitSlots = static_cast<uint64_t>(nSlots) << run.passBits;
-        run.start.Reset(nParts);
-        std::vector<omg::RadixUnit> units;
-        std::vector<omg::RadixUnit> whole;
-        const uint64_t perCta = (rows / (2 * omg::DeviceSMCount()) + omg::kRadixStepRows) / omg::kRadixStepRows;
-        const uint64_t unitRows = std::min<uint64_t>(kRadixUnitRows, perCta * omg::kRadixStepRows);
-        uint64_t first = 0;
-        uint64_t multi = 0;
-        for (uint32_t q = 0; q < nParts; ++q) {
-            uint64_t n = 0;
-            for (uint32_t f = q * fine; f < (q + 1) * fine; ++f) {
-                n += h[f];
-            }
-            run.start[q] = static_cast<unsigned int>(first);
-            if (n > 2 * unitRows) {
-                ++multi;
-                for (uint64_t r = 0; r < n; r += unitRows) {
-                    const uint64_t m = std::min(unitRows, n - r);
-                    units.push_back(omg::RadixUnit{static_cast<uint32_t>(first + r), static_cast<uint32_t>(m), 1, 0});
-                    run.spillCap += std::min(m, unitSlots);
-                }
-            } else if (n > 0) {
-                whole.push_back(omg::RadixUnit{static_cast<uint32_t>(first), static_cast<uint32_t>(n), 0, 0});
-                run.denseCap += std::min(n, unitSlots);
-            }
-            first += n;
-        }
-        run.nMulti = static_cast<int32_t>(units.size());
-        units.insert(units.end(), whole.begin(), whole.end());
-        run.nUnits = static_cast<int32_t>(units.size());
-        run.tableGroups = static_cast<uint64_t>(1.1 * groups / nParts * static_cast<double>(multi)) + 64;
-        run.units.Reset(units.size());
-        std::copy(units.begin(), units.end(), run.units.Get());
-        run.cursor.Reset(nParts, s);
-        run.dUnits.Reset(units.size(), s);
-        CudaCheck(cudaMemcpyAsync(run.cursor.Get(), run.start.Get(), sizeof(unsigned int) * nParts,
-                      cudaMemcpyHostToDevice, s),
-            "upload partition starts");
-        CudaCheck(cudaMemcpyAsync(run.dUnits.Get(), run.units.Get(), sizeof(omg::RadixUnit) * units.size(),
-                      cudaMemcpyHostToDevice, s),
-            "upload radix units");
-        run.records.Reset(rows * run.layout.words + 2, s);
-        run.dense.Reset(std::max<uint64_t>(run.denseCap, 1) * plan_.slotWords, s);
-        if (2 * static_cast<uint64_t>(groups) > NextPow2(2 * im.estimate)) {
-            ++counters_[1];  // the estimate would have undersized the table: resized by the key pass
-        }
-    } catch (const OmniException &e) {
-        if (e.GetCode() != "MEM_CAP_EXCEEDED") {
-            throw;
-        }
-        return false;
+        first += n;
+    }
+    run.nMulti = static_cast<int32_t>(units.size());
+    units.insert(units.end(), whole.begin(), whole.end());
+    run.nUnits = static_cast<int32_t>(units.size());
+    run.tableGroups = static_cast<uint64_t>(1.1 * groups / nParts * static_cast<double>(multi)) + 64;
+    run.units.Reset(units.size());
+    std::copy(units.begin(), units.end(), run.units.Get());
+    run.cursor.Reset(nParts, s);
+    run.dUnits.Reset(units.size(), s);
+    CudaCheck(cudaMemcpyAsync(run.cursor.Get(), run.start.Get(), sizeof(unsigned int) * nParts,
+                  cudaMemcpyHostToDevice, s),
+        "upload partition starts");
+    CudaCheck(cudaMemcpyAsync(run.dUnits.Get(), run.units.Get(), sizeof(omg::RadixUnit) * units.size(),
+                  cudaMemcpyHostToDevice, s),
+        "upload radix units");
+    run.records.Reset(rows * run.layout.words + 2, s);
+    run.dense.Reset(std::max<uint64_t>(run.denseCap, 1) * plan_.slotWords, s);
+    if (2 * static_cast<uint64_t>(groups) > NextPow2(2 * im.estimate)) {
+        ++counters_[1];  // the estimate would have undersized the table: resized by the key pass
     }
     return true;
 }
@@ -1592,6 +1595,48 @@ void HashAggregationOperator::Flush(bool last)
         Decide(bt, s);
     }
     FoldDense(s);
+    if (!freshStats) {
+        CudaCheck(cudaMemsetAsync(im.stats.Get() + 1, 0, 5 * sizeof(unsigned long long), s), "reset stats");
+    }
+    // The radix passes need memory that grows with the rows; without it the rows go the other way, as if there were no
+    // such passes.  They are the operator's first, so that there is nothing else in the tables dropped.
+    const bool radix = RadixWanted(rows);
+    try {
+        AggregateRows(bt, last, radix, s);
+    } catch (const OmniException &e) {
+        if (!radix || e.GetCode() != "MEM_CAP_EXCEEDED") {
+            throw;
+        }
+        im.stream.Sync();
+        im.slots.Release();
+        im.special.Release();
+        im.capacity = 0;
+        im.groups = 0;
+        im.dense.Release();
+        im.denseGroups = 0;
+        CudaCheck(cudaMemsetAsync(im.stats.Get(), 0, kStatsWords * sizeof(unsigned long long), s), "reset stats");
+        AggregateRows(bt, last, false, s);
+    }
+    counters_[3] = static_cast<int64_t>(im.groups + im.denseGroups);
+    if (!plan_.orderDependent) {
+        im.keptIds.clear();  // freed stream-ordered, after the kernels that read them
+    }
+    if (plan_.orderDependent) {
+        for (auto *b : pending_) {
+            im.retained.push_back(b);
+        }
+        pending_.clear();
+        pendingRows_ = 0;
+    } else {
+        ReleasePending();
+    }
+}
+
+// The pending rows into the table, or into the dense groups; radix: by the radix passes if they can be had.
+void HashAggregationOperator::AggregateRows(omg::BatchTable &bt, bool last, bool radix, cudaStream_t s)
+{
+    Impl &im = *impl_;
+    const int64_t rows = bt.TotalRows();
     // As few groups as fit every thread's own states: no partitions and no atomics (0.15 ms against 1.22 ms
     // for 2^22 rows of 6 groups).  A group that the estimate missed goes to the global table.
     omg::FewLayout fewLayout;
@@ -1604,12 +1649,8 @@ void HashAggregationOperator::Flush(bool last)
         few = omg::LayoutAggFew(MakeLaunch(plan_, nullptr, 0, nullptr, nullptr), nullable, &fewLayout) &&
             im.estimate + 2 <= static_cast<uint64_t>(fewLayout.maxGroups + fewLayout.firstSlot);
     }
-    // The radix aggregation, on the operator's first rows (later ones go to the table): more groups than the
-    // partitions of the partitioned strategy hold (the global table it replaces there was behind at every
-    // size measured), or rows that those take longer for.
     RadixRun radixRun;
-    const bool radix = strategy_ == 0 && im.capacity == 0 && im.estimate > 0 && rows >= kSketchMinRows && !few &&
-        (im.partBits < 0 || RadixBeatsPartitions(rows)) && PlanRadix(bt, radixRun, s);
+    radix = radix && !few && PlanRadix(bt, radixRun, s);
     // Create the table on first use, sized for the group estimate (load factor <= 1/2).
     if (im.capacity == 0) {
         uint64_t cap = radix ? NextPow2(radixRun.tableGroups * 2)
@@ -1658,9 +1699,6 @@ void HashAggregationOperator::Flush(bool last)
         spillA.Reset(spillCap * plan_.slotWords, s);
     }
     DevArray<uint64_t> spillB;
-    if (!freshStats) {
-        CudaCheck(cudaMemsetAsync(im.stats.Get() + 1, 0, 5 * sizeof(unsigned long long), s), "reset stats");
-    }
     p.retry = retryA.Get();
     p.retryCap = static_cast<uint32_t>(rows);
     p.smemSlots = smemSlots;
@@ -1776,19 +1814,6 @@ void HashAggregationOperator::Flush(bool last)
         im.capacity = need;
         ++counters_[1];
         im.stream.Sync();
-    }
-    counters_[3] = static_cast<int64_t>(im.groups + im.denseGroups);
-    if (!plan_.orderDependent) {
-        im.keptIds.clear();  // freed stream-ordered, after the kernels that read them
-    }
-    if (plan_.orderDependent) {
-        for (auto *b : pending_) {
-            im.retained.push_back(b);
-        }
-        pending_.clear();
-        pendingRows_ = 0;
-    } else {
-        ReleasePending();
     }
 }
 

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
@@ -16,6 +17,10 @@ namespace omg {
 namespace {
 
 std::atomic<int32_t> g_failNext{0};
+std::atomic<int64_t> g_limit{0};       // of g_device
+std::atomic<int64_t> g_device{0};      // bytes of the device buffers alive
+std::atomic<int64_t> g_deviceMost{0};  // the most since MemoryHeld was last called
+std::atomic<int64_t> g_host{0};        // bytes of the pinned buffers alive
 
 // Size classes: powers of two from 4 KiB; larger than 1 GiB is exact-size.
 size_t RoundClass(size_t bytes)
@@ -140,6 +145,17 @@ void HostFree(void *p, size_t bytes)
 
 void SetFailNextDeviceAllocs(int32_t n) { g_failNext.store(n); }
 
+void LimitDeviceMemory(int64_t bytes) { g_limit.store(bytes); }
+
+void MemoryHeld(int64_t *out, int32_t n)
+{
+    const int64_t held = g_device.load();
+    const int64_t v[3] = {held, std::max(held, g_deviceMost.exchange(held)), g_host.load()};
+    for (int32_t i = 0; i < n; ++i) {
+        out[i] = i < 3 ? v[i] : 0;
+    }
+}
+
 void *DeviceAlloc(size_t bytes, void *stream)
 {
     using omniruntime::exception::OmniException;
@@ -151,6 +167,11 @@ void *DeviceAlloc(size_t bytes, void *stream)
         if (g_failNext.compare_exchange_weak(f, f - 1)) {
             throw OmniException("MEM_CAP_EXCEEDED", "injected device allocation failure", -4);
         }
+    }
+    const int64_t limit = g_limit.load();
+    if (limit > 0 && g_device.load() + static_cast<int64_t>(bytes) > limit) {
+        throw OmniException("MEM_CAP_EXCEEDED",
+            "device allocation of " + std::to_string(bytes) + " bytes is beyond the limit set", -4);
     }
     ConfigurePool();
     void *p = nullptr;
@@ -174,11 +195,13 @@ Buffer::~Buffer()
 {
     switch (kind_) {
         case Kind::HOST:
+            g_host -= static_cast<int64_t>(bytes_);
             HostFree(ptr_, bytes_);
             break;
         case Kind::DEVICE:
             // Stream-ordered free: every use of this buffer was issued on its stream before
             // the buffer's last reference went away.
+            g_device -= static_cast<int64_t>(bytes_);
             DeviceFree(ptr_, stream_);
             break;
         default:
@@ -193,6 +216,7 @@ std::shared_ptr<Buffer> Buffer::NewHost(size_t bytes, bool zero)
         throw omniruntime::exception::OmniException("MEM_CAP_EXCEEDED",
             "host allocation of " + std::to_string(bytes) + " bytes failed", -4);
     }
+    g_host += static_cast<int64_t>(bytes);
     return std::make_shared<Buffer>(Kind::HOST, p, bytes);
 }
 
@@ -201,6 +225,10 @@ std::shared_ptr<Buffer> Buffer::NewDevice(size_t bytes, void *stream, bool zero)
     void *p = DeviceAlloc(bytes, stream);
     if (zero) {
         cudaMemsetAsync(p, 0, bytes, static_cast<cudaStream_t>(stream));
+    }
+    const int64_t held = g_device += static_cast<int64_t>(bytes);
+    int64_t most = g_deviceMost.load();
+    while (held > most && !g_deviceMost.compare_exchange_weak(most, held)) {
     }
     return std::make_shared<Buffer>(Kind::DEVICE, p, bytes, stream);
 }

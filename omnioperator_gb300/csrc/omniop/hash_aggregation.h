@@ -153,10 +153,12 @@ private:
     void Partition(omg::BatchTable &bt, omg::AggLaunch &p, PartBuffers &pb, cudaStream_t s);
     bool PlanRadix(omg::BatchTable &bt, RadixRun &run, cudaStream_t s);
     bool RadixBeatsPartitions(int64_t rows) const;
+    bool RadixWanted(int64_t rows) const;
     void FoldDense(cudaStream_t s);
     struct ExtractRun;
     // last: no more rows will come.
     void Flush(bool last = false);
+    void AggregateRows(omg::BatchTable &bt, bool last, bool radix, cudaStream_t s);
     void AllocOutputs(ExtractRun &x, uint64_t bound, cudaStream_t s);
     void LaunchExtract(ExtractRun &x, uint64_t bound, cudaStream_t s);
     bool ExtractSmall();

@@ -33,6 +33,10 @@ void DeviceFree(void *p, void *stream);
 
 // Host-side fault injection: the next n DeviceAlloc calls fail.
 void SetFailNextDeviceAllocs(int32_t n);
+// Device allocations beyond `bytes` in all fail (0: no limit); up to n of: device bytes held, the most since the latest
+// call, pinned host bytes held.
+void LimitDeviceMemory(int64_t bytes);
+void MemoryHeld(int64_t *out, int32_t n);
 
 // A reference-counted memory block: host (pinned) or device, owned or borrowed.
 class Buffer {
