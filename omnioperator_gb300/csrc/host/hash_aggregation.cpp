@@ -1290,11 +1290,12 @@ bool LayoutRecord(const AggPlan &plan, const omg::BatchTable &bt, omg::RecLayout
 
 // Whether the radix aggregation is for these rows.  It takes an operator's first rows (later ones go to the table):
 // more groups than the partitions of the partitioned strategy hold (the global table it replaces there was behind
-// at every size measured), or rows that those take longer for.
+// at every size measured), or rows that those take longer for.  Not under a memory budget, which is for the table: the
+// passes hold the rows once more, and their groups beside the table.
 bool HashAggregationOperator::RadixWanted(int64_t rows) const
 {
     const Impl &im = *impl_;
-    return strategy_ == 0 && im.capacity == 0 && im.estimate > 0 && rows >= kSketchMinRows &&
+    return strategy_ == 0 && !spillEnabled_ && !spillPart_ && im.capacity == 0 && im.estimate > 0 && rows >= kSketchMinRows &&
         (im.partBits < 0 || RadixBeatsPartitions(rows));
 }
 
@@ -2106,6 +2107,7 @@ bool HashAggregationOperator::ExtractSpilled()
         }
         HashAggregationOperator part(partPlan, sizer_);
         part.SetStrategy(strategy_, 0);
+        part.spillPart_ = true;
         // String keys are decoded on the device: the partition's output stays there until then.
         part.SetDeviceOutput(deviceOutput_ || !strKeyOuts.empty());
         if (userStreamSet_) {

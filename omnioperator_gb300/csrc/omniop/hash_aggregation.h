@@ -184,6 +184,7 @@ private:
     int64_t capacityHint_ = 0;
     int32_t sizing_ = 0;
     bool spillEnabled_ = false;
+    bool spillPart_ = false;  // aggregates one partition of a spilled run
     uint64_t spillBudget_ = 0;
     uint64_t spilledBytes_ = 0;
     omg::SizingModel *sizer_ = nullptr;

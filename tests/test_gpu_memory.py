@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 import omnioperator_gb300 as omg
+from helpers import run_agg
 
 pytestmark = pytest.mark.gpu
 
@@ -70,3 +71,21 @@ def test_radix_passes_without_the_memory_for_them(gpu):
         assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
     assert kernels == {1}
     assert np.array_equal(free[0], want[0]) and np.array_equal(free[1], want[1])
+
+
+@pytest.mark.parametrize("budget", [40 * MB, 200 * MB])
+def test_budgeted_aggregations_take_no_radix_passes(gpu, budget):
+    """A budget is for the group table (64 MB here): neither the partitions of a spilled run nor a run that fits are
+    aggregated by passes that hold the rows and the groups once more."""
+    rng = np.random.default_rng(2)
+    n = 2_000_000
+    key = rng.integers(0, 1_000_000, n) * 7919
+    v = rng.integers(-2**40, 2**40, n)
+    cols, _ = run_agg([0], [L], [[1], [1]], [[L], [L]], [[L], [L]], [SUM, CNT], [key, v], [L, L], batch_sizes=(n,),
+                      spill_budget=budget)
+    assert last_agg_kernel() != 4
+    order = np.argsort(cols[0][0])
+    uniq, inv = np.unique(key, return_inverse=True)
+    want = np.zeros(len(uniq), np.int64)
+    np.add.at(want, inv, v)
+    assert np.array_equal(cols[0][0][order], uniq) and np.array_equal(cols[1][0][order], want)
