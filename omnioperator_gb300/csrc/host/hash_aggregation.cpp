@@ -1410,7 +1410,8 @@ bool HashAggregationOperator::PlanRadix(omg::BatchTable &bt, RadixRun &run, cuda
     return true;
 }
 
-// Move the dense groups into the table, grown to hold them, for more input or an ordered replay.
+// Move the dense groups into the table, grown to hold them at a load of at most one half as for a good estimate,
+// for more input or an ordered replay.
 void HashAggregationOperator::FoldDense(cudaStream_t s)
 {
     Impl &im = *impl_;
@@ -1418,7 +1419,7 @@ void HashAggregationOperator::FoldDense(cudaStream_t s)
         return;
     }
     const uint64_t all = im.groups + im.denseGroups;
-    const uint64_t need = NextPow2(std::max<uint64_t>(im.capacity, 4 * all));
+    const uint64_t need = NextPow2(std::max<uint64_t>(im.capacity, 2 * all));
     DevArray<uint64_t> newSlots((need + 2) * plan_.slotWords, s);
     DevArray<uint32_t> newSpecial(2, s, true);
     DevArray<uint32_t> noSpecial(2, s, true);

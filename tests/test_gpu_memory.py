@@ -89,3 +89,32 @@ def test_budgeted_aggregations_take_no_radix_passes(gpu, budget):
     want = np.zeros(len(uniq), np.int64)
     np.add.at(want, inv, v)
     assert np.array_equal(cols[0][0][order], uniq) and np.array_equal(cols[1][0][order], want)
+
+
+def test_more_rows_after_a_radix_flush(gpu):
+    """The groups of the first rows move into a table of the size that an exact estimate would have given it."""
+    n, groups = 500_000, 260_000
+    key = np.arange(n, dtype=np.int64) % groups * 7919
+    slots = 1 << 19  # the least power of two that is at least twice the groups
+    slot_bytes = 8 * 4  # key, COUNT(*), NULLs, sum
+    fac = omg.HashAggregationOperatorFactory([0], [L], [[1], [1]], [[L], [L]], [[L], [L]], [SUM, CNT])
+    op = fac.create_operator()
+    try:
+        op.set_agg_strategy(omg.AGG_STRATEGY_AUTO, groups)
+        omg.lib().omg_debug_set_agg_flush_rows(n)
+        before = memory()[0]
+        for k in range(2):
+            op.add_input(omg.make_batch([L, L], [key, np.full(n, k + 1)]))
+            assert last_agg_kernel() == (4, 1)[k]
+        assert memory()[0] - before <= (slots + 2) * slot_bytes + MB
+        outs = op.drain()
+        cols = [omg.batch_to_numpy(b) for b in outs]
+        omg.free_batches(outs)
+    finally:
+        omg.lib().omg_debug_set_agg_flush_rows(0)
+        op.delete()
+        fac.close()
+    got = np.concatenate([c[0][0] for c in cols])
+    order = np.argsort(got)
+    assert np.array_equal(got[order], np.unique(key))
+    assert np.array_equal(np.concatenate([c[1][0] for c in cols])[order], 3 * np.bincount(key // 7919))
