@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <condition_variable>
 #include <cstring>
 #include <exception>
@@ -83,7 +84,8 @@ struct JoinBuildState {
     DevArray<int32_t> csr;
     int64_t csrCount = 0;
     omg::JoinTable table{};
-    uint32_t maxDup = 0;
+    uint32_t maxDup = 0;   // the most rows of a key
+    double meanDup = 1.0;  // rows per key
     DevArray<uint8_t> visited;  // BUILD_OUTER / FULL: one byte per build row, set by the probes
     // Several key columns (or one 16-byte key): the table is keyed by the tuple hash of each row,
     // unless the key columns are fixed widths of 1-8 bytes whose build value ranges multiply to at
@@ -290,6 +292,7 @@ void JoinBuildState::Build()
     uint32_t *sentinelCount = reinterpret_cast<uint32_t *>(stats.Get() + 4);
     unsigned int *sentinelCursor = reinterpret_cast<unsigned int *>(stats.Get() + 5);
     int64_t *sentinelEntry = reinterpret_cast<int64_t *>(stats.Get() + 6);
+    unsigned int *distinct = reinterpret_cast<unsigned int *>(stats.Get() + 7);  // zero so far
     CudaCheck(cudaMemsetAsync(stats.Get() + 3, 0, 3 * sizeof(long long), s), "reset");
     CudaCheck(omg::LaunchFillI64(sentinelEntry, -1, 1, s), "reset");
     uint64_t n;
@@ -306,9 +309,9 @@ void JoinBuildState::Build()
     }
     DevArray<uint32_t> counts(n, s, true);
     CudaCheck(omg::LaunchBuildCount(table, keys, keyNulls, rows, keyWidth, hashSlots.Get(), counts.Get(), sentinelCount,
-                  maxCount, err.Get(), s),
+                  maxCount, distinct, err.Get(), s),
         "build count");
-    long long h2[3];
+    long long h2[5];
     CudaCheck(cudaMemcpyAsync(h2, stats.Get() + 3, sizeof(h2), cudaMemcpyDeviceToHost, s), "read build stats");
     int32_t herr = 0;
     CudaCheck(cudaMemcpyAsync(&herr, err.Get(), sizeof(herr), cudaMemcpyDeviceToHost, s), "read error");
@@ -317,6 +320,7 @@ void JoinBuildState::Build()
         throw OmniException("OPERATOR_RUNTIME_ERROR", "join build failed", -9);
     }
     maxDup = static_cast<uint32_t>(h2[0] & 0xffffffffll);
+    meanDup = static_cast<double>(nonNull) / static_cast<double>(std::max<long long>(h2[4] & 0xffffffffll, 1));
     const uint32_t nSentinel = static_cast<uint32_t>(h2[1] & 0xffffffffll);
     table.unique = (maxDup <= 1 && nSentinel <= 1) ? 1 : 0;
     if (arrayMode) {
@@ -1442,7 +1446,7 @@ std::unique_ptr<LookupJoinOperator::ProbeCall> LookupJoinOperator::LaunchBatches
         }
     }
     // Output regions: tile t writes into region t % nRegions (see ProbeLaunch).  A region's
-    // capacity starts at its probe rows (times up to 2 for duplicate build keys), rounded to 64
+    // capacity starts at its probe rows (times what duplicate build keys may come to), rounded to 64
     // rows so that every region starts on a byte of the null bitmaps.
     const int32_t nRegions = std::max(1, std::min<int32_t>(omg::kMaxRegions, bt.NumTiles()));
     const std::vector<int64_t> regionRows = bt.RegionRows(nRegions);
@@ -1451,14 +1455,22 @@ std::unique_ptr<LookupJoinOperator::ProbeCall> LookupJoinOperator::LaunchBatches
         regionCap = std::max<uint64_t>(regionCap, static_cast<uint64_t>(r));
     }
     if (!b.table.unique) {
-        // Room for every key's duplicates while that is at most a gigabyte (64 MiB of pinned memory): a
-        // region that overflows costs the probe a second run.
-        uint64_t rowBytes = 0;
+        // Room for the rows of a key in the mean and an eighth more, while that is at most a gigabyte (64 MiB of
+        // pinned memory), or for two: a region that overflows costs the probe a second run, and the key with the
+        // most rows may have a thousand times the mean.
+        double rowBytes = 0.0;
         for (const omg::OutColumn &c : cols) {
-            rowBytes += c.width == 0 ? 8 : static_cast<uint64_t>(c.width);
+            rowBytes += c.width == 0 ? 8 : c.width;
         }
-        const uint64_t bytes = regionCap * static_cast<uint64_t>(nRegions) * rowBytes * b.maxDup;
-        regionCap *= bytes <= (uint64_t(1) << (deviceOutput_ ? 30 : 26)) ? b.maxDup : std::min<uint32_t>(b.maxDup, 2);
+        const double most = std::max<uint32_t>(b.maxDup, 1);
+        const double least = std::min(most, 2.0);
+        const bool oneRow = b.kind == omg::JOIN_KIND_SEMI || b.kind == omg::JOIN_KIND_ANTI ||
+            b.kind == omg::JOIN_KIND_EXISTENCE;  // at most, for a probe row
+        double times = oneRow ? least : std::min(most, std::max(least, 1.125 * b.meanDup));
+        if (static_cast<double>(regionCap) * nRegions * rowBytes * times > (deviceOutput_ ? 1 << 30 : 1 << 26)) {
+            times = least;
+        }
+        regionCap = static_cast<uint64_t>(std::ceil(static_cast<double>(regionCap) * times));
     }
     regionCap = (regionCap + 63) / 64 * 64;
     // The region counters, then one more 128-byte line whose first word is the kernel's error.

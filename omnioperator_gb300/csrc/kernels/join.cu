@@ -169,9 +169,11 @@ __device__ __forceinline__ int64_t HashSlot(uint64_t *slots, uint64_t capacity, 
 }
 
 __global__ void BuildCountKernel(JoinTable t, const void *keys, const uint8_t *nulls, int64_t n, int32_t width,
-    uint64_t *hashSlots, uint32_t *counts, uint32_t *sentinelCount, unsigned int *maxCount, int32_t *error)
+    uint64_t *hashSlots, uint32_t *counts, uint32_t *sentinelCount, unsigned int *maxCount, unsigned int *distinct,
+    int32_t *error)
 {
-    uint32_t most = 0;  // the largest count this thread saw: one atomic per warp, not one per duplicate
+    uint32_t most = 0;   // the largest count this thread saw: one atomic per warp, not one per duplicate
+    uint32_t fresh = 0;  // keys that this thread saw first
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         if (RowIsNull(nulls, i)) {
@@ -192,8 +194,13 @@ __global__ void BuildCountKernel(JoinTable t, const void *keys, const uint8_t *n
             old = atomicAdd(&counts[s], 1u);
         }
         most = max(most, old + 1);
+        fresh += old == 0 ? 1u : 0u;
     }
     most = __reduce_max_sync(0xffffffffu, most);
+    fresh = __reduce_add_sync(0xffffffffu, fresh);
+    if ((threadIdx.x & 31) == 0 && fresh != 0) {
+        atomicAdd(distinct, fresh);
+    }
     if ((threadIdx.x & 31) == 0 && most > 1) {
         atomicMax(maxCount, most);
     }
@@ -3048,14 +3055,14 @@ cudaError_t LaunchKeyStats(const void *keys, const uint8_t *nulls, int64_t n, in
 }
 
 cudaError_t LaunchBuildCount(JoinTable t, const void *keys, const uint8_t *nulls, int64_t n, int32_t width,
-    uint64_t *hashSlotsMutable, uint32_t *counts, uint32_t *sentinelCount, unsigned int *maxCount, int32_t *error,
-    cudaStream_t stream)
+    uint64_t *hashSlotsMutable, uint32_t *counts, uint32_t *sentinelCount, unsigned int *maxCount,
+    unsigned int *distinct, int32_t *error, cudaStream_t stream)
 {
     if (n == 0) {
         return cudaSuccess;
     }
     BuildCountKernel<<<GridFor(n, 256, 8), 256, 0, stream>>>(t, keys, nulls, n, width, hashSlotsMutable, counts,
-        sentinelCount, maxCount, error);
+        sentinelCount, maxCount, distinct, error);
     return cudaGetLastError();
 }
 

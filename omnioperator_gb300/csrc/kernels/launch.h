@@ -91,10 +91,11 @@ cudaError_t LaunchGatherColumn(const BatchDesc *batches, const TileDesc *tiles, 
 // stats[0] = min, stats[1] = max, stats[2] = count (initialised by the launcher).
 cudaError_t LaunchKeyStats(const void *keys, const uint8_t *nulls, int64_t n, int32_t width,
     long long *stats, cudaStream_t stream);
-// ARRAY mode: counts[key - min] += 1; HASH mode: insert keys, counts per slot.
+// ARRAY mode: counts[key - min] += 1; HASH mode: insert keys, counts per slot.  maxCount: the largest count
+// above 1; distinct: keys (both added to, from 0).
 cudaError_t LaunchBuildCount(JoinTable t, const void *keys, const uint8_t *nulls, int64_t n, int32_t width,
     uint64_t *hashSlotsMutable, uint32_t *counts, uint32_t *sentinelCount, unsigned int *maxCount,
-    int32_t *error, cudaStream_t stream);
+    unsigned int *distinct, int32_t *error, cudaStream_t stream);
 // Exclusive scan of uint32 counts into int64 offsets; total written to *total.
 cudaError_t LaunchScanCounts(const uint32_t *counts, int64_t n, int64_t *offsets, int64_t *blockSums,
     long long *total, cudaStream_t stream);

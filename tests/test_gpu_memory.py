@@ -118,3 +118,73 @@ def test_more_rows_after_a_radix_flush(gpu):
     order = np.argsort(got)
     assert np.array_equal(got[order], np.unique(key))
     assert np.array_equal(np.concatenate([c[1][0] for c in cols])[order], 3 * np.bincount(key // 7919))
+
+
+def _join(bkey, pay, ptype, pkey, batch=None, device=True, limit=0, filt=None, kind=omg.OMNI_JOIN_TYPE_INNER, state=None):
+    """Rows (key, payload) of the join and what memory it took: (rows sorted, device bytes held by the outputs, peak,
+    counters, pinned bytes held by the outputs)."""
+    bf = omg.HashBuilderOperatorFactory(kind, [L, ptype], [0])
+    bop = bf.create_operator()
+    bop.add_input(omg.make_batch([L, ptype], [bkey, pay]))
+    bop.get_output()
+    pf = omg.LookupJoinOperatorFactory([L], [0], [0], [1], [ptype], bf, filter_expr=filt)
+    op = pf.create_operator()
+    try:
+        op.set_device_output(device)
+        host = omg.make_batch([L], [pkey])
+        b = omg.batch_to_device(host)
+        omg.free_batch(host)
+        before = memory()
+        omg.lib().omg_debug_limit_device_memory(before[0] + limit if limit else 0)
+        op.add_input(b)
+        outs = op.drain()
+        ctr = op.counters()
+        after = memory()
+        omg.lib().omg_debug_limit_device_memory(0)
+        parts = []
+        for o in outs:
+            h = omg.batch_to_host(o) if device else o
+            parts.append(omg.batch_to_numpy(h))
+            if device:
+                omg.free_batch(h)
+        omg.free_batches(outs)
+    finally:
+        omg.lib().omg_debug_limit_device_memory(0)
+        op.delete()
+        pf.close()
+        bop.delete()
+        bf.close()
+    keys, vals = (np.concatenate([p[c][0] for p in parts]) if parts else np.zeros(0, np.int64) for c in (0, 1))
+    order = np.lexsort([vals, keys])
+    return keys[order], vals[order], after[0] - before[0], after[1] - before[0], ctr, after[2] - before[2]
+
+
+def _joined(bkey, pay, pkey):
+    order = np.argsort(bkey, kind="stable")
+    lo, hi = np.searchsorted(bkey[order], pkey, "left"), np.searchsorted(bkey[order], pkey, "right")
+    n = hi - lo
+    rows = np.repeat(lo, n) + np.arange(n.sum()) - np.repeat(np.cumsum(n) - n, n)
+    keys, vals = np.repeat(pkey, n), pay[order][rows]
+    order = np.lexsort([vals, keys])
+    return keys[order], vals[order]
+
+
+def _hot_build():
+    """One key of 1,000 rows, 64,000 of one row."""
+    bkey = np.concatenate([np.arange(64_000), np.full(999, 77)]) * 1_000_003
+    return bkey, np.arange(len(bkey), dtype=np.int32)
+
+
+@pytest.mark.parametrize("hot", [0, 300])
+def test_join_reserves_for_the_mean_of_a_key(gpu, hot):
+    """65,536 probe rows, of which none or 300 are of the key with 1,000 rows: rooms for 1,000 rows each would be
+    786 MB.  Where the hot key overflows them the probe runs once more at the exact size."""
+    bkey, pay = _hot_build()
+    pkey = (np.random.default_rng(3).integers(100, 64_000, 65_536)) * 1_000_003
+    pkey[:hot] = 77 * 1_000_003
+    keys, vals, held, peak, ctr, _ = _join(bkey, pay, I, pkey)
+    want = _joined(bkey, pay, pkey)
+    assert np.array_equal(keys, want[0]) and np.array_equal(vals, want[1])
+    assert ctr["resizes"] == (1 if hot else 0)
+    if not hot:
+        assert held <= 2 * len(pkey) * 12 + 2 * MB and peak <= 4 * len(pkey) * 12 + 2 * MB
