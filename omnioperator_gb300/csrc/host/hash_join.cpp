@@ -1458,15 +1458,18 @@ std::unique_ptr<LookupJoinOperator::ProbeCall> LookupJoinOperator::LaunchBatches
         // Room for the rows of a key in the mean and an eighth more, while that is at most a gigabyte (64 MiB of
         // pinned memory), or for two: a region that overflows costs the probe a second run, and the key with the
         // most rows may have a thousand times the mean.
+        // Strings are built by passes over every position reserved, with more bytes each: two there.
         double rowBytes = 0.0;
+        bool strings = false;
         for (const omg::OutColumn &c : cols) {
-            rowBytes += c.width == 0 ? 8 : c.width;
+            rowBytes += c.width;
+            strings = strings || c.width == 0;
         }
         const double most = std::max<uint32_t>(b.maxDup, 1);
         const double least = std::min(most, 2.0);
         const bool oneRow = b.kind == omg::JOIN_KIND_SEMI || b.kind == omg::JOIN_KIND_ANTI ||
             b.kind == omg::JOIN_KIND_EXISTENCE;  // at most, for a probe row
-        double times = oneRow ? least : std::min(most, std::max(least, 1.125 * b.meanDup));
+        double times = oneRow || strings ? least : std::min(most, std::max(least, 1.125 * b.meanDup));
         if (static_cast<double>(regionCap) * nRegions * rowBytes * times > (deviceOutput_ ? 1 << 30 : 1 << 26)) {
             times = least;
         }

@@ -188,3 +188,24 @@ def test_join_reserves_for_the_mean_of_a_key(gpu, hot):
     assert ctr["resizes"] == (1 if hot else 0)
     if not hot:
         assert held <= 2 * len(pkey) * 12 + 2 * MB and peak <= 4 * len(pkey) * 12 + 2 * MB
+
+
+def _few_hits(varchar):
+    """2,000 keys of 50 rows each, and 65,536 probe rows of which one in a hundred has a match."""
+    rng = np.random.default_rng(4)
+    bkey = np.repeat(np.arange(2000), 50) * 1_000_003
+    pay = np.arange(len(bkey), dtype=np.int32)
+    if varchar:
+        pay = np.array([b"%05d" % p for p in pay], dtype=object)
+    pkey = np.where(rng.random(65_536) < 0.01, rng.integers(0, 2000, 65_536), 5000 + rng.integers(0, 2000, 65_536))
+    return bkey, pay, pkey * 1_000_003
+
+
+@pytest.mark.parametrize("device", [False, True])
+def test_strings_of_a_join_are_built_over_two_rows_a_probe_row(gpu, device):
+    """Not over the 50 rows that a key has: row numbers, lengths, two kinds of offsets, 24 bytes a position."""
+    bkey, pay, pkey = _few_hits(True)
+    keys, vals, _, peak, _, _ = _join(bkey, pay, V, pkey, device=device)
+    want = _joined(bkey, pay, pkey)
+    assert np.array_equal(keys, want[0]) and np.array_equal(vals, want[1])
+    assert peak <= 2 * len(pkey) * (8 + 24) + 2 * MB
