@@ -979,6 +979,7 @@ struct LookupJoinOperator::ProbeCall {
     size_t nProbeOut = 0;
     int32_t nRegions = 0;
     uint64_t regionCap = 0;
+    uint64_t leastCap = 0;  // what a region needs to hold before it may be told to hold less
     bool hostDirect = false;
     DevArray<unsigned long long> count;
     omg::PinnedArray<unsigned long long> hostCount;
@@ -1454,6 +1455,7 @@ std::unique_ptr<LookupJoinOperator::ProbeCall> LookupJoinOperator::LaunchBatches
     for (int64_t r : regionRows) {
         regionCap = std::max<uint64_t>(regionCap, static_cast<uint64_t>(r));
     }
+    uint64_t leastCap = regionCap;
     if (!b.table.unique) {
         // Room for the rows of a key in the mean and an eighth more, while that is at most a gigabyte (64 MiB of
         // pinned memory), or for two: a region that overflows costs the probe a second run, and the key with the
@@ -1473,9 +1475,11 @@ std::unique_ptr<LookupJoinOperator::ProbeCall> LookupJoinOperator::LaunchBatches
         if (static_cast<double>(regionCap) * nRegions * rowBytes * times > (deviceOutput_ ? 1 << 30 : 1 << 26)) {
             times = least;
         }
+        leastCap = regionCap * std::min<uint32_t>(std::max<uint32_t>(b.maxDup, 1), 2);
         regionCap = static_cast<uint64_t>(std::ceil(static_cast<double>(regionCap) * times));
     }
     regionCap = (regionCap + 63) / 64 * 64;
+    leastCap = (leastCap + 63) / 64 * 64;
     // The region counters, then one more 128-byte line whose first word is the kernel's error.
     pc.count.Reset(static_cast<size_t>(nRegions + 1) * omg::kRegionStride, s, true);
     pc.hostCount.Reset(static_cast<size_t>(nRegions + 1) * omg::kRegionStride);
@@ -1494,6 +1498,7 @@ std::unique_ptr<LookupJoinOperator::ProbeCall> LookupJoinOperator::LaunchBatches
     p.hostOutput = hostDirect ? 1 : 0;
     p.deviceKeys = b.packed || (!b.multiKey && bt.AllOnDevice(p.keyInput)) ? 1 : 0;
     pc.regionCap = regionCap;
+    pc.leastCap = leastCap;
     pc.nRegions = nRegions;
     pc.nOut = nOut;
     pc.nProbeOut = nProbeOut;
@@ -1524,12 +1529,9 @@ std::unique_ptr<LookupJoinOperator::ProbeCall> LookupJoinOperator::LaunchBatches
     return call;
 }
 
-// Output buffers for the call's region capacity, the kernel, and the asynchronous copy of the
-// region counts; the call's event marks the end.
-void LookupJoinOperator::LaunchAttempt(ProbeCall &pc)
+// Output buffers for the call's region capacity.
+void LookupJoinOperator::ReserveOutput(ProbeCall &pc)
 {
-    cudaStream_t s = pc.s;
-    omg::ProbeLaunch &p = pc.p;
     const uint64_t capacity = pc.regionCap * static_cast<uint64_t>(pc.nRegions);
     for (size_t o = 0; o < pc.nOut; ++o) {
         omg::OutColumn &c = pc.cols[o];
@@ -1537,11 +1539,78 @@ void LookupJoinOperator::LaunchAttempt(ProbeCall &pc)
         const size_t vw = c.width == 0 ? 8 : static_cast<size_t>(c.width);
         const size_t nb = omg::NullBitmapBytes(static_cast<int64_t>(capacity));
         c.values = pc.hostDirect ? omg::Buffer::NewHost(capacity * vw + 16, false)
-                                 : omg::Buffer::NewDevice(capacity * vw + 16, s, false);
+                                 : omg::Buffer::NewDevice(capacity * vw + 16, pc.s, false);
         c.nulls = !c.hasNull ? nullptr
-                             : (pc.hostDirect ? omg::Buffer::NewHost(nb, true) : omg::Buffer::NewDevice(nb, s, true));
-        p.out[o].values = c.values->Data();
-        p.out[o].nulls = c.nulls ? static_cast<uint8_t *>(c.nulls->Data()) : nullptr;
+                             : (pc.hostDirect ? omg::Buffer::NewHost(nb, true) : omg::Buffer::NewDevice(nb, pc.s, true));
+    }
+}
+
+// The rows of a region (of at most `most` each) side by side in buffers of their size, where the rooms for duplicates
+// have turned out more than twice too large: the output batches hold the buffers for as long as any of them lives.
+void LookupJoinOperator::TrimOutput(ProbeCall &pc, uint64_t most)
+{
+    const uint64_t cap = std::max<uint64_t>((most + 63) / 64 * 64, 64);
+    if (pc.regionCap <= pc.leastCap || 2 * cap > pc.regionCap) {
+        return;
+    }
+    // Columns and then bitmaps, `width` bytes a region.
+    auto move = [&](omg::BufferPtr &buf, size_t width, size_t pitch, size_t extra) {
+        const size_t n = static_cast<size_t>(pc.nRegions);
+        if (pc.hostDirect) {
+            auto to = omg::Buffer::NewHost(width * n + extra, false);
+            for (size_t r = 0; r < n; ++r) {
+                std::memcpy(static_cast<char *>(to->Data()) + r * width, static_cast<char *>(buf->Data()) + r * pitch, width);
+            }
+            buf = to;
+            return;
+        }
+        auto to = omg::Buffer::NewDevice(width * n + extra, pc.s, false);
+        CudaCheck(cudaMemcpy2DAsync(to->Data(), width, buf->Data(), pitch, width, n, cudaMemcpyDeviceToDevice, pc.s),
+            "trim output");
+        buf = to;
+    };
+    std::vector<omg::OutColumn> cols = pc.cols;
+    try {
+        for (omg::OutColumn &c : cols) {
+            move(c.values, cap * static_cast<size_t>(c.width), pc.regionCap * static_cast<size_t>(c.width), 16);
+            if (c.nulls) {
+                move(c.nulls, cap / 8, pc.regionCap / 8, 12);
+            }
+        }
+    } catch (const OmniException &e) {
+        if (e.GetCode() != "MEM_CAP_EXCEEDED") {
+            throw;
+        }
+        return;  // no memory for the copies: the rows stay where they are
+    }
+    if (!pc.hostDirect) {
+        CudaCheck(cudaStreamSynchronize(pc.s), "cudaStreamSynchronize");  // readable on every stream, as they were
+    }
+    pc.cols = std::move(cols);
+    pc.regionCap = cap;
+}
+
+// The output buffers, the kernel, and the asynchronous copy of the region counts; the call's event marks the end.
+void LookupJoinOperator::LaunchAttempt(ProbeCall &pc)
+{
+    cudaStream_t s = pc.s;
+    omg::ProbeLaunch &p = pc.p;
+    try {
+        ReserveOutput(pc);
+    } catch (const OmniException &e) {
+        if (e.GetCode() != "MEM_CAP_EXCEEDED" || pc.regionCap <= pc.leastCap) {
+            throw;
+        }
+        for (omg::OutColumn &c : pc.cols) {
+            c.values.reset();
+            c.nulls.reset();
+        }
+        pc.regionCap = pc.leastCap;
+        ReserveOutput(pc);
+    }
+    for (size_t o = 0; o < pc.nOut; ++o) {
+        p.out[o].values = pc.cols[o].values->Data();
+        p.out[o].nulls = pc.cols[o].nulls ? static_cast<uint8_t *>(pc.cols[o].nulls->Data()) : nullptr;
     }
     p.regionCap = pc.regionCap;
     CudaCheck(cudaMemsetAsync(pc.count.Get(), 0, sizeof(unsigned long long) * pc.count.Size(), s), "reset counts");
@@ -1572,6 +1641,7 @@ void LookupJoinOperator::FinishProbe(ProbeCall &pc, std::deque<VectorBatch *> &o
     const int32_t nRegions = pc.nRegions;
     const bool hostDirect = pc.hostDirect;
     std::vector<int64_t> regionCount(nRegions, 0);
+    uint64_t most = 0;
     for (int attempt = 0; attempt < 2; ++attempt) {
         const auto tw = std::chrono::steady_clock::now();
         CudaCheck(cudaEventSynchronize(pc.done), "probe kernel");
@@ -1584,7 +1654,7 @@ void LookupJoinOperator::FinishProbe(ProbeCall &pc, std::deque<VectorBatch *> &o
                 kerr == 7 ? "probe kernel: a bounded wait for a bulk copy ran out" : "probe kernel error " + std::to_string(kerr),
                 kerr == 7 ? -7 : -9);
         }
-        uint64_t most = 0;
+        most = 0;
         for (int32_t r = 0; r < nRegions; ++r) {
             regionCount[r] = static_cast<int64_t>(pc.hostCount[static_cast<size_t>(r) * omg::kRegionStride]);
             most = std::max<uint64_t>(most, static_cast<uint64_t>(regionCount[r]));
@@ -1593,9 +1663,11 @@ void LookupJoinOperator::FinishProbe(ProbeCall &pc, std::deque<VectorBatch *> &o
             break;
         }
         pc.regionCap = (most + 63) / 64 * 64;  // exact size known now: run once more
+        pc.leastCap = pc.regionCap;
         ++counters_[1];
         LaunchAttempt(pc);
     }
+    TrimOutput(pc, most);
     const uint64_t regionCap = pc.regionCap;
     // VARCHAR outputs: row handles -> lengths -> offsets -> characters, over all regions at once
     // (positions past a region's count contribute nothing).

@@ -142,6 +142,8 @@ private:
     void ProcessPending();
     std::unique_ptr<ProbeCall> LaunchPending();
     std::unique_ptr<ProbeCall> LaunchBatches(std::vector<VectorBatch *> &&batches);
+    void ReserveOutput(ProbeCall &pc);
+    void TrimOutput(ProbeCall &pc, uint64_t most);
     void LaunchAttempt(ProbeCall &pc);
     void FinishProbe(ProbeCall &pc, std::deque<VectorBatch *> &out);
     // Pipelined callers: full chunks go to a worker thread that launches and finishes the probe

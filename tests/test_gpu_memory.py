@@ -209,3 +209,22 @@ def test_strings_of_a_join_are_built_over_two_rows_a_probe_row(gpu, device):
     want = _joined(bkey, pay, pkey)
     assert np.array_equal(keys, want[0]) and np.array_equal(vals, want[1])
     assert peak <= 2 * len(pkey) * (8 + 24) + 2 * MB
+
+
+@pytest.mark.parametrize("kind", [omg.OMNI_JOIN_TYPE_INNER, omg.OMNI_JOIN_TYPE_LEFT])
+@pytest.mark.parametrize("device,limit", [(True, 0), (True, 12 * MB), (False, 0)])
+def test_joins_that_come_to_less_than_the_mean(gpu, device, limit, kind):
+    """The output holds about what it needs, not 56 rows a probe row (44 MB), which the probe can do without, too."""
+    bkey, pay, pkey = _few_hits(False)
+    keys, vals, held, _, ctr, pinned = _join(bkey, pay, I, pkey, device=device, limit=limit, kind=kind)
+    want = _joined(bkey, pay, pkey)
+    if kind == omg.OMNI_JOIN_TYPE_LEFT:
+        miss = pkey[pkey >= 5000 * 1_000_003]
+        want = np.concatenate([want[0], miss]), np.concatenate([want[1], np.zeros(len(miss), np.int32)])
+        order = np.lexsort([want[1], want[0]])
+        want = want[0][order], want[1][order]
+    assert np.array_equal(keys, want[0])
+    hits = keys < 2000 * 1_000_003
+    assert np.array_equal(vals[hits], want[1][hits])
+    assert ctr["resizes"] == 0
+    assert (held if device else pinned) <= 2 * len(pkey) * 13 + 2 * MB
