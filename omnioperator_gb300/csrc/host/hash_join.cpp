@@ -1394,7 +1394,9 @@ std::unique_ptr<LookupJoinOperator::ProbeCall> LookupJoinOperator::LaunchBatches
     // Unique build keys and <= 8 bytes of NULL-free build output per row: fetch the build
     // values with the table entry from a per-slot packed copy (built once per factory).
     {
-        bool eligible = (b.table.unique || b.csrCount > 0) && nOut > nProbeOut && b.kind != omg::JOIN_KIND_EXISTENCE && !b.multiKey;
+        // (With duplicates and a filter the probe gathers by row: no kernel reads a payload there.)
+        bool eligible = (b.table.unique || (b.csrCount > 0 && p.nFilter == 0)) && nOut > nProbeOut &&
+            b.kind != omg::JOIN_KIND_EXISTENCE && !b.multiKey;
         int shift = 0;
         for (size_t o = nProbeOut; o < nOut && eligible; ++o) {
             const int w = p.out[o].width;
@@ -1404,11 +1406,21 @@ std::unique_ptr<LookupJoinOperator::ProbeCall> LookupJoinOperator::LaunchBatches
         }
         std::lock_guard<std::mutex> g(f_.payloadMu);
         if (eligible && !f_.payloadDecided && !b.table.unique) {
-            f_.slotPayload = omg::Buffer::NewDevice(static_cast<size_t>(b.csrCount) * sizeof(uint64_t), s, false);
-            CudaCheck(omg::LaunchBuildCsrPayload(p, b.csrCount, static_cast<uint64_t *>(f_.slotPayload->Data()), s),
-                "build CSR payload");
-            impl_->stream.Sync();
-            f_.payloadDecided = true;
+            omg::BufferPtr payload;
+            try {
+                payload = omg::Buffer::NewDevice(static_cast<size_t>(b.csrCount) * sizeof(uint64_t), s, false);
+            } catch (const OmniException &e) {
+                if (e.GetCode() != "MEM_CAP_EXCEEDED") {
+                    throw;
+                }
+            }
+            if (payload) {  // else the rows are gathered
+                CudaCheck(omg::LaunchBuildCsrPayload(p, b.csrCount, static_cast<uint64_t *>(payload->Data()), s),
+                    "build CSR payload");
+                impl_->stream.Sync();
+                f_.slotPayload = payload;
+                f_.payloadDecided = true;
+            }
         } else if (eligible && !f_.payloadDecided) {
             const uint64_t nSlots = b.table.mode == omg::JOIN_ARRAY ? b.table.range : b.table.capacity;
             f_.slotPayload = omg::Buffer::NewDevice((nSlots + 1) * sizeof(uint64_t), s, false);

@@ -228,3 +228,19 @@ def test_joins_that_come_to_less_than_the_mean(gpu, device, limit, kind):
     assert np.array_equal(vals[hits], want[1][hits])
     assert ctr["resizes"] == 0
     assert (held if device else pinned) <= 2 * len(pkey) * 13 + 2 * MB
+
+
+@pytest.mark.parametrize("filtered,limit", [(True, 0), (False, 2 * MB)])
+def test_payload_of_duplicates_only_where_it_is_read_and_fits(gpu, filtered, limit):
+    """The build side's payload in key order, 3.2 MB here: not for a join with a filter, whose kernel does not read it,
+    and not a reason for a probe to fail."""
+    bkey = np.repeat(np.arange(200_000), 2) * 1_000_003
+    pay = np.arange(len(bkey), dtype=np.int32) - 200_000
+    pkey = np.random.default_rng(5).integers(0, 250_000, 4096) * 1_000_003
+    filt = omg.Binary(omg.EXPR_GTE, omg.Field(2, I), omg.Literal(0, I)) if filtered else None
+    keys, vals, held, *_ = _join(bkey, pay, I, pkey, filt=filt, limit=limit)
+    want = _joined(bkey, pay, pkey)
+    if filtered:
+        want = want[0][want[1] >= 0], want[1][want[1] >= 0]
+    assert np.array_equal(keys, want[0]) and np.array_equal(vals, want[1])
+    assert held <= MB
