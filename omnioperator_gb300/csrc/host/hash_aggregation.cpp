@@ -831,6 +831,10 @@ constexpr size_t kExtractStats = 8;  // first of the extraction's words
 // Output columns of up to this many bytes for a host caller are written straight to pinned host memory
 // by the extraction, without a copy behind it.
 constexpr size_t kHostDirectBytes = size_t(4) << 20;
+// Output blocks of more than this that are more than kTrimTimes too large are copied to one of their size.  (A table
+// sized by a good estimate has room for up to four times its groups.)
+constexpr size_t kTrimBytes = size_t(256) << 10;
+constexpr size_t kTrimTimes = 5;
 // Tables of up to this many slots are extracted without waiting for the group count.
 constexpr uint64_t kAheadSlots = uint64_t(1) << 16;
 }  // namespace
@@ -2143,16 +2147,19 @@ bool HashAggregationOperator::ExtractSpilled()
     return true;
 }
 
+namespace {
+size_t Up256(size_t n) { return (n + 255) / 256 * 256; }
+}  // namespace
+
 // Output columns for up to `bound` groups, in one block, and what an extraction needs to know of them.
 void HashAggregationOperator::AllocOutputs(ExtractRun &x, uint64_t bound, cudaStream_t s)
 {
     const size_t nOut = plan_.outs.size();
     x.cols.assign(nOut, omg::OutColumn{});
-    auto up = [](size_t n) { return (n + 255) / 256 * 256; };
-    const size_t nullBytes = up(omg::NullBitmapBytes(static_cast<int64_t>(bound)));
+    const size_t nullBytes = Up256(omg::NullBitmapBytes(static_cast<int64_t>(bound)));
     size_t values = 0;
     for (const OutSpec &os : plan_.outs) {
-        values += up(bound * os.outWidth + 16);
+        values += Up256(bound * os.outWidth + 16);
     }
     const size_t bytes = values + nOut * nullBytes;
     x.onHost = !deviceOutput_ && plan_.dictInputs.empty() && bytes <= kHostDirectBytes;
@@ -2165,7 +2172,7 @@ void HashAggregationOperator::AllocOutputs(ExtractRun &x, uint64_t bound, cudaSt
         x.cols[o].values = omg::Buffer::Slice(block, at, bound * os.outWidth + 16);
         x.cols[o].nulls = omg::Buffer::Slice(block, values + o * nullBytes, nullBytes);
         x.cols[o].hasNull = os.kind != omg::OUT_COUNT && os.kind != omg::OUT_IS_EMPTY;
-        at += up(bound * os.outWidth + 16);
+        at += Up256(bound * os.outWidth + 16);
     }
     for (size_t o = 0; o < nOut && o < plan_.outContainer.size(); ++o) {
         // A container's fields (a partial AVG's sum and count) are never NULL.
@@ -2301,6 +2308,45 @@ bool HashAggregationOperator::ExtractSmall()
     return true;
 }
 
+// The first `rows` rows of the output columns in a block of their size, where the one that was allocated before their
+// number was known is much larger: the output batches hold it for as long as any of them lives.
+void HashAggregationOperator::TrimOutputs(ExtractRun &x, int64_t rows, cudaStream_t s)
+{
+    if (!x.onHost && !deviceOutput_) {
+        return;  // copied to the host anyway
+    }
+    const size_t nullBytes = Up256(omg::NullBitmapBytes(rows));
+    size_t held = 0;
+    size_t need = 0;
+    for (const omg::OutColumn &c : x.cols) {
+        held += c.values->Bytes() + c.nulls->Bytes();
+        need += Up256(static_cast<size_t>(rows) * c.width + 16) + nullBytes;
+    }
+    if (held <= kTrimBytes || held <= kTrimTimes * need) {
+        return;
+    }
+    omg::BufferPtr block = x.onHost ? omg::Buffer::NewHost(need, false) : omg::Buffer::NewDevice(need, s, false);
+    size_t at = 0;
+    auto move = [&](omg::BufferPtr &buf, size_t bytes, size_t room) {
+        omg::BufferPtr to = omg::Buffer::Slice(block, at, room);
+        if (x.onHost) {
+            std::memcpy(to->Data(), buf->Data(), bytes);
+        } else {
+            CudaCheck(cudaMemcpyAsync(to->Data(), buf->Data(), bytes, cudaMemcpyDeviceToDevice, s), "trim output");
+        }
+        buf = to;
+        at += Up256(room);
+    };
+    for (omg::OutColumn &c : x.cols) {
+        const size_t bytes = static_cast<size_t>(rows) * c.width;
+        move(c.values, bytes, bytes + 16);
+        move(c.nulls, std::min(nullBytes, c.nulls->Bytes()), nullBytes);
+    }
+    if (!x.onHost) {
+        impl_->stream.Sync();  // readable on every stream, as it was
+    }
+}
+
 // The first `rows` rows of the output columns as the operator's output batches.
 void HashAggregationOperator::EmitOutputs(ExtractRun &x, int64_t rows, cudaStream_t s)
 {
@@ -2308,8 +2354,10 @@ void HashAggregationOperator::EmitOutputs(ExtractRun &x, int64_t rows, cudaStrea
     uniqueKeys_ = static_cast<uint64_t>(rows);
     counters_[3] = rows;
     if (rows == 0) {
+        x.cols.clear();
         return;
     }
+    TrimOutputs(x, rows, s);
     if (!plan_.dictInputs.empty()) {
         DecodeStrings(x.cols, rows, s);
     }

@@ -162,6 +162,7 @@ private:
     void AllocOutputs(ExtractRun &x, uint64_t bound, cudaStream_t s);
     void LaunchExtract(ExtractRun &x, uint64_t bound, cudaStream_t s);
     bool ExtractSmall();
+    void TrimOutputs(ExtractRun &x, int64_t rows, cudaStream_t s);
     void EmitOutputs(ExtractRun &x, int64_t rows, cudaStream_t s);
     void RunExtract(ExtractRun &x, cudaStream_t s);
     void EncodeStrings(omg::BatchTable &bt, cudaStream_t s);

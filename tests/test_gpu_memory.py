@@ -244,3 +244,37 @@ def test_payload_of_duplicates_only_where_it_is_read_and_fits(gpu, filtered, lim
         want = want[0][want[1] >= 0], want[1][want[1] >= 0]
     assert np.array_equal(keys, want[0]) and np.array_equal(vals, want[1])
     assert held <= MB
+
+
+@pytest.mark.parametrize("device", [False, True])
+@pytest.mark.parametrize("rows", [5_000, 40_000, 300_000])
+def test_aggregation_results_hold_about_their_rows(gpu, rows, device):
+    """100 groups, for which up to a row per input row was reserved: 2 MB for 40,000 rows."""
+    rng = np.random.default_rng(6)
+    key = rng.integers(0, 100, rows)
+    v, d = rng.integers(-100, 100, rows), rng.integers(-100, 100, rows).astype(np.float64)
+    nulls = [None, rng.random(rows) < 0.5, (key % 3 == 0)]
+    fac = omg.HashAggregationOperatorFactory([0], [L], [[1], [1], [2], []], [[L], [L], [D], []], [[L], [L], [D], [L]],
+                                             [SUM, CNT, SUM, CALL])
+    before = memory()
+    op = fac.create_operator()
+    try:
+        op.set_device_output(device)
+        op.add_input(omg.make_batch([L, L, D], [key, v, d], nulls))
+        outs = op.drain()
+    finally:
+        op.delete()
+        fac.close()
+    held = memory()
+    parts = [omg.batch_to_numpy(omg.batch_to_host(b) if device else b) for b in outs]
+    omg.free_batches(outs)
+    cols = [(np.concatenate([p[c][0] for p in parts]), np.concatenate([p[c][1] for p in parts])) for c in range(5)]
+    order = np.argsort(cols[0][0])
+    assert np.array_equal(cols[0][0][order], np.arange(100))
+    assert np.array_equal(cols[1][0][order], np.bincount(key, weights=np.where(nulls[1], 0, v), minlength=100))
+    assert np.array_equal(cols[2][0][order], np.bincount(key[~nulls[1]], minlength=100))
+    assert np.array_equal(cols[3][1][order], np.arange(100) % 3 == 0)
+    live = np.arange(100) % 3 != 0
+    assert np.array_equal(cols[3][0][order][live], np.bincount(key, weights=d, minlength=100)[live])
+    assert np.array_equal(cols[4][0][order], np.bincount(key, minlength=100))
+    assert (held[0] if device else held[2]) - (before[0] if device else before[2]) <= 320 << 10
