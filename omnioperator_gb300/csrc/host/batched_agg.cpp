@@ -59,7 +59,8 @@ int Log2Bucket(uint64_t v)
     return b;
 }
 
-// Tuned launch shape per (slot words, key kind, accumulators, log2 rows, log2 tasks).
+// Tuned launch shape per (slot words, key kind, accumulators, log2 rows, log2 tasks): the rows and tasks that go to their
+// own tables at once, which are what the launch is for.
 using TuneKey = std::tuple<int, int, int, int, int>;
 std::mutex g_tuneMu;
 std::map<TuneKey, int32_t> *g_tuned = new std::map<TuneKey, int32_t>();  // process lifetime
@@ -110,7 +111,8 @@ struct BatchedAggregation::Impl {
     DevArray<uint8_t> shared;
     DevArray<unsigned int> nextUnit;
     int32_t nUnits = 0;
-    bool anyGlobal = true;  // tasks whose rows go to their own tables at once
+    int32_t globalTasks = 0;  // tasks whose rows go to their own tables at once, and their rows
+    int64_t globalRows = 0;
     DevArray<unsigned long long> cursor;
     DevArray<int64_t> blockSums;
     DevArray<long long> total;
@@ -172,7 +174,7 @@ struct BatchedAggregation::Impl {
         CudaCheck(cudaMemsetAsync(specials.Get(), 0, sizeof(uint32_t) * 2 * n, s), "reset special slots");
         CudaCheck(cudaMemsetAsync(failed.Get(), 0, sizeof(uint32_t) * n, s), "reset task flags");
         CudaCheck(omg::LaunchAggInitTable(p, s), "init task tables");
-        if (anyGlobal) {
+        if (globalTasks > 0) {
             CudaCheck(omg::LaunchAggTasks(p, variant, s), "batched aggregation");
         }
         CudaCheck(omg::LaunchAggTaskUnits(p, units.Get(), nUnits, nextUnit.Get(), s), "batched aggregation by units");
@@ -314,7 +316,8 @@ struct BatchedAggregation::Impl {
         const uint64_t minGroups = std::any_of(plan.accs.begin(), plan.accs.end(),
             [](const omg::AccSpec &a) { return a.kind == omg::ACC_DSUM; }) ? 256 : 0;
         const int32_t minTiles = std::min(kUnitMinTiles, bt.NumTiles() / (2 * omg::DeviceSMCount()) + 1);
-        anyGlobal = false;
+        globalTasks = 0;
+        globalRows = 0;
         int32_t tile = 0;
         for (int32_t t = 0; t < n; ++t) {
             const int32_t tiles = static_cast<int32_t>((tasks[t]->GetRowCount() + omg::kTileRows - 1) / omg::kTileRows);
@@ -336,7 +339,10 @@ struct BatchedAggregation::Impl {
                     }
                 }
             }
-            anyGlobal = anyGlobal || hostShared[t] == 0;
+            if (hostShared[t] == 0) {
+                ++globalTasks;
+                globalRows += tasks[t]->GetRowCount();
+            }
             tile += tiles;
         }
         nUnits = static_cast<int32_t>(hostUnits.size());
@@ -387,8 +393,12 @@ struct BatchedAggregation::Impl {
     // and keep the fastest; cached per plan shape and workload size.
     void Tune(cudaStream_t s)
     {
+        if (globalTasks == 0) {
+            variant = kDefaultVariant;  // the kernel has nothing to do, so there is nothing to time
+            return;
+        }
         const TuneKey key{plan.slotWords, plan.key.kind, static_cast<int>(plan.accs.size()),
-            Log2Bucket(static_cast<uint64_t>(std::max<int64_t>(rows, 1))), Log2Bucket(static_cast<uint64_t>(n))};
+            Log2Bucket(static_cast<uint64_t>(globalRows)), Log2Bucket(static_cast<uint64_t>(globalTasks))};
         {
             std::lock_guard<std::mutex> g(g_tuneMu);
             auto it = g_tuned->find(key);

@@ -186,3 +186,35 @@ def test_batched_units_of_two_column_keys(gpu, groups):
         assert np.array_equal(~null[order], count > 0)
         assert np.array_equal(cols[2][order][count > 0], want[count > 0])
         assert np.array_equal(cols[3][order], count)
+
+
+def test_tuning_times_the_tasks_that_the_launch_is_for(gpu):
+    """Tasks that go by units leave the launch nothing to time, and what was found for one number of rows in the tasks'
+    own tables is not taken for another."""
+    rng = np.random.default_rng(41)
+    # Seven sums of one column of its own each: a plan shape that no other test tunes.
+    fac = omg.HashAggregationOperatorFactory([0], [L], [[c] for c in range(1, 8)], [[L]] * 7, [[L]] * 7,
+                                             [omg.OMNI_AGGREGATION_TYPE_SUM] * 7)
+
+    def tuned(groups):
+        tasks = []
+        for g in groups:
+            key = rng.integers(0, g, 60_000)
+            tasks.append(omg.make_batch([L] * 8, [key] + [key * k for k in range(1, 8)]))
+        batch = omg.AggBatch(fac, tasks)
+        batch.run()
+        for t, b in batch.outputs():
+            cols = omg.batch_to_numpy(b)
+            omg.free_batch(b)
+            n = cols[1][0] // np.where(cols[0][0] == 0, 1, cols[0][0])  # rows of the group
+            assert np.array_equal(cols[7][0], 7 * n * cols[0][0])
+        us = batch.info()["tune_us"]
+        batch.close()
+        omg.free_batches(tasks)
+        return us
+
+    assert tuned([10] * 16) == 0
+    assert tuned([50_000] * 16) > 0
+    assert tuned([50_000] + [10] * 15) > 0
+    assert tuned([50_000] * 15 + [10]) == 0  # as sixteen, to a power of two
+    fac.close()
