@@ -1306,20 +1306,26 @@ bool HashAggregationOperator::RadixWanted(int64_t rows) const
 // Whether the rows of a first flush, whose groups fit the partitions, are better sorted by step than added to
 // the partitions' tables row by row.
 // A double sum there is a compare-and-swap loop, and a CTA takes the rows of one group one after the other, at
-// some 0.35 us; the radix passes cost about 0.1 ms and 50 ps a row more.  4M rows in 10,000 groups, six
-// aggregates: the hottest key with a tenth of the rows 12.3 ms against 0.65, uniform 0.40 against 0.62;
-// 300,000 rows in 1,000 groups, Zipf, 0.34 against 0.33.
-// Two-column keys take the tables longer the more groups they hold: with a double sum the line is at 900
-// groups and 2^21 rows (at 2^22 rows 700 groups 0.56 ms against 0.77, 1,000 groups 0.94 against 0.73, 10,000
-// groups 1.41 against 0.77; at 2^20 rows 1,000 groups 0.39 against 0.45), and without one at 2^22 rows in
-// several partitions (10,000 groups 0.70 against 0.58, 1,000 in one partition 0.44 against 0.57).
+// some 0.35 us; the radix passes cost about 0.1 ms and 50 ps a row more.  2^22 rows in 10,000 groups, six
+// aggregates: the hottest key with a tenth of the rows 5.7 ms against 0.57, uniform 0.34 against 0.53;
+// 2^19 rows in 1,000 groups, a tenth one key's, 0.25 against 0.28.
+// Two-column keys take the tables longer the fuller they are: with a double sum the line is at 2^21 rows and
+// 900 groups that fill 0.38 of a CTA's table (wider states were not measured below 900).  Six aggregates (0.38: 884
+// groups), at 2^22 rows 700 groups 0.60 ms
+// against 0.68, 900 groups 0.76 against 0.63, 10,000 groups 1.37 against 0.69; at 2^20 rows 1,000 groups 0.32
+// against 0.35.  One sum and a count (0.38: 1,390 groups), at 2^21, 2^22 and 2^24 rows: 1,000 groups 0.26, 0.37 and
+// 1.26 against 0.42, 0.58 and 1.71, 1,500 groups 0.34, 0.52 and 1.79 against 0.41, 0.56 and 1.63, 3,000 groups 0.44,
+// 0.71 and 2.45 against 0.42, 0.57 and 1.62.  Without a double sum it is at 2^22 rows in
+// several partitions (10,000 groups 0.66 against 0.49, 1,000 in one partition 0.33 against 0.50).
 bool HashAggregationOperator::RadixBeatsPartitions(int64_t rows) const
 {
     const Impl &im = *impl_;
     const bool doubles = std::any_of(plan_.accs.begin(), plan_.accs.end(),
         [](const AccSpec &a) { return a.kind == omg::ACC_DSUM; });
+    const double load = static_cast<double>(im.estimate) / omg::AggPartSmemSlots(plan_.smemStride);
     if (plan_.key.kind == omg::KEY_PACKED &&
-        (doubles ? im.estimate >= 900 && rows >= (int64_t(1) << 21) : im.partBits > 0 && rows >= (int64_t(1) << 22))) {
+        (doubles ? im.estimate >= 900 && load >= 0.38 && rows >= (int64_t(1) << 21)
+                 : im.partBits > 0 && rows >= (int64_t(1) << 22))) {
         return true;
     }
     if (!doubles || im.sketch[0] == 0) {

@@ -162,7 +162,8 @@ def test_several_passes_over_a_partition(gpu):
 
 @pytest.mark.parametrize("keys,groups,rows,share,kernel", [
     (1, 500, 400_003, 0.02, PARTITIONS), (1, 500, 400_003, 0.95, RADIX),
-    (2, 2000, (1 << 21) - 1, 0.0, PARTITIONS), (2, 2000, 1 << 21, 0.0, RADIX), (2, 300, 1 << 21, 0.0, PARTITIONS)])
+    (2, 2000, (1 << 21) - 1, 0.0, PARTITIONS), (2, 2000, 1 << 21, 0.0, RADIX), (2, 300, 1 << 21, 0.0, PARTITIONS),
+    (2, 1000, 1 << 21, 0.0, PARTITIONS)])  # (0.27 of a table's 3,657 slots; 2,000 groups 0.55)
 def test_groups_that_fit_the_partitions(gpu, keys, groups, rows, share, kernel):
     """With sums of doubles the radix passes take hot groups, and wide keys of many rows and groups."""
     rng = np.random.default_rng(rows + groups)
