@@ -484,7 +484,9 @@ int32_t omg_op_set_agg_sizing(void *op, int32_t mode);
 int32_t omg_op_set_spill(void *op, int32_t enabled, int64_t device_budget_bytes);
 /* Operator::GetSpilledBytes (core/src/operator/operator.h:66): bytes moved to host memory. */
 int64_t omg_op_spilled_bytes(void *op);
-/* Counters of the last run: [0]=kernel launches, [1]=table resizes, [2]=retried rows,
+/* Counters of the last run: [0]=kernel launches, [1]=table resizes (the radix passes build no
+ * table by the estimate: for them also 1 where the key pass finds more groups than the table
+ * would have had room for) or probes run a second time, [2]=retried rows,
  * [3]=groups, [4]=ordered-fallback groups, [5]=output rows, [6]=kernel ns, [7]=timed kernel
  * launches; LookupJoin host time: [8]=ns setting up and launching probe calls, [9]=ns waiting
  * for their kernels, [10]=ns carving output batches, [11]=ns freeing probe input batches. */

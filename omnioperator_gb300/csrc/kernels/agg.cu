@@ -515,8 +515,9 @@ __device__ __forceinline__ int PartOf(uint64_t hash, int partBits)
 
 // ------------------------------------------------------------------ batched tasks
 // Many independent aggregations (tasks) in one launch: task i is batch i and owns table
-// taskTables[i] inside one slab.  AggTasksKernel walks the tiles of all tasks (tiles of a task are
-// adjacent); per-task sketch, count and extraction kernels run one CTA per task.
+// taskTables[i] inside one slab.  AggTaskUnitsKernel adds up the tasks with few groups in shared tables, by units
+// of their tiles; AggTasksKernel walks the tiles of the others (tiles of a task are adjacent).  The sketch runs one
+// CTA per task, the count and the extraction one per kTaskChunkSlots slots of the tables.
 
 // Rows per thread per step: their loads and first probes are issued together.
 constexpr int kTaskRows = 1;

@@ -353,13 +353,15 @@ __device__ __forceinline__ void AtomicStrMinMax(const AggLaunch &p, int input, u
     }
 }
 
-// Double sums: the first kPlainSumRows rows of a table slot (by their COUNT_ALL arrival order)
-// are added with a plain atomic add, the later ones with the compensated add.  A slot of a
-// shared table or of the global table therefore leaves at most kPlainSumRows additions
+// Double sums that are added to row by row: the first kPlainSumRows rows of a slot of the global table,
+// of a shared table in front of it or of a partition's shared table (by their COUNT_ALL arrival order)
+// are added with a plain atomic add, the later ones with the compensated add.  Such a slot
+// therefore leaves at most kPlainSumRows additions
 // uncompensated, whose rounding errors add up to at most kPlainSumRows * 2^-53 * sum|x| (the
 // slots of one group hold disjoint rows, so the bound holds for the group too): 7.1e-15 of
 // sum|x| for 64.  Shared-table partials are merged compensated.  (2048 plain rows, 2.3e-13,
-// measured no faster on the uniform workload: 190.7 us against 182-192 us.)
+// measured no faster on the uniform workload: 190.7 us against 182-192 us.)  The states per thread, the
+// steps (small calls, radix passes) and the batched tasks' units compensate every addition.
 constexpr unsigned long long kPlainSumRows = 64;
 
 __device__ __forceinline__ void AddDoubleState(uint64_t *w, double x, unsigned long long arrival)

@@ -126,7 +126,8 @@ __global__ void __launch_bounds__(kKeyThreads, 2) RadixKeyKernel(const __grid_co
 // stores each, 1.75 ms as one of 32 bytes), so records of three or more words are padded to 32 bytes and
 // stored 32 bytes at a time; columns apart would take a request each.  Every pass over rows loads several
 // rows' values before it uses any, and what must outlive a pass is in shared memory: a register spill is a
-// store request too.  Wide records are bound by latency before that: 32 warps of 64 registers with three
+// store request too (packed keys spill 24 bytes a thread at 64 registers, and none at the 128 that were
+// slower).  Wide records are bound by latency before that: 32 warps of 64 registers with three
 // sources in flight instead of 16 of 128 with six took 2^26 records of a two-column key from 3.10 to 2.35 ms
 // (two sources 2.69; 2^24 of 16 bytes 0.44 -> 0.36; steps of eight tiles 2.42 and 0.41).
 constexpr int kScatterThreads = 1024;

@@ -240,7 +240,9 @@ __device__ __forceinline__ void AddDouble(uint64_t *w, const Sum &v, bool shared
 
 // The sum over the warp's threads, in thread 0.  Each value is cut at a bit that is the same for all of them, so far
 // below 2^8 times their largest power of two that the upper parts, 46 bits each, add up without rounding, and the
-// lower parts' roundings are of second order: 14 FP64 operations where five times AddTo and an error takes 25.
+// lower parts' roundings are of second order: 14 FP64 operations where five times AddTo and an error takes 25
+// (2^26 rows of a skewed two-column key, decimal sum, count and average: 9.60 -> 9.18 ms; 8.54 to 8.77 with plain
+// sums in the runs).
 __device__ __forceinline__ void SumWarp(Sum &v)
 {
     const unsigned int most =
