@@ -172,7 +172,14 @@ __global__ void BuildCountKernel(JoinTable t, const void *keys, const uint8_t *n
     uint64_t *hashSlots, uint32_t *counts, uint32_t *sentinelCount, unsigned int *maxCount, unsigned int *distinct,
     int32_t *error)
 {
-    uint32_t most = 0;   // the largest count this thread saw: one atomic per warp, not one per duplicate
+    __shared__ uint32_t blockMost;
+    __shared__ uint32_t blockFresh;
+    if (threadIdx.x == 0) {
+        blockMost = 0;
+        blockFresh = 0;
+    }
+    __syncthreads();
+    uint32_t most = 0;   // the largest count this thread saw: one atomic per block, not one per duplicate
     uint32_t fresh = 0;  // keys that this thread saw first
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -198,11 +205,16 @@ __global__ void BuildCountKernel(JoinTable t, const void *keys, const uint8_t *n
     }
     most = __reduce_max_sync(0xffffffffu, most);
     fresh = __reduce_add_sync(0xffffffffu, fresh);
-    if ((threadIdx.x & 31) == 0 && fresh != 0) {
-        atomicAdd(distinct, fresh);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&blockMost, most);
+        atomicAdd(&blockFresh, fresh);
     }
-    if ((threadIdx.x & 31) == 0 && most > 1) {
-        atomicMax(maxCount, most);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (blockMost > 1) {
+            atomicMax(maxCount, blockMost);
+        }
+        atomicAdd(distinct, blockFresh);
     }
 }
 
