@@ -1658,8 +1658,7 @@ void HashAggregationOperator::AggregateRows(omg::BatchTable &bt, bool last, bool
         for (size_t i = 0; i < plan_.inputCols.size(); ++i) {
             nullable |= bt.AnyNulls(static_cast<int32_t>(i)) ? 1u << i : 0u;
         }
-        few = omg::LayoutAggFew(MakeLaunch(plan_, nullptr, 0, nullptr, nullptr), nullable, &fewLayout) &&
-            im.estimate + 2 <= static_cast<uint64_t>(fewLayout.maxGroups + fewLayout.firstSlot);
+        few = omg::LayoutAggFew(MakeLaunch(plan_, nullptr, 0, nullptr, nullptr), nullable, im.estimate + 2, &fewLayout);
     }
     RadixRun radixRun;
     radix = radix && !few && PlanRadix(bt, radixRun, s);

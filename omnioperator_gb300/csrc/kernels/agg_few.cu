@@ -2,12 +2,13 @@
 //
 // With few groups the shared tables' atomics are all on the same words: 2^22 rows of 6 groups, two INT keys
 // and six aggregates ran 1.22 ms, and 0.18 ms here (507 instructions a warp's row, a third of them the packed
-// key, at 0.33 of the issue slots and 0.39 of the FP64 pipe: latency at 16 warps an SM; 0.144 ms and 480
-// without the errors of the double sums).  Here every thread keeps states of its own for every group, in planes of shared
+// key, at 0.33 of the issue slots and 0.39 of the FP64 pipe; 0.144 ms and 480 without the errors of the double
+// sums, three FP64 operations a row; their chains side by side for a step's rows measured no faster).  Here every thread keeps states of its own for every group, in planes of shared
 // memory where the threads of a warp are side by side: no atomics and no bank conflicts.  A sum of doubles has a
 // plane for the rounding errors of its additions.  Exact sums move to the CTA's state of the group every 64
 // rows (magnitudes of up to 64 values below 2^57), and at the end a warp adds up each group's private states
 // and the CTA's records are merged into the global table.
+#include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -24,9 +25,9 @@ constexpr size_t kFewSmemBytes = 110 * 1024;  // two CTAs per SM
 constexpr unsigned int kFoldRows = 64;
 constexpr int kFewIndex = 256;
 
-template <class T> __device__ __forceinline__ T *Plane(unsigned char *smem, int off, int group)
+template <class T, int kThreads> __device__ __forceinline__ T *Plane(unsigned char *smem, int off, int group)
 {
-    return reinterpret_cast<T *>(smem + off) + group * kFewThreads + threadIdx.x;
+    return reinterpret_cast<T *>(smem + off) + group * kThreads + threadIdx.x;
 }
 
 __device__ __forceinline__ void AddTwoSum(double &s, double &c, double x)
@@ -44,7 +45,8 @@ struct FewInput {
     uint32_t null;
 };
 
-__device__ __forceinline__ void LoadFew(const BatchRows<kFewThreads> &rows, int input, int width, uint32_t live,
+template <int kThreads>
+__device__ __forceinline__ void LoadFew(const BatchRows<kThreads> &rows, int input, int width, uint32_t live,
     FewInput &in)
 {
     in.null = 0;
@@ -171,6 +173,7 @@ __device__ __forceinline__ void ApplyFew(const AggLaunch &p, const FewLayout &l,
 }
 
 // Add up the private states of group `group` (by one warp) into the CTA's slot.
+template <int kThreads>
 __device__ __forceinline__ void FoldGroup(const AggLaunch &p, const FewLayout &l, unsigned char *smem, int group,
     uint64_t *state)
 {
@@ -182,12 +185,12 @@ __device__ __forceinline__ void FoldGroup(const AggLaunch &p, const FewLayout &l
             continue;
         }
         uint64_t *w = state + s.word;
-        const unsigned int *n32 = reinterpret_cast<const unsigned int *>(smem + off) + group * kFewThreads;
-        const uint64_t *n64 = reinterpret_cast<const uint64_t *>(smem + off) + group * kFewThreads;
+        const unsigned int *n32 = reinterpret_cast<const unsigned int *>(smem + off) + group * kThreads;
+        const uint64_t *n64 = reinterpret_cast<const uint64_t *>(smem + off) + group * kThreads;
         if (s.kind == ACC_DSUM) {
             const uint64_t *e64 = n64 + l.planeStep[a] / 8;
             double sum = 0.0, err = 0.0;
-            for (int t = lane; t < kFewThreads; t += 32) {
+            for (int t = lane; t < kThreads; t += 32) {
                 AddTwoSum(sum, err, __longlong_as_double(static_cast<long long>(n64[t])));
                 err = __dadd_rn(err, __longlong_as_double(static_cast<long long>(e64[t])));
             }
@@ -209,7 +212,7 @@ __device__ __forceinline__ void FoldGroup(const AggLaunch &p, const FewLayout &l
         if (s.kind == ACC_IMIN || s.kind == ACC_IMAX || s.kind == ACC_DMIN || s.kind == ACC_DMAX) {
             const bool isMin = s.kind == ACC_IMIN || s.kind == ACC_DMIN;
             long long x = static_cast<long long>(s.init);
-            for (int t = lane; t < kFewThreads; t += 32) {
+            for (int t = lane; t < kThreads; t += 32) {
                 const long long v = static_cast<long long>(n64[t]);
                 x = isMin ? min(x, v) : max(x, v);
             }
@@ -226,7 +229,7 @@ __device__ __forceinline__ void FoldGroup(const AggLaunch &p, const FewLayout &l
         for (int side = 0; side < planes; ++side) {
             const uint64_t *n = n64 + side * (l.planeStep[a] / 8);
             unsigned long long lo = 0, hi = 0;  // chunk sums of the magnitudes, or the plain sum in lo
-            for (int t = lane; t < kFewThreads; t += 32) {
+            for (int t = lane; t < kThreads; t += 32) {
                 if (s.kind == ACC_WSUM2) {
                     lo += n[t] & 0xffffffffull;
                     hi += n[t] >> 32;
@@ -248,8 +251,8 @@ __device__ __forceinline__ void FoldGroup(const AggLaunch &p, const FewLayout &l
     }
 }
 
-template <int kKind>
-__global__ void __launch_bounds__(kFewThreads, 2) AggFewKernel(const __grid_constant__ AggLaunch p,
+template <int kKind, int kThreads>
+__global__ void __launch_bounds__(kThreads, 2) AggFewKernel(const __grid_constant__ AggLaunch p,
     const __grid_constant__ FewLayout l, const __grid_constant__ SpillArgs sp)
 {
     // The private planes (from byte 0), then the CTA's slots and their index.
@@ -263,10 +266,10 @@ __global__ void __launch_bounds__(kFewThreads, 2) AggFewKernel(const __grid_cons
     const int nAll = nSlots + kSpecialSlots;
     uint64_t *slots = reinterpret_cast<uint64_t *>(smem8 + l.smemBytes) - static_cast<int64_t>(nAll) * sw;
     uint64_t *st = slots + l.firstSlot * sw + kw;
-    for (int i = threadIdx.x; i < nAll; i += kFewThreads) {
+    for (int i = threadIdx.x; i < nAll; i += kThreads) {
         InitSlot(p, slots + static_cast<int64_t>(i) * sw);
     }
-    for (int i = threadIdx.x; i < kFewIndex; i += kFewThreads) {
+    for (int i = threadIdx.x; i < kFewIndex; i += kThreads) {
         index[i] = 0;
     }
     for (int a = 0; a < p.nAccs; ++a) {
@@ -276,12 +279,12 @@ __global__ void __launch_bounds__(kFewThreads, 2) AggFewKernel(const __grid_cons
         }
         for (int g = 0; g < l.maxGroups; ++g) {
             if (s.kind == ACC_COUNT_ALL || s.kind == ACC_NULLS) {
-                *Plane<unsigned int>(smem8, l.off[a], g) = 0;
+                *Plane<unsigned int, kThreads>(smem8, l.off[a], g) = 0;
             } else {
-                *Plane<uint64_t>(smem8, l.off[a], g) = s.kind == ACC_DSUM || s.kind == ACC_ISUM || s.kind == ACC_WSUM2
+                *Plane<uint64_t, kThreads>(smem8, l.off[a], g) = s.kind == ACC_DSUM || s.kind == ACC_ISUM || s.kind == ACC_WSUM2
                     ? 0ull : static_cast<uint64_t>(s.init);
                 if (s.kind == ACC_WSUM2 || s.kind == ACC_DSUM) {
-                    *Plane<uint64_t>(smem8, l.off[a] + l.planeStep[a], g) = 0;
+                    *Plane<uint64_t, kThreads>(smem8, l.off[a] + l.planeStep[a], g) = 0;
                 }
             }
         }
@@ -294,13 +297,13 @@ __global__ void __launch_bounds__(kFewThreads, 2) AggFewKernel(const __grid_cons
     for (int t = blockIdx.x; t < p.nTiles; t += gridDim.x) {
         const TileDesc tile = p.tiles[t];
         const BatchDesc &b = p.batches[tile.batch];
-        for (int r0 = threadIdx.x; r0 < tile.rows; r0 += kFewRows * kFewThreads) {
+        for (int r0 = threadIdx.x; r0 < tile.rows; r0 += kFewRows * kThreads) {
             uint32_t live = 0;
 #pragma unroll
             for (int k = 0; k < kFewRows; ++k) {
-                live |= r0 + k * kFewThreads < tile.rows ? 1u << k : 0u;
+                live |= r0 + k * kThreads < tile.rows ? 1u << k : 0u;
             }
-            const BatchRows<kFewThreads> rows{b, static_cast<int64_t>(tile.row0) + r0};
+            const BatchRows<kThreads> rows{b, static_cast<int64_t>(tile.row0) + r0};
             // The first input's values come with the keys, each later one's with the work on the one before.
             FewInput in;
             LoadFew(rows, l.nInputs > 0 ? l.input[0] : -1, l.nInputs > 0 ? l.width[0] : 0, live, in);
@@ -331,7 +334,7 @@ __global__ void __launch_bounds__(kFewThreads, 2) AggFewKernel(const __grid_cons
                     global |= slot == -1 ? 1u << k : 0u;
                     continue;
                 }
-                at[k] = (slot - l.firstSlot) * kFewThreads + threadIdx.x;
+                at[k] = (slot - l.firstSlot) * kThreads + threadIdx.x;
                 states[k] = st + (slot - l.firstSlot) * sw;
                 unsigned int *c = reinterpret_cast<unsigned int *>(smem8 + l.off[0]) + at[k];  // accs[0]: COUNT_ALL
                 const unsigned int n = *c + 1;
@@ -342,7 +345,7 @@ __global__ void __launch_bounds__(kFewThreads, 2) AggFewKernel(const __grid_cons
 #pragma unroll 1
                 for (int k = 0; k < kFewRows; ++k) {
                     if ((global >> k) & 1u) {
-                        const int64_t row = rows.row0 + k * kFewThreads;
+                        const int64_t row = rows.row0 + k * kThreads;
                         ProcessRow<kKind>(p, tile.batch, b, row, LoadRow<kKind>(p, b, row), nullptr, 0, &newGroups);
                     }
                 }
@@ -359,11 +362,11 @@ __global__ void __launch_bounds__(kFewThreads, 2) AggFewKernel(const __grid_cons
     }
     __syncthreads();
     const int nUsed = static_cast<int>(min(used, static_cast<unsigned int>(nSlots))) + kSpecialSlots;
-    for (int slot = l.firstSlot + (threadIdx.x >> 5); slot < nUsed; slot += kFewThreads / 32) {
-        FoldGroup(p, l, smem8, slot - l.firstSlot, slots + static_cast<int64_t>(slot) * sw + kw);
+    for (int slot = l.firstSlot + (threadIdx.x >> 5); slot < nUsed; slot += kThreads / 32) {
+        FoldGroup<kThreads>(p, l, smem8, slot - l.firstSlot, slots + static_cast<int64_t>(slot) * sw + kw);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < nUsed; i += kFewThreads) {
+    for (int i = threadIdx.x; i < nUsed; i += kThreads) {
         uint64_t *slot = slots + static_cast<int64_t>(i) * sw;
         if (i >= kSpecialSlots) {
             MergeRecord<kKind>(p, sp, slot, &newGroups);
@@ -380,9 +383,10 @@ __global__ void __launch_bounds__(kFewThreads, 2) AggFewKernel(const __grid_cons
 
 }  // namespace
 
-bool LayoutAggFew(const AggLaunch &p, uint32_t nullable, FewLayout *l)
+bool LayoutAggFew(const AggLaunch &p, uint32_t nullable, uint64_t slots, FewLayout *l)
 {
     int perGroup = 0;  // bytes of a thread's states of one group
+    int errors = 0;    // of them, for the errors of double sums
     int bytes[kMaxAccs];
     bool keyNullable = false;
     for (int c = 0; c < p.key.nCols; ++c) {
@@ -405,6 +409,9 @@ bool LayoutAggFew(const AggLaunch &p, uint32_t nullable, FewLayout *l)
                 bytes[a] = 8;
                 break;
             case ACC_DSUM:
+                errors += 8;
+                bytes[a] = 16;
+                break;
             case ACC_WSUM2:
                 bytes[a] = 16;
                 break;
@@ -416,13 +423,23 @@ bool LayoutAggFew(const AggLaunch &p, uint32_t nullable, FewLayout *l)
     l->firstSlot = keyNullable ? 0 : kSpecialSlots;
     const int slotBytes = p.table.slotWords * 8;
     const int room = static_cast<int>(kFewSmemBytes) - kSpecialSlots * slotBytes - 16;
-    l->maxGroups = room / (perGroup * kFewThreads + slotBytes);
-    if (l->maxGroups > kFewIndex / 2) {
-        l->maxGroups = kFewIndex / 2;
-    }
-    if (l->maxGroups - (kSpecialSlots - l->firstSlot) < 4) {
+    auto fits = [&](int threads, int bytesPerGroup) {
+        return std::min(room / (bytesPerGroup * threads + slotBytes), kFewIndex / 2);
+    };
+    // The line: as many groups as 256 threads have room for beside the errors of their double sums.  With the errors,
+    // the most of them takes fewer threads: 2^24 rows, two-column key, 12 groups of six aggregates (192 threads) 0.86 ms
+    // against 2.53 by the partitions' tables, 30 groups of one double sum (128 threads) 1.02 against 1.33; at 2^19
+    // rows 0.16 against 0.24 and 0.20 against 0.16.
+    const int most = fits(kFewMaxThreads, perGroup - errors);
+    if (most - (kSpecialSlots - l->firstSlot) < 4 || slots > static_cast<uint64_t>(most + l->firstSlot)) {
         return false;
     }
+    for (l->threads = kFewMaxThreads; l->threads > kFewMinThreads; l->threads -= 64) {
+        if (slots <= static_cast<uint64_t>(fits(l->threads, perGroup) + l->firstSlot)) {
+            break;
+        }
+    }
+    l->maxGroups = fits(l->threads, perGroup);
     // 8-byte planes first, then the counters; the slots end the block on an 8-byte boundary.
     int at = 0;
     for (int pass = 0; pass < 2; ++pass) {
@@ -433,8 +450,8 @@ bool LayoutAggFew(const AggLaunch &p, uint32_t nullable, FewLayout *l)
                 l->planeStep[a] = 0;
             } else if ((pass == 0) == (unit == 8)) {
                 l->off[a] = at;
-                l->planeStep[a] = unit * kFewThreads * l->maxGroups;
-                at += bytes[a] * kFewThreads * l->maxGroups;
+                l->planeStep[a] = unit * l->threads * l->maxGroups;
+                at += bytes[a] * l->threads * l->maxGroups;
             }
         }
     }
@@ -471,13 +488,16 @@ cudaError_t LaunchAggFew(const AggLaunch &p, const FewLayout &l, uint64_t *spill
         return cudaSuccess;
     }
     const SpillArgs sp{spill, nSpill, spillCap, nullptr, 0};
-    auto kernel = p.key.kind == KEY_SINGLE ? AggFewKernel<KEY_SINGLE> : AggFewKernel<KEY_PACKED>;
+    const bool single = p.key.kind == KEY_SINGLE;
+    auto kernel = l.threads == 256 ? (single ? AggFewKernel<KEY_SINGLE, 256> : AggFewKernel<KEY_PACKED, 256>)
+        : l.threads == 192         ? (single ? AggFewKernel<KEY_SINGLE, 192> : AggFewKernel<KEY_PACKED, 192>)
+                                   : (single ? AggFewKernel<KEY_SINGLE, 128> : AggFewKernel<KEY_PACKED, 128>);
     const cudaError_t err = EnsureDynamicSmem(reinterpret_cast<const void *>(kernel), kFewSmemBytes);
     if (err != cudaSuccess) {
         return err;
     }
     const int grid = p.nTiles < LaunchAggFewGrid() ? p.nTiles : LaunchAggFewGrid();
-    kernel<<<grid, kFewThreads, l.smemBytes, stream>>>(p, l, sp);
+    kernel<<<grid, l.threads, l.smemBytes, stream>>>(p, l, sp);
     return cudaGetLastError();
 }
 

@@ -218,3 +218,38 @@ def test_radix_tables_that_overflow(gpu, copies):
     assert np.array_equal(cols[1][0][order], want)
     assert np.array_equal(cols[2][0][order], np.bincount(inv, weights=d, minlength=len(uniq)))
     assert np.array_equal(cols[3][0][order], top)
+
+
+@pytest.mark.parametrize("key", ["long", "pair"])
+@pytest.mark.parametrize("plan,groups,kernel", [
+    ("six", 9, FEW), ("six", 10, FEW), ("six", 12, FEW), ("six", 13, PARTITIONS),
+    ("sum", 21, FEW), ("sum", 22, FEW), ("sum", 29, FEW), ("sum", 34, FEW), ("sum", 40, PARTITIONS)])
+def test_few_groups_up_to_the_most(gpu, key, plan, groups, kernel):
+    """Up to what 256 threads have room for without the errors of the double sums; with them the most groups take 192
+    threads (six aggregates from 10, one sum from 22) and 128 (one sum from 29)."""
+    rng = np.random.default_rng(groups)
+    n = 270_001
+    code = rng.integers(0, groups, n)
+    keys, ktypes = ([code * 2**40], [L]) if key == "long" else ([(code % 13).astype(np.int32), code * 2**33], [I, L])
+    k = len(keys)
+    v = rng.integers(-2**40, 2**40, n)
+    d = rng.integers(-2**30, 2**30, n).astype(np.float64)
+    spec = [(SUM, k, L, L), (CNT, k, L, L), (MIN, k, L, L), (MAX, k, L, L), (SUM, k + 1, D, D), (AVG, k + 1, D, D)]
+    spec = spec if plan == "six" else spec[4:5]
+    cols, _ = run_agg(list(range(k)), ktypes, [[c] for _, c, _, _ in spec], [[t] for _, _, t, _ in spec],
+                      [[o] for *_, o in spec], [f for f, *_ in spec], keys + [v, d], ktypes + [L, D], batch_sizes=(100_000,))
+    assert last_kernel()[0] == kernel
+    order = np.argsort(cols[k - 1][0])
+    count = np.bincount(code, minlength=groups)
+    total = np.bincount(code, weights=d, minlength=groups)
+    lo, hi = np.full(groups, 2**60), np.full(groups, -2**60)
+    np.minimum.at(lo, code, v)
+    np.maximum.at(hi, code, v)
+    want = {"six": [np.bincount(code, weights=v, minlength=groups).astype(np.int64), count, lo, hi, total, total / count],
+            "sum": [total]}[plan]
+    if plan == "six":
+        want[0] = np.zeros(groups, np.int64)
+        np.add.at(want[0], code, v)
+    assert len(order) == groups
+    for (got, _), w in zip(cols[k:], want):
+        assert np.array_equal(got[order], w)
