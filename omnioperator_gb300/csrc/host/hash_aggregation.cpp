@@ -1745,17 +1745,8 @@ void HashAggregationOperator::AggregateRows(omg::BatchTable &bt, bool last, bool
     im.timer.Stop(s);
     ++counters_[0];
     if (last && im.capacity <= kAheadSlots && !radix && im.denseGroups == 0 && plan_.dictInputs.empty()) {
-        // The groups out, without waiting to hear how many there are: at most one per slot, or per row.  Not into
-        // device columns that would have to be copied for being much too large, as where nothing is known of the
-        // groups: some 30 copies, 90 us, where the wait takes 15.
-        const uint64_t bound = std::min<uint64_t>(im.capacity, im.groups + static_cast<uint64_t>(rows)) + 2;
-        size_t rowBytes = 0;
-        for (const OutSpec &os : plan_.outs) {
-            rowBytes += static_cast<size_t>(os.outWidth);
-        }
-        if (im.estimate > 0 || !deviceOutput_ || bound * rowBytes <= kTrimBytes) {
-            LaunchExtract(im.ahead, bound, s);
-        }
+        // The groups out, without waiting to hear how many there are: at most one per slot, or per row.
+        LaunchExtract(im.ahead, std::min<uint64_t>(im.capacity, im.groups + static_cast<uint64_t>(rows)) + 2, s);
     }
     unsigned long long *h = im.hostStats.Get();
     CudaCheck(cudaMemcpyAsync(h, im.stats.Get(), kStatsWords * sizeof(*h), cudaMemcpyDeviceToHost, s), "read stats");
@@ -2341,13 +2332,17 @@ void HashAggregationOperator::TrimOutputs(ExtractRun &x, int64_t rows, cudaStrea
     }
     omg::BufferPtr block = x.onHost ? omg::Buffer::NewHost(need, false) : omg::Buffer::NewDevice(need, s, false);
     size_t at = 0;
+    omg::CopyRanges ranges;
+    ranges.n = 0;
+    std::vector<omg::BufferPtr> old;
     auto move = [&](omg::BufferPtr &buf, size_t bytes, size_t room) {
         omg::BufferPtr to = omg::Buffer::Slice(block, at, room);
         if (x.onHost) {
             std::memcpy(to->Data(), buf->Data(), bytes);
         } else {
-            CudaCheck(cudaMemcpyAsync(to->Data(), buf->Data(), bytes, cudaMemcpyDeviceToDevice, s), "trim output");
+            ranges.r[ranges.n++] = omg::CopyRange{buf->Data(), to->Data(), bytes};
         }
+        old.push_back(buf);
         buf = to;
         at += Up256(room);
     };
@@ -2357,6 +2352,7 @@ void HashAggregationOperator::TrimOutputs(ExtractRun &x, int64_t rows, cudaStrea
         move(c.nulls, std::min(nullBytes, c.nulls->Bytes()), nullBytes);
     }
     if (!x.onHost) {
+        CudaCheck(omg::LaunchCopyRanges(ranges, s), "trim output");
         impl_->stream.Sync();  // readable on every stream, as it was
     }
 }

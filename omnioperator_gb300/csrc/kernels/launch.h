@@ -76,6 +76,17 @@ int LastProbeKernel();
 
 // ---- utilities (util.cu)
 // Masked-input NULL bitmaps, one per job (see MaskJob).
+// r[0, n): `bytes` bytes each from one 256-byte boundary to another (up to 15 bytes more are copied).
+struct CopyRange {
+    const void *from;
+    void *to;
+    size_t bytes;
+};
+struct CopyRanges {
+    int32_t n;
+    CopyRange r[2 * kMaxOutCols];
+};
+cudaError_t LaunchCopyRanges(const CopyRanges &ranges, cudaStream_t stream);
 cudaError_t LaunchMaskNulls(const MaskJob *jobs, int32_t nJobs, cudaStream_t stream);
 // [0] rows, [1] and [2] two order-independent 64-bit sums of per-row column hashes.
 cudaError_t LaunchFingerprint(const BatchDesc *batches, const TileDesc *tiles, int32_t nTiles, int32_t nCols,

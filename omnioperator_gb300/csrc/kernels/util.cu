@@ -159,6 +159,27 @@ int BlocksPerSM(const void *kernel, int threads, size_t smemBytes)
     return n;
 }
 
+// Output columns and their bitmaps to buffers of their size in one launch: as 30 copies they took 90 us for columns of
+// 2,000 rows, whose time is launches.
+__global__ void __launch_bounds__(256) CopyRangesKernel(const __grid_constant__ CopyRanges c)
+{
+    const CopyRange r = c.r[blockIdx.y];
+    const uint4 *from = static_cast<const uint4 *>(r.from);
+    uint4 *to = static_cast<uint4 *>(r.to);
+    for (size_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (r.bytes + 15) / 16; i += gridDim.x * blockDim.x) {
+        to[i] = from[i];
+    }
+}
+
+cudaError_t LaunchCopyRanges(const CopyRanges &ranges, cudaStream_t stream)
+{
+    if (ranges.n <= 0) {
+        return cudaSuccess;
+    }
+    CopyRangesKernel<<<dim3(DeviceSMCount() / 8, ranges.n), 256, 0, stream>>>(ranges);
+    return cudaGetLastError();
+}
+
 cudaError_t LaunchMaskNulls(const MaskJob *jobs, int32_t nJobs, cudaStream_t stream)
 {
     if (nJobs <= 0) {
